@@ -258,3 +258,101 @@ def tolerance(case):
         # (single rows of 1024 to 3328 values, where one such step weighs most), 1.1e-4 and below for larger cases.
         return {"rel": 1e-3, "max": 1.2e-2}
     return {"rel": 3e-6, "max": 1.2e-5}            # seen: 8e-7 and 3e-6
+
+
+# ------------------------------------------------- the same results in 64 bits
+
+def _half_at(b, i):                               # fp16 at byte i of every block [..., bytes]
+    return b[..., i:i + 2].contiguous().view(torch.float16)[..., 0].double()
+
+
+def _unpack_nibbles(q):                           # the inverse of _nibbles
+    return torch.cat([q & 15, q >> 4], -1)
+
+
+def _unpack_rows(t, raw, n, k):
+    """The values of n rows' GGUF bytes, in 64 bits."""
+    rb = any_row_bytes(GGMLType[t], k)
+    raw = raw[: n * rb].view(n, rb)
+    if t == "F16":
+        return raw.view(torch.float16).double()
+    if t in ("Q4_0", "Q5_0", "Q8_0"):
+        b = raw.view(n, k // 32, -1)
+        if t == "Q8_0":
+            q = b[..., 2:].contiguous().view(torch.int8).double()
+        elif t == "Q4_0":
+            q = _unpack_nibbles(b[..., 2:]).double() - 8
+        else:
+            bit = (b[..., 2:6, None] >> torch.arange(8, dtype=torch.uint8, device=raw.device)) & 1
+            q = (_unpack_nibbles(b[..., 6:]) | (bit.reshape(n, k // 32, 32) << 4)).double() - 16
+        return (_half_at(b, 0)[..., None] * q).view(n, k)
+    b = raw.view(n, k // 256, -1)
+    if t == "Q6_K":
+        ql, qh = b[..., :128].reshape(n, k // 256, 2, 2, 32), b[..., 128:192].reshape(n, k // 256, 2, 32)
+        low = torch.cat([ql & 15, ql >> 4], -2)
+        high = torch.stack([(qh >> (2 * i)) & 3 for i in range(4)], -2)
+        q = (low | (high << 4)).double() - 32
+        sc = b[..., 192:208].contiguous().view(torch.int8).double()
+        return (_half_at(b, 208)[..., None, None] * sc[..., None] * q.reshape(n, k // 256, 16, 16)).view(n, k)
+    s = b[..., 4:16]                              # Q4_K, Q5_K
+    sc = torch.cat([s[..., :4] & 63, (s[..., 8:] & 15) | ((s[..., :4] >> 6) << 4)], -1).double()
+    mn = torch.cat([s[..., 4:8] & 63, (s[..., 8:] >> 4) | ((s[..., 4:8] >> 6) << 4)], -1).double()
+    qs = b[..., -128:].reshape(n, k // 256, 4, 32)
+    q = torch.stack([qs & 15, qs >> 4], -2).reshape(n, k // 256, 8, 32)
+    if t == "Q5_K":
+        high = (b[..., None, 16:48] >> torch.arange(8, dtype=torch.uint8, device=raw.device)[:, None]) & 1
+        q = q | (high << 4)
+    return (_half_at(b, 0)[..., None, None] * sc[..., None] * q.double() - (_half_at(b, 2)[..., None] * mn)[..., None]).view(n, k)
+
+
+def _seen(t, x):
+    """Activations as the matmul of weight type t sees them: rounded to 8 bits per 32 values, or as they are."""
+    if t in ("F16", "Q5_K"):
+        return x.double()
+    b = x.float().view(*x.shape[:-1], -1, 32)
+    d = b.abs().amax(-1, keepdim=True) / 127
+    q = (b * torch.where(d > 0, 1 / d, d)).round()
+    return (d.double() * q.double()).view(x.shape)
+
+
+def exact(case, seed):
+    """What run() returns, in 64 bits except for the rounding of the activations to 8 bits, which the path prescribes in 32."""
+    s = prepare(case, seed)
+    kind, t = case["kind"], case["type"]
+
+    def mm(x, raw, t, k, n):
+        x = _seen(t, x)
+        return torch.cat([x @ _unpack_rows(t, raw[r * any_row_bytes(GGMLType[t], k):], min(4096, n - r), k).T for r in range(0, n, 4096)], -1)
+
+    if kind == "layer":
+        h, kv, f = case["hidden"], case["kv"], case["ffn"]
+
+        def norm(x, w):
+            inv = (1 / (x.double().square().mean(-1, keepdim=True) + EPS).sqrt()).float()
+            return x * inv * w
+
+        a, b = norm(s["x"], s["norm1"]), norm(s["mid"], s["norm2"])
+        return ([mm(a, w, t, h, n) for w, n in zip(s["qkv"], (h, kv, kv))] + [mm(s["attn"], s["o"], t, h, h)] +
+                [mm(b, w, t, h, f) for w in s["gate_up"]] + [mm(s["act"], s["down"], case["down_type"], f, h)])
+    if kind == "matmul":
+        return mm(s["x"], s["w"], t, case["k"], case["n"])
+    if kind == "head":
+        y, cap = mm(s["x"], s["w"], t, case["hidden"], case["vocab"]), case["softcap"]
+        return cap * (y / cap).tanh() if cap else y
+    if kind == "host":
+        return mm(torch.from_numpy(s["x"]), torch.from_numpy(s["w"].data.reshape(-1)), t, case["k"], case["n"]).numpy()
+    e, h, i, k = case["experts"], case["hidden"], case["inter"], case["top_k"]
+    gu_bytes, dn_bytes = 2 * i * any_row_bytes(GGMLType[t], h), h * any_row_bytes(GGMLType[t], i)
+    gate_up, down = (lambda x, j: mm(x, s["gate_up"][j * gu_bytes:], t, h, 2 * i)), (lambda x, j: mm(x, s["down"][j * dn_bytes:], t, i, h))
+    if kind == "moe_token":
+        chosen = s["idx"].tolist()
+        return [torch.cat([gate_up(s["x"], j) for j in chosen]), torch.cat([down(s["act"][n:n + 1], j) for n, j in enumerate(chosen)])]
+    weight, idx = s["logits"].double().softmax(-1).topk(k)
+    weight = weight / weight.sum(-1, keepdim=True)
+    out = torch.zeros(case["tokens"], h, dtype=torch.float64, device="cuda")
+    for j in range(e):
+        token, slot = (idx == j).nonzero(as_tuple=True)
+        if len(token):
+            gate, up = gate_up(s["x"][token], j).split(i, -1)
+            out.index_add_(0, token, weight[token, slot, None] * down(torch.nn.functional.silu(gate) * up, j))
+    return [None, weight, out]
