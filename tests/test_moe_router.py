@@ -67,3 +67,28 @@ def test_fused_ffn_with_router_and_down_scale(oracle):
         wgt = (wts[tok] * scale[idx[tok]]).astype(np.float32)
         want[tok] = (dn.astype(np.float64) * wgt[:, None]).sum(axis=0)
     check_close(out.cpu().numpy(), want, "fused FFN with down_scale")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,E,k", [(3, 1, 1), (9, 33, 33), (2, 3073, 5), (6, 600, 40)])
+def test_device_router_edges(T, E, k):
+    """One expert, every expert selected, more experts than a warp keeps in shared memory, several equal probabilities (zeros
+    among them), rows with infinities and with a value that is not a number."""
+    import torch
+    from laplace_b200 import device
+    logits = synth.normal_f32(150 + E, (T, E))
+    logits[0, ::3] = logits[0, 0]
+    if E > 1:
+        logits[1, : E // 2] = -np.inf
+        logits[1, E // 2:: 7] -= 200.0
+    bad = T > 4 and E > 1
+    if bad:
+        logits[4, E // 3] = np.nan
+    idx, wts = (v.cpu().numpy() for v in device.moe_route(torch.from_numpy(logits).cuda(), k))
+    device.sync()
+    rows = [r for r in range(T) if not (bad and r == 4)]
+    ridx, rw = route(logits[rows], k)
+    assert np.array_equal(idx[rows], ridx)
+    assert np.allclose(wts[rows], rw, rtol=2e-6, atol=0.0)
+    if bad:
+        assert not idx[4].any() and np.isnan(wts[4]).all()
