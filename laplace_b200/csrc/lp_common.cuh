@@ -94,7 +94,17 @@ struct PeerOut {
     int       col0;              // first column of this GPU's slice
 };
 int launch_gemv_stream(const GemvArgs& a, cudaStream_t st);
-int launch_gemv_mma_q4k(const float* x, const uint8_t* w, float* y, int M, int K, int N, cudaStream_t st);
+// 2..32 activation rows on mma.sync int8 (lp_gemm_i8.cu): one or several matrices, optional RMSNorm in front
+bool gemm_i8_supports(uint32_t type, int M, int K, const uint8_t* const* ws, int n_mats);
+int  launch_gemm_i8(const float* x, const float* norm_w, float eps, float* x_norm_out, const uint8_t* const* ws, float* const* ys,
+                    const int* ns, int n_mats, uint32_t type, int M, int K, cudaStream_t st);
+int  launch_quantize_i8(const float* x, const float* norm_w, float eps, float* x_norm_out, uint32_t type, int M, int K, uint8_t* img, cudaStream_t st);
+constexpr int I8_JOB_ROWS = 256;       // weight rows of an expert job
+int      gemm_i8_job_tokens(uint32_t type, int K, const uint8_t* w);
+uint32_t gemm_i8_act_bytes(uint32_t type);
+bool     gemm_i8_lane8(uint32_t type);
+int launch_gemm_i8_jobs(const uint8_t* w, uint32_t type, long long w_rows, const uint8_t* img, float* y, int K, int N, int tokens, int jobs_max,
+                        const int4* tab, const int* n_jobs, const int* out_row, int out_identity, cudaStream_t st);
 // weight types served with fp32 activations (the reference's scalar path), dequantize() and friends (lp_types.cu)
 bool   f32act_type(uint32_t type);
 bool   dequant_type(uint32_t type);

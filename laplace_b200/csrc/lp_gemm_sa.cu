@@ -36,8 +36,8 @@
 // All mbarrier waits are bounded; a wait that gives up raises the status word and every role leaves its loop.
 #include <cuda_fp16.h>
 
-#include <vector>
-
+#include "lp_i8.cuh"
+#include "lp_scratch.cuh"
 #include "lp_tc.cuh"
 
 namespace lp {
@@ -1078,34 +1078,6 @@ __global__ void __launch_bounds__(256) sk_fixup_kernel(const float* __restrict__
 
 inline size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
-// Scratch owned by this translation unit. A buffer that has been handed to a launch may be baked into a captured
-// CUDA graph (its address and the tensor maps built from it), so a buffer is never freed when a larger one is
-// needed: superseded buffers are kept until laplace_cuda_shutdown. Growing calls the allocator, which is illegal
-// while the call's stream is being captured: such a call is refused and the capture stays valid.
-struct Scratch {
-    void*  p = nullptr;
-    size_t cap = 0;
-    std::vector<void*> retired;
-    int ensure(size_t n, cudaStream_t st) {
-        if (n <= cap) return LAPLACE_OK;
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
-            return fail(LAPLACE_ERR_STATE, "the call needs %zu bytes of scratch but only %zu are allocated, and its stream is being "
-                                           "captured: make the same call once before the capture begins", n, cap);
-        if (p) retired.push_back(p);
-        p = nullptr; cap = 0;
-        cudaError_t e = cudaMalloc(&p, n + n / 8);
-        if (e != cudaSuccess) return cuda_check(e, "cudaMalloc scratch");
-        cap = n + n / 8;
-        return LAPLACE_OK;
-    }
-    void release() {
-        if (p) cudaFree(p);
-        for (void* q : retired) cudaFree(q);
-        retired.clear();
-        p = nullptr; cap = 0;
-    }
-};
 Scratch g_scratch;
 
 struct OperandBytes { size_t a, g, s; size_t total() const { return a + g + s; } };
@@ -1429,6 +1401,7 @@ __global__ void __launch_bounds__(1024) moe_plan_sa_kernel(const int* __restrict
         dst_row[p] = r;
         out_row[r] = p;
     }
+Scratch& gemm_scratch() { return g_scratch; }
 }
 
 // quantize_sa_kernel with a row gather on the way in and a row scatter on the way out: pair p reads x row
