@@ -1349,12 +1349,12 @@ int launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const 
 namespace {
 
 // One block plans the whole call: pairs per expert, every pair's slot inside its expert, the first operand row of
-// every expert (counts padded to 16 rows), the operand row of every pair and the inverse map, and the tile tables
+// every expert (counts padded to `pad` rows: 16 for the tcgen05 kernels, 8 for the int8 one), the operand row of every pair and the inverse map, and the tile tables
 // {first operand row, first weight row inside the expert, first weight row of the expert, tokens}: for every expert,
-// for every group of up to 128 of its tokens, one tile per 128 weight rows. A second table (another N over the same
+// for every group of up to `group` of its tokens, one tile per `tile` weight rows. A second table (another N over the same
 // row groups) serves the second matmul of a fused FFN; tiles_n2 = 0 leaves it out. Which slot a pair gets depends on
 // the order the atomics land in; results do not.
-__global__ void __launch_bounds__(1024) moe_plan_sa_kernel(const int* __restrict__ pair_expert, int P, int E, int rows_max,
+__global__ void __launch_bounds__(1024) moe_plan_sa_kernel(const int* __restrict__ pair_expert, int P, int E, int pad, int group, int tile, int rows_max,
                                                            int* __restrict__ dst_row, int* __restrict__ out_row,
                                                            int N1, int tiles_n1, int4* __restrict__ tab1, int* __restrict__ n_tiles1,
                                                            int N2, int tiles_n2, int4* __restrict__ tab2, int* __restrict__ n_tiles2,
@@ -1379,19 +1379,19 @@ __global__ void __launch_bounds__(1024) moe_plan_sa_kernel(const int* __restrict
         for (int e = 0; e < E; ++e) {
             base[e] = rows;
             grp0[e] = groups;
-            rows += (cnt[e] + 15) & ~15;
-            groups += (cnt[e] + TT - 1) / TT;
+            rows += (cnt[e] + pad - 1) / pad * pad;
+            groups += (cnt[e] + group - 1) / group;
         }
         *n_tiles1 = groups * tiles_n1;
         if (tiles_n2) *n_tiles2 = groups * tiles_n2;
     }
     __syncthreads();
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        const int groups = (cnt[e] + TT - 1) / TT;
+        const int groups = (cnt[e] + group - 1) / group;
         for (int g = 0; g < groups; ++g) {
-            const int nt = cnt[e] - g * TT < TT ? cnt[e] - g * TT : TT;
-            for (int t = 0; t < tiles_n1; ++t) tab1[(grp0[e] + g) * tiles_n1 + t] = make_int4(base[e] + g * TT, t * TW, e * N1, nt);
-            for (int t = 0; t < tiles_n2; ++t) tab2[(grp0[e] + g) * tiles_n2 + t] = make_int4(base[e] + g * TT, t * TW, e * N2, nt);
+            const int nt = cnt[e] - g * group < group ? cnt[e] - g * group : group;
+            for (int t = 0; t < tiles_n1; ++t) tab1[(grp0[e] + g) * tiles_n1 + t] = make_int4(base[e] + g * group, t * tile, e * N1, nt);
+            for (int t = 0; t < tiles_n2; ++t) tab2[(grp0[e] + g) * tiles_n2 + t] = make_int4(base[e] + g * group, t * tile, e * N2, nt);
         }
     }
     for (int p = threadIdx.x; p < P; p += blockDim.x) {
@@ -1401,7 +1401,6 @@ __global__ void __launch_bounds__(1024) moe_plan_sa_kernel(const int* __restrict
         dst_row[p] = r;
         out_row[r] = p;
     }
-Scratch& gemm_scratch() { return g_scratch; }
 }
 
 // quantize_sa_kernel with a row gather on the way in and a row scatter on the way out: pair p reads x row
@@ -1476,20 +1475,20 @@ Scratch g_moe_scratch;
 
 // Upper bounds that hold for every routing of P pairs over E experts.
 struct GroupBounds { size_t rows, groups; };
-GroupBounds group_bounds(int P, int E) {
+GroupBounds group_bounds(int P, int E, int group = TT) {
     const size_t live = static_cast<size_t>(E < P ? E : P);
     GroupBounds b;
     b.rows = ((static_cast<size_t>(P) + 15 * live + TT - 1) / TT + 1) * TT;       // every expert pads to 16 rows; one box of slack
-    b.groups = static_cast<size_t>(P) / TT + live;
+    b.groups = static_cast<size_t>(P) / group + live;
     return b;
 }
 
-int launch_plan(const int* pair_expert, int P, int E, int rows_max, int* dst_row, int* out_row, int N1, int tiles_n1, int4* tab1,
+int launch_plan(const int* pair_expert, int P, int E, int pad, int group, int tile, int rows_max, int* dst_row, int* out_row, int N1, int tiles_n1, int4* tab1,
                 int* n_tiles1, int N2, int tiles_n2, int4* tab2, int* n_tiles2, cudaStream_t st) {
     Context& c = ctx();
     const size_t sm = 3 * static_cast<size_t>(E) * sizeof(int);
     if (sm > 40 * 1024) return fail(LAPLACE_ERR_LIMIT, "moe: %d experts are more than the planning kernel holds", E);
-    moe_plan_sa_kernel<<<1, 1024, sm, st>>>(pair_expert, P, E, rows_max, dst_row, out_row, N1, tiles_n1, tab1, n_tiles1,
+    moe_plan_sa_kernel<<<1, 1024, sm, st>>>(pair_expert, P, E, pad, group, tile, rows_max, dst_row, out_row, N1, tiles_n1, tab1, n_tiles1,
                                             N2, tiles_n2, tab2, n_tiles2, c.d_err);
     c.launches++;
     return cuda_check(cudaGetLastError(), "moe_plan launch");
@@ -1525,7 +1524,7 @@ int launch_moe_grouped_sa(const float* x, const uint8_t* w, uint32_t type, const
     int* out_row = reinterpret_cast<int*>(s);       s += out_bytes;
     int4* tab = reinterpret_cast<int4*>(s);         s += tab_bytes;
     int* n_tiles = reinterpret_cast<int*>(s);
-    if ((rc = launch_plan(pair_expert, P, E, static_cast<int>(gb.rows), dst_row, out_row, N, tiles_n, tab, n_tiles, 0, 0, nullptr, nullptr, st)))
+    if ((rc = launch_plan(pair_expert, P, E, 16, TT, TW, static_cast<int>(gb.rows), dst_row, out_row, N, tiles_n, tab, n_tiles, 0, 0, nullptr, nullptr, st)))
         return rc;
     quantize_sa_mapped_kernel<<<P, 256, 0, st>>>(x, K, pair_row, 1, dst_row, op);
     c.launches++;
@@ -1570,7 +1569,7 @@ int launch_moe_ffn_sa(const float* x, const uint8_t* w_gate_up, const uint8_t* w
     float* dn = reinterpret_cast<float*>(s);        s += dn_bytes;
     int* n_tiles1 = reinterpret_cast<int*>(s);
     int* n_tiles2 = n_tiles1 + 1;
-    if ((rc = launch_plan(top_idx, P, E, static_cast<int>(gb.rows), dst_row, out_row, 2 * I, tiles_n1, tab1, n_tiles1, H, tiles_n2, tab2, n_tiles2, st)))
+    if ((rc = launch_plan(top_idx, P, E, 16, TT, TW, static_cast<int>(gb.rows), dst_row, out_row, 2 * I, tiles_n1, tab1, n_tiles1, H, tiles_n2, tab2, n_tiles2, st)))
         return rc;
     quantize_sa_mapped_kernel<<<P, 256, 0, st>>>(x, H, nullptr, top_k, dst_row, op1);
     c.launches++;
@@ -1592,13 +1591,7 @@ int launch_moe_ffn_sa(const float* x, const uint8_t* w_gate_up, const uint8_t* w
     L2.tiles_m = 1; L2.tiles_n = tiles_n2; L2.grid = grid_for_tiles(gb.groups * tiles_n2);
     if ((rc = run_sa_kernel(L2, st))) return rc;
 
-    const long long total4 = static_cast<long long>(T) * (H / 4);
-    long long blocks = (total4 + 255) / 256;
-    if (blocks > static_cast<long long>(c.sm_count) * 8) blocks = static_cast<long long>(c.sm_count) * 8;
-    moe_combine_sa_kernel<<<static_cast<int>(blocks < 1 ? 1 : blocks), 256, 0, st>>>(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out);
-    c.launches++;
-    c.last_path = 4;
-    return cuda_check(cudaGetLastError(), "moe_combine launch");
+    return launch_combine(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out, st);
 }
 
 
@@ -1655,6 +1648,32 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(const float
     for (int k = 0; k < top_k; ++k) {
         float best_p = -1.0f;
         int best = 0x7fffffff;
+// The same two steps for the int8 kernel: rows in its fragment order (lp_i8.cuh).
+__global__ void __launch_bounds__(256) quantize_i8_mapped_kernel(const float* __restrict__ x, int K, const int* __restrict__ src_rows, int src_div,
+                                                                 const int* __restrict__ dst_rows, int lane8, uint32_t act_bytes, uint8_t* __restrict__ img) {
+    const int p = blockIdx.x;
+    const int dr = __ldg(dst_rows + p);
+    if (dr < 0) return;
+    const float* xr = x + static_cast<size_t>(src_rows ? __ldg(src_rows + p) : p / src_div) * K;
+    i8::quantize_row_i8([&](int b, int t8) { return __ldg(reinterpret_cast<const float4*>(xr + b * 32) + t8); }, K, lane8, act_bytes,
+                        img + static_cast<size_t>(dr >> 3) * (K / 256) * act_bytes, dr & 7);
+}
+__global__ void __launch_bounds__(256) moe_act_quant_i8_kernel(const float* __restrict__ gu, int I, int activation, const int* __restrict__ dst_rows,
+                                                               int lane8, uint32_t act_bytes, uint8_t* __restrict__ img, float* __restrict__ h_out) {
+    const int p = blockIdx.x;
+    const int r = __ldg(dst_rows + p);
+    if (r < 0) return;
+    const float* row = gu + static_cast<size_t>(r) * (2 * I);
+    i8::quantize_row_i8([&](int b, int t8) {
+        const float4 g = __ldg(reinterpret_cast<const float4*>(row + b * 32) + t8);
+        const float4 u = __ldg(reinterpret_cast<const float4*>(row + I + b * 32) + t8);
+        const float4 h = activation == 1 ? make_float4(act_geglu(g.x, u.x), act_geglu(g.y, u.y), act_geglu(g.z, u.z), act_geglu(g.w, u.w))
+                                         : make_float4(act_swiglu(g.x, u.x), act_swiglu(g.y, u.y), act_swiglu(g.z, u.z), act_swiglu(g.w, u.w));
+        if (h_out) reinterpret_cast<float4*>(h_out + static_cast<size_t>(p) * I + b * 32)[t8] = h;
+        return h;
+    }, I, lane8, act_bytes, img + static_cast<size_t>(r >> 3) * (I / 256) * act_bytes, r & 7);
+}
+
         for (int e = lane; e < E; e += 32) {
             const float v = p_ld ? p[e] : __fdiv_rn(expf(__fsub_rn(__ldg(l + e), maxl)), suml);
             if ((v < last_p || (v == last_p && e > last_e)) && v > best_p) { best = e; best_p = v; }
@@ -1714,11 +1733,49 @@ __global__ void moe_unpack_kernel(const float* __restrict__ packed, int T, int H
         if (c < H) x[static_cast<long long>(t) * H + c] = v;
         else if (c < H + k) {
             const int e = __float_as_int(v) - first;
+namespace {
+
+// A few tokens per expert: the int8 kernel, which costs in proportion to the tokens, else the tcgen05 kernels, which cost the
+// same up to 32 tokens and little more up to 128.
+constexpr int I8_PAIRS_PER_EXPERT = 32;
+bool few_per_expert(int P, int E) { return P <= I8_PAIRS_PER_EXPERT * static_cast<long long>(E < P ? E : P); }
+
+size_t image_bytes(uint32_t type, size_t rows, int K) { return align256((rows + 7) / 8 * (K / 256) * gemm_i8_act_bytes(type)); }
+
+int launch_moe_grouped_i8(const float* x, const uint8_t* w, uint32_t type, const int* pair_expert, const int* pair_row, int P, int E, float* y, int K, int N,
+                          int tokens, cudaStream_t st) {
+    Context& c = ctx();
+    const int tiles_n = (N + I8_JOB_ROWS - 1) / I8_JOB_ROWS;
+    const GroupBounds gb = group_bounds(P, E, tokens);
+    const size_t pair_bytes = align256(sizeof(int) * static_cast<size_t>(P)), out_bytes = align256(sizeof(int) * gb.rows);
+    const size_t tab_bytes = align256(sizeof(int4) * gb.groups * tiles_n), img_bytes = image_bytes(type, gb.rows, K);
+    int rc;
+    if ((rc = g_moe_scratch.ensure(img_bytes + pair_bytes + out_bytes + tab_bytes + 256, st))) return rc;
+    uint8_t* s = static_cast<uint8_t*>(g_moe_scratch.p);
+    uint8_t* img = s;                               s += img_bytes;
+    int* dst_row = reinterpret_cast<int*>(s);       s += pair_bytes;
+    int* out_row = reinterpret_cast<int*>(s);       s += out_bytes;
+    int4* tab = reinterpret_cast<int4*>(s);         s += tab_bytes;
+    int* n_tiles = reinterpret_cast<int*>(s);
+    if ((rc = launch_plan(pair_expert, P, E, 8, tokens, I8_JOB_ROWS, static_cast<int>(gb.rows), dst_row, out_row, N, tiles_n, tab, n_tiles, 0, 0, nullptr, nullptr, st)))
+        return rc;
+    quantize_i8_mapped_kernel<<<P, 256, 0, st>>>(x, K, pair_row, 1, dst_row, gemm_i8_lane8(type), gemm_i8_act_bytes(type), img);
+    c.launches++;
+    if ((rc = cuda_check(cudaGetLastError(), "moe quantize launch"))) return rc;
+    rc = launch_gemm_i8_jobs(w, type, static_cast<long long>(E) * N, img, y, K, N, tokens, static_cast<int>(gb.groups * tiles_n), tab, n_tiles, out_row, 0, st);
+    if (rc == LAPLACE_OK) c.last_path = 3;
+    return rc;
+}
+
+}  // namespace
+
             idx_local[t * k + (c - H)] = (e >= 0 && e < count) ? e : -1;
         } else wts[t * k + (c - H - k)] = v;
     }
 }
 
+    if (few_per_expert(P, E))
+        if (const int tokens = gemm_i8_job_tokens(type, K, w)) return launch_moe_grouped_i8(x, w, type, pair_expert, pair_row, P, E, y, K, N, tokens, st);
 }  // namespace
 
 int launch_moe_pack(const float* x, const int* idx, const float* wts, int T, int H, int k, float* packed, cudaStream_t st) {
@@ -1747,6 +1804,61 @@ int launch_moe_unpack(const float* packed, int T, int H, int k, int first, int c
 // path: a serving process that has handed all free HBM to its own pools (KV cache,
 // activations), so that cudaMalloc would fail or fragment them, and latency-bound loops that
 // cannot take the allocator's locks or the implicit device synchronisation that comes with
+namespace {
+
+int launch_combine(const float* dn, const int* dst_row, const float* top_w, const int* top_idx, const float* down_scale, int T, int top_k, int H, float* out,
+                   cudaStream_t st) {
+    Context& c = ctx();
+    const long long total4 = static_cast<long long>(T) * (H / 4);
+    long long blocks = (total4 + 255) / 256;
+    if (blocks > static_cast<long long>(c.sm_count) * 8) blocks = static_cast<long long>(c.sm_count) * 8;
+    moe_combine_sa_kernel<<<static_cast<int>(blocks < 1 ? 1 : blocks), 256, 0, st>>>(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out);
+    c.launches++;
+    c.last_path = 4;
+    return cuda_check(cudaGetLastError(), "moe_combine launch");
+}
+
+int launch_moe_ffn_i8(const float* x, const uint8_t* w_gate_up, const uint8_t* w_down, uint32_t type_gu, uint32_t type_dn, const int* top_idx, const float* top_w,
+                      const float* down_scale, int T, int top_k, int E, int H, int I, int activation, float* out, float* h_out, int tokens, cudaStream_t st) {
+    Context& c = ctx();
+    const int P = T * top_k;
+    const int tiles_n1 = (2 * I + I8_JOB_ROWS - 1) / I8_JOB_ROWS, tiles_n2 = (H + I8_JOB_ROWS - 1) / I8_JOB_ROWS;
+    const GroupBounds gb = group_bounds(P, E, tokens);
+    const size_t pair_bytes = align256(sizeof(int) * static_cast<size_t>(P)), out_bytes = align256(sizeof(int) * gb.rows);
+    const size_t tab1_bytes = align256(sizeof(int4) * gb.groups * tiles_n1), tab2_bytes = align256(sizeof(int4) * gb.groups * tiles_n2);
+    const size_t gu_bytes = align256(gb.rows * 2 * I * sizeof(float)), dn_bytes = align256(gb.rows * H * sizeof(float));
+    const size_t img1_bytes = image_bytes(type_gu, gb.rows, H), img2_bytes = image_bytes(type_dn, gb.rows, I);
+    int rc;
+    if ((rc = g_moe_scratch.ensure(img1_bytes + img2_bytes + pair_bytes + out_bytes + tab1_bytes + tab2_bytes + gu_bytes + dn_bytes + 256, st))) return rc;
+    uint8_t* s = static_cast<uint8_t*>(g_moe_scratch.p);
+    uint8_t* img1 = s;                              s += img1_bytes;
+    uint8_t* img2 = s;                              s += img2_bytes;
+    int* dst_row = reinterpret_cast<int*>(s);       s += pair_bytes;
+    int* out_row = reinterpret_cast<int*>(s);       s += out_bytes;
+    int4* tab1 = reinterpret_cast<int4*>(s);        s += tab1_bytes;
+    int4* tab2 = reinterpret_cast<int4*>(s);        s += tab2_bytes;
+    float* gu = reinterpret_cast<float*>(s);        s += gu_bytes;
+    float* dn = reinterpret_cast<float*>(s);        s += dn_bytes;
+    int* n_tiles1 = reinterpret_cast<int*>(s);
+    int* n_tiles2 = n_tiles1 + 1;
+    if ((rc = launch_plan(top_idx, P, E, 8, tokens, I8_JOB_ROWS, static_cast<int>(gb.rows), dst_row, out_row, 2 * I, tiles_n1, tab1, n_tiles1, H, tiles_n2, tab2, n_tiles2, st)))
+        return rc;
+    quantize_i8_mapped_kernel<<<P, 256, 0, st>>>(x, H, nullptr, top_k, dst_row, gemm_i8_lane8(type_gu), gemm_i8_act_bytes(type_gu), img1);
+    c.launches++;
+    if ((rc = cuda_check(cudaGetLastError(), "moe quantize launch"))) return rc;
+    // gu and dn stay in activation-row order
+    if ((rc = launch_gemm_i8_jobs(w_gate_up, type_gu, static_cast<long long>(E) * 2 * I, img1, gu, H, 2 * I, tokens, static_cast<int>(gb.groups * tiles_n1), tab1, n_tiles1, out_row, 1, st)))
+        return rc;
+    moe_act_quant_i8_kernel<<<P, 256, 0, st>>>(gu, I, activation, dst_row, gemm_i8_lane8(type_dn), gemm_i8_act_bytes(type_dn), img2, h_out);
+    c.launches++;
+    if ((rc = cuda_check(cudaGetLastError(), "moe_act_quant launch"))) return rc;
+    if ((rc = launch_gemm_i8_jobs(w_down, type_dn, static_cast<long long>(E) * H, img2, dn, I, H, tokens, static_cast<int>(gb.groups * tiles_n2), tab2, n_tiles2, out_row, 1, st)))
+        return rc;
+    return launch_combine(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out, st);
+}
+
+}  // namespace
+
 // cudaFree when a buffer has to grow. For them the scratch of the prefill GEMM
 // (the quantized activations) lives in a fixed array inside the library image instead of a
 // growable cudaMalloc'd buffer.
@@ -1756,6 +1868,11 @@ int launch_moe_unpack(const float* packed, int T, int H, int k, int first, int c
 // address comes from cudaGetSymbolAddress, asked once per device with that device current.
 constexpr size_t NOALLOC_SCRATCH_BYTES = 10u << 20;    // 10 MiB: e.g. M = 512, K = 4096 needs 8.3 MiB
 static __device__ __align__(256) uint8_t g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
+    if (few_per_expert(T * top_k, E)) {
+        const int t1 = gemm_i8_job_tokens(type_gu, H, w_gate_up), t2 = gemm_i8_job_tokens(type_dn, I, w_down);
+        if (t1 && t2)
+            return launch_moe_ffn_i8(x, w_gate_up, w_down, type_gu, type_dn, top_idx, top_w, down_scale, T, top_k, E, H, I, activation, out, h_out, t1 < t2 ? t1 : t2, st);
+    }
 
 namespace {
 uint8_t* g_noalloc_ptr = nullptr;     // device address of g_noalloc_scratch on g_noalloc_dev
