@@ -908,6 +908,140 @@ gemm_w2_sa_kernel(const __grid_constant__ SaMaps maps, const SaParams p, const S
 }  // namespace w2
 
 
+// ---- the same tiles on the warp-level int8 instruction ------------------------------------------------------------
+// Integer block sums of 128 weight rows x up to 128 tokens from mma.sync (super_block in lp_i8.cuh: one super-block of 32 weight
+// rows x 64 tokens per consumer warp), the fp32 scale chain in registers, results, pieces and tables as in the kernels above.
+// Bound by the FP32 pipe: the chain costs 12 cycles of it per 16 x 8 x 32 products, the MMA 8 cycles of the tensor pipe beside
+// it. The two-piece tcgen05 form needs four fp16 products a value and eight fp16 values written per packed one, which its
+// converter warps cannot feed. A producer warp fills three stages of one super-block: the packed rows by one tensor-map tile,
+// the quantized tokens by one bulk copy per eight.
+namespace i8t {
+
+constexpr int STAGES = 3, CONSUMERS = 8, THREADS = (CONSUMERS + 1) * 32;
+constexpr int PARTS = CONSUMERS / 4, NT = (TT / 8 + PARTS - 1) / PARTS;      // consumer warps side by side along the tokens, 8-token tiles of each
+template <uint32_t TYPE> using Geo = i8::GeoWide<TYPE>;
+template <uint32_t TYPE> struct Lay {
+    static constexpr uint32_t RAW = TW * Geo<TYPE>::PITCH, STAGE = RAW + TT / 8 * i8::Geo<TYPE>::ACT_BYTES,
+                              SMEM = 128 + STAGES * STAGE + 16;                        // + read-ahead of the unaligned loads
+};
+
+template <uint32_t TYPE, bool PEERS>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_i8_tile_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t* __restrict__ img, const SaParams p, const SaPeers<PEERS> pe) {
+    using G = Geo<TYPE>;
+    constexpr int PITCH = G::PITCH;
+    extern __shared__ __align__(128) uint8_t smem[];
+    static_assert(Lay<TYPE>::SMEM <= 227 * 1024, "shared memory budget");
+    const uint32_t sbase = smem_u32(smem), stage0 = sbase + 128;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto bar_full = [&](int s) { return sbase + 8 * s; };
+    auto bar_empty = [&](int s) { return sbase + 32 + 8 * s; };
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), CONSUMERS); }
+        fence_barrier_init();
+    }
+    __syncthreads();
+    // the quantized tokens (and a job table) are the kernel's before this one, which this one's launch and set-up overlap
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const Segments sg = segments(p);
+    const int nsb = p.K / 256;
+
+    if (warp == CONSUMERS) {
+        int s = 0, issued = 0;
+        uint32_t phase = 0;
+        bool gave_up = false;
+        for (int seg = 0; seg < sg.n && !gave_up; ++seg) {
+            const TileRef tr = seg_ref(p, sg, seg);
+            const int nt = (tr.nt + 7) >> 3;
+            const uint8_t* act = img + static_cast<size_t>(tr.m0 >> 3) * nsb * G::ACT_BYTES;
+            for (int sb = tr.sb0; sb < tr.sb1; ++sb) {
+                bool free = true;
+                if (issued >= STAGES && lane == 0) free = mbar_wait_bounded(bar_empty(s), phase ^ 1);
+                if (!__shfl_sync(0xffffffffu, free, 0)) { gave_up = true; break; }
+                const uint32_t st = stage0 + s * Lay<TYPE>::STAGE;
+                if (lane == 0) {
+                    mbar_expect_tx(bar_full(s), Lay<TYPE>::RAW + nt * G::ACT_BYTES);
+                    tma_load_2d(st, &wmap, G::first_word(sb), tr.wrow0 + tr.n0, bar_full(s));
+                }
+                __syncwarp();
+                if (lane < nt)
+                    bulk_g2s(st + Lay<TYPE>::RAW + lane * G::ACT_BYTES, act + (static_cast<size_t>(lane) * nsb + sb) * G::ACT_BYTES, G::ACT_BYTES, bar_full(s));
+                ++issued;
+                if (++s == STAGES) { s = 0; phase ^= 1; }
+            }
+        }
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        if (gave_up && lane == 0) report_status(p.err, DEV_TIMEOUT_EMPTY);
+        // the copies in flight land before the CTA gives its shared memory back
+        const int pending = issued < STAGES ? issued : STAGES;
+        for (int k = 0; k < pending; ++k) {
+            if (s == 0) { s = STAGES; phase ^= 1; }
+            --s;
+            if (!mbar_wait_bounded(bar_full(s), phase) && lane == 0) report_status(p.err, DEV_TIMEOUT_DRAIN);
+        }
+        return;
+    }
+
+    const int wm = warp & 3, side = warp >> 2, gq = lane >> 2, tq = lane & 3;
+    int s = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int seg = 0; seg < sg.n && ok; ++seg) {
+        const TileRef tr = seg_ref(p, sg, seg);
+        const int nt = (tr.nt + 7) >> 3, first = nt * side / PARTS;                     // 8-token tiles: of the tile, before this warp's
+        const int live = nt * (side + 1) / PARTS - first;
+        float2 acc[2][NT][2];
+#pragma unroll
+        for (int g = 0; g < 2; ++g)
+#pragma unroll
+            for (int t = 0; t < NT; ++t) acc[g][t][0] = acc[g][t][1] = make_float2(0.f, 0.f);
+        for (int sb = tr.sb0; sb < tr.sb1; ++sb) {
+            if (!mbar_wait_bounded(bar_full(s), phase)) { ok = false; break; }
+            const uint32_t st = stage0 + s * Lay<TYPE>::STAGE;
+            i8::super_block<TYPE, PITCH, 2, NT>(st + (32 * wm + gq) * PITCH + G::offset_in_unit(sb, 0), st + Lay<TYPE>::RAW + first * G::ACT_BYTES, G::ACT_BYTES, lane, live, acc);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_empty(s));
+            if (++s == STAGES) { s = 0; phase ^= 1; }
+        }
+        if (!ok) break;
+        // lane: weight rows gq and gq + 8 of two groups of 16, tokens 2 tq and 2 tq + 1 of every eight
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            if (t >= live) break;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int col = 8 * (first + t) + 2 * tq + e;
+                if (col >= tr.nt) continue;
+                const int row = tr.m0 + col;
+                const float v[4] = {e ? acc[0][t][0].y : acc[0][t][0].x, e ? acc[0][t][1].y : acc[0][t][1].x, e ? acc[1][t][0].y : acc[1][t][0].x, e ? acc[1][t][1].y : acc[1][t][1].x};
+                if (tr.part >= 0) {
+                    float* part = p.y_part + static_cast<size_t>(tr.part) * (TT * TW) + col * TW + 32 * wm + gq;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) part[8 * k] = v[k];
+                    continue;
+                }
+                const int n = tr.n0 + 32 * wm + gq;
+                if constexpr (PEERS) {
+                    for (int r = 0; r < pe.n; ++r)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (n + 8 * k < p.N) pe.y[r][static_cast<size_t>(row) * pe.ld + pe.col0 + n + 8 * k] = v[k];
+                } else {
+                    int orow = p.out_row ? __ldg(p.out_row + row) : row;
+                    if (p.out_identity && orow >= 0) orow = row;
+                    if (orow < 0) continue;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (n + 8 * k < p.N) p.y[static_cast<size_t>(orow) * p.N + n + 8 * k] = v[k];
+                }
+            }
+        }
+    }
+    if (!ok && lane == 0) report_status(p.err, DEV_TIMEOUT_FULL);       // the producer drains the copies
+}
+
+}  // namespace i8t
+
 // ---- activation quantizer ------------------------------------------------------------------
 // One CTA per activation row. The int8 values q and the block scales d are the reference's (Laplace
 // src/matmul_simd.cpp:348-410: d = amax / 127, q = rne(x * (1 / d)), sums from the unclamped integers); what is
@@ -981,6 +1115,8 @@ struct SaOperand {          // operand buffers of one matmul
     float*  g;              // [m_pad / 2][K / 16]: block sums of a pair of rows, interleaved
     float*  inv_s;          // [m_pad]
     int     m_pad;
+    // the int8 kernel's operand instead, in the same place (a third of its size): quantized rows in fragment order (lp_i8.cuh)
+    uint8_t* img() const { return reinterpret_cast<uint8_t*>(a); }
 };
 
 __global__ void __launch_bounds__(256) quantize_sa_kernel(const float* __restrict__ x, int K, SaOperand op) {
@@ -1034,6 +1170,7 @@ __global__ void __launch_bounds__(256) quantize_sa_norm_kernel(const float* __re
 template <bool PEERS>
 __global__ void __launch_bounds__(256) sk_fixup_kernel(const float* __restrict__ part, long long units, int grid, int nsb, int tiles_m,
                                                        int M, int N, float* __restrict__ y, const SaPeers<PEERS> pe) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");        // the pieces are there
     const int t = blockIdx.x;
     const long long ua = static_cast<long long>(t) * nsb, ub = ua + nsb - 1;
     // the CTA that holds unit u is the largest c with sk_start(c) <= u
@@ -1102,11 +1239,88 @@ struct SaLaunch {
     int tiles_m, tiles_n, grid;
     long long sk_units; float* y_part;
     const PeerOut* peers;        // nullptr, or: the result goes to every GPU's buffer
+    bool i8;                     // on the int8 kernel (op.img())
 };
+
+// Which kernel a call's tiles run on. The int8 kernel needs rows that a tensor-map copy can address. Q4_0 and Q8_0 run on it for any
+// number of rows; for Q4_K (one-piece weights) and Q6_K (16-value scales) the tcgen05 kernels overtake it.
+constexpr int I8_TILES_Q4K = 80, I8_TILES_Q6K = 112;
+bool i8_tiles(uint32_t type, int M, int K, const uint8_t* const* ws, int n_mats) {
+    if ((type == LAPLACE_TYPE_Q4_K && M > I8_TILES_Q4K) || (type == LAPLACE_TYPE_Q6_K && M > I8_TILES_Q6K)) return false;
+    for (int i = 0; i < n_mats; ++i)
+        if (reinterpret_cast<uintptr_t>(ws[i]) & 15) return false;
+    return row_bytes(type, K) % 16 == 0;
+}
+
+// A launch that may overlap the end of the kernel before it in the stream: the kernel waits (griddepcontrol.wait) before it
+// touches what that one reads or writes.
+template <class K, class... A>
+int launch_early(K* kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
+    return cuda_check(cudaLaunchKernelEx(&cfg, kernel, args...), "kernel launch");
+}
+
+template <uint32_t TYPE>
+int launch_i8_tiles(const CUtensorMap& map, const SaLaunch& L, const SaParams& p, const SaPeers<true>& pe, cudaStream_t st) {
+    using namespace i8t;
+    static bool configured = false;
+    if (!configured) {
+        cudaError_t e = cudaFuncSetAttribute(gemm_i8_tile_kernel<TYPE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Lay<TYPE>::SMEM));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_i8_tile_kernel<TYPE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Lay<TYPE>::SMEM));
+        if (e != cudaSuccess) return cuda_check(e, "cudaFuncSetAttribute gemm_i8_tile");
+        configured = true;
+    }
+    const uint8_t* img = L.op.img();
+    return L.peers ? launch_early(gemm_i8_tile_kernel<TYPE, true>, dim3(L.grid), i8t::THREADS, Lay<TYPE>::SMEM, st, map, img, p, pe)
+                   : launch_early(gemm_i8_tile_kernel<TYPE, false>, dim3(L.grid), i8t::THREADS, Lay<TYPE>::SMEM, st, map, img, p, SaPeers<false>{});
+}
+int run_i8_kernel(const SaLaunch& L, const SaParams& p, const SaPeers<true>& pe, cudaStream_t st) {
+    const uint64_t rb = row_bytes(L.type, L.K);
+    int pitch;
+    switch (L.type) {
+        case LAPLACE_TYPE_Q4_K: pitch = i8t::Geo<LAPLACE_TYPE_Q4_K>::PITCH; break;
+        case LAPLACE_TYPE_Q4_0: pitch = i8t::Geo<LAPLACE_TYPE_Q4_0>::PITCH; break;
+        case LAPLACE_TYPE_Q8_0: pitch = i8t::Geo<LAPLACE_TYPE_Q8_0>::PITCH; break;
+        default: pitch = i8t::Geo<LAPLACE_TYPE_Q6_K>::PITCH; break;
+    }
+    CUtensorMap map;
+    if (!make_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, L.w, rb / 4, static_cast<uint64_t>(L.w_rows), rb, pitch / 4, TW, CU_TENSOR_MAP_SWIZZLE_NONE, "weights"))
+        return LAPLACE_ERR_CUDA;
+    int rc;
+    switch (L.type) {
+        case LAPLACE_TYPE_Q4_K: rc = launch_i8_tiles<LAPLACE_TYPE_Q4_K>(map, L, p, pe, st); break;
+        case LAPLACE_TYPE_Q4_0: rc = launch_i8_tiles<LAPLACE_TYPE_Q4_0>(map, L, p, pe, st); break;
+        case LAPLACE_TYPE_Q8_0: rc = launch_i8_tiles<LAPLACE_TYPE_Q8_0>(map, L, p, pe, st); break;
+        case LAPLACE_TYPE_Q6_K: rc = launch_i8_tiles<LAPLACE_TYPE_Q6_K>(map, L, p, pe, st); break;
+        default: return LAPLACE_UNSUPPORTED;
+    }
+    if (rc) return rc;
+    ctx().launches++;
+    ctx().last_path = 2;
+    return cuda_check(cudaGetLastError(), "gemm_i8_tile launch");
+}
 
 int run_sa_kernel(const SaLaunch& L, cudaStream_t st) {
     Context& c = ctx();
     const int K = L.K;
+    SaParams p{};
+    p.w = L.w; p.rb = static_cast<uint32_t>(row_bytes(L.type, K));
+    p.y = L.y; p.inv_s = L.op.inv_s; p.err = c.d_err;
+    p.M = L.M; p.N = L.N; p.K = K; p.m_pad = L.op.m_pad;
+    p.tiles_m = L.tiles_m; p.tiles_n = L.tiles_n;
+    p.tile_tab = L.tile_tab; p.n_tiles_dev = L.n_tiles_dev; p.out_row = L.out_row; p.out_identity = L.out_identity;
+    p.sk_units = L.sk_units; p.y_part = L.y_part;
+    SaPeers<true> pe{};
+    if (L.peers) {
+        for (int r = 0; r < L.peers->world; ++r) pe.y[r] = L.peers->y[r];
+        pe.n = L.peers->world; pe.ld = L.peers->ld; pe.col0 = L.peers->col0;
+    }
+    if (L.peers && (L.out_row || L.tile_tab)) return fail(LAPLACE_ERR_STATE, "gemm_sa: the peer-store form takes a plain dense call");
+    if (L.i8) return run_i8_kernel(L, p, pe, st);
     SaMaps maps;
     for (int bk = 0; bk < 4; ++bk) {
         if (!make_map_2d(&maps.a[bk], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, L.op.a, static_cast<uint64_t>(K), 2ull * L.op.m_pad,
@@ -1122,18 +1336,6 @@ int run_sa_kernel(const SaLaunch& L, cudaStream_t st) {
             return LAPLACE_ERR_CUDA;
     } else {
         maps.w = maps.a[0];      // not used by the two-piece kernels (they copy weight rows by address)
-    }
-    SaParams p{};
-    p.w = L.w; p.rb = static_cast<uint32_t>(rb);
-    p.y = L.y; p.inv_s = L.op.inv_s; p.err = c.d_err;
-    p.M = L.M; p.N = L.N; p.K = K; p.m_pad = L.op.m_pad;
-    p.tiles_m = L.tiles_m; p.tiles_n = L.tiles_n;
-    p.tile_tab = L.tile_tab; p.n_tiles_dev = L.n_tiles_dev; p.out_row = L.out_row; p.out_identity = L.out_identity;
-    p.sk_units = L.sk_units; p.y_part = L.y_part;
-    SaPeers<true> pe{};
-    if (L.peers) {
-        for (int r = 0; r < L.peers->world; ++r) pe.y[r] = L.peers->y[r];
-        pe.n = L.peers->world; pe.ld = L.peers->ld; pe.col0 = L.peers->col0;
     }
     const SaPeers<false> none{};
     static bool configured = false;
@@ -1151,7 +1353,6 @@ int run_sa_kernel(const SaLaunch& L, cudaStream_t st) {
         if (e != cudaSuccess) return cuda_check(e, "cudaFuncSetAttribute gemm_sa");
         configured = true;
     }
-    if (L.peers && (L.out_row || L.tile_tab)) return fail(LAPLACE_ERR_STATE, "gemm_sa: the peer-store form takes a plain dense call");
     const bool peers = L.peers != nullptr;
     switch (L.type) {
         case LAPLACE_TYPE_Q4_K:
@@ -1200,6 +1401,7 @@ SplitPlan plan_split(int M, int K, int N, bool allow) {
 
 }  // namespace
 
+Scratch& gemm_scratch() { return g_scratch; }
 void release_gemm_sa_scratch() { g_scratch.release(); }
 
 bool gemm_sa_supports(uint32_t type, int M, int K, int N) {
@@ -1236,19 +1438,27 @@ int check_args(const float* x, const uint8_t* w, uint32_t type, int M, int K, in
     return LAPLACE_OK;
 }
 
+// The quantized (optionally normalised) rows as the operand of the kernel that the call runs on.
+int launch_operand(bool i8, const float* x, const float* norm_w, float eps, float* x_norm_out, uint32_t type, int M, int K, const SaOperand& op, cudaStream_t st) {
+    if (i8) return launch_quantize_i8(x, norm_w, eps, x_norm_out, type, M, K, op.img(), st);
+    if (norm_w) quantize_sa_norm_kernel<<<M, 256, 0, st>>>(x, norm_w, eps, x_norm_out, K, op);
+    else quantize_sa_kernel<<<M, 256, 0, st>>>(x, K, op);
+    ctx().launches++;
+    return cuda_check(cudaGetLastError(), "quantize_sa launch");
+}
+
 // Quantizes x into `scratch` (device memory of at least pl.total() bytes, 256-byte aligned) and runs the kernel.
-int gemm_sa_on_scratch(uint8_t* scratch, const SaPlan& pl, const float* x, const uint8_t* w, uint32_t type, float* y, int M, int K, int N,
+int gemm_sa_on_scratch(uint8_t* scratch, const SaPlan& pl, bool i8, const float* x, const uint8_t* w, uint32_t type, float* y, int M, int K, int N,
                        cudaStream_t st, const PeerOut* peers = nullptr) {
     Context& c = ctx();
     int rc;
     uint8_t* s = scratch;
     const SaOperand op = carve_operand(s, pl.m_pad, K);
     if (x) {                          // nullptr: the operand is in place already (several matrices share one input)
-        quantize_sa_kernel<<<M, 256, 0, st>>>(x, K, op);
-        c.launches++;
-        if ((rc = cuda_check(cudaGetLastError(), "quantize_sa launch"))) return rc;
+        if ((rc = launch_operand(i8, x, nullptr, 0.f, nullptr, type, M, K, op, st))) return rc;
     }
     SaLaunch L{};
+    L.i8 = i8;
     L.w = w; L.type = type; L.y = y; L.M = M; L.K = K; L.N = N; L.w_rows = N; L.op = op;
     L.tiles_m = pl.tiles_m; L.tiles_n = pl.tiles_n;
     L.sk_units = pl.sp.units;
@@ -1262,12 +1472,12 @@ int gemm_sa_on_scratch(uint8_t* scratch, const SaPlan& pl, const float* x, const
             SaPeers<true> pe{};
             for (int r = 0; r < peers->world; ++r) pe.y[r] = peers->y[r];
             pe.n = peers->world; pe.ld = peers->ld; pe.col0 = peers->col0;
-            sk_fixup_kernel<true><<<fg, 256, 0, st>>>(L.y_part, pl.sp.units, pl.sp.grid, K / 256, pl.tiles_m, M, N, nullptr, pe);
+            rc = launch_early(sk_fixup_kernel<true>, fg, 256, 0, st, L.y_part, pl.sp.units, pl.sp.grid, K / 256, pl.tiles_m, M, N, static_cast<float*>(nullptr), pe);
         } else {
-            sk_fixup_kernel<false><<<fg, 256, 0, st>>>(L.y_part, pl.sp.units, pl.sp.grid, K / 256, pl.tiles_m, M, N, y, SaPeers<false>{});
+            rc = launch_early(sk_fixup_kernel<false>, fg, 256, 0, st, L.y_part, pl.sp.units, pl.sp.grid, K / 256, pl.tiles_m, M, N, y, SaPeers<false>{});
         }
         c.launches++;
-        return cuda_check(cudaGetLastError(), "sk_fixup launch");
+        return rc;
     }
     return LAPLACE_OK;
 }
@@ -1280,7 +1490,7 @@ int launch_gemm_sa(const float* x, const uint8_t* w, uint32_t type, float* y, in
     if (rc) return rc;
     const SaPlan pl = plan_sa(M, K, N, true);
     if ((rc = g_scratch.ensure(pl.total(), st))) return rc;
-    return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, x, w, type, y, M, K, N, st);
+    return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, i8_tiles(type, M, K, &w, 1), x, w, type, y, M, K, N, st);
 }
 
 // Several matrices of one type and K against the same input rows (q / k / v, gate / up of src/arch_llama.cpp:475-499): the
@@ -1298,16 +1508,14 @@ int launch_gemm_sa_multi(const float* x, const float* norm_w, float eps, float* 
         return fail(LAPLACE_ERR_ARG, "gemm_multi: the norm weights (and the optional output) must be 16-byte aligned");
     if ((rc = g_scratch.ensure(need, st))) return rc;
     uint8_t* scratch = static_cast<uint8_t*>(g_scratch.p);
+    const bool i8 = i8_tiles(type, M, K, ws, n_mats);
     {
         uint8_t* s = scratch;
         const SaOperand op = carve_operand(s, plan_sa(M, K, ns[0], true).m_pad, K);
-        if (norm_w) quantize_sa_norm_kernel<<<M, 256, 0, st>>>(x, norm_w, eps, x_norm_out, K, op);
-        else quantize_sa_kernel<<<M, 256, 0, st>>>(x, K, op);
-        ctx().launches++;
-        if ((rc = cuda_check(cudaGetLastError(), "quantize_sa launch"))) return rc;
+        if ((rc = launch_operand(i8, x, norm_w, eps, x_norm_out, type, M, K, op, st))) return rc;
     }
     for (int i = 0; i < n_mats; ++i)
-        if ((rc = gemm_sa_on_scratch(scratch, plan_sa(M, K, ns[i], true), nullptr, ws[i], type, ys[i], M, K, ns[i], st))) return rc;
+        if ((rc = gemm_sa_on_scratch(scratch, plan_sa(M, K, ns[i], true), i8, nullptr, ws[i], type, ys[i], M, K, ns[i], st))) return rc;
     return LAPLACE_OK;
 }
 
@@ -1319,7 +1527,7 @@ int launch_gemm_sa_peers(const float* x, const uint8_t* w, uint32_t type, const 
     if (rc) return rc;
     const SaPlan pl = plan_sa(M, K, N, true);
     if ((rc = g_scratch.ensure(pl.total(), st))) return rc;
-    return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, x, w, type, nullptr, M, K, N, st, &po);
+    return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, i8_tiles(type, M, K, &w, 1), x, w, type, nullptr, M, K, N, st, &po);
 }
 
 // The same call on scratch memory the caller owns (`cap` bytes at `scratch`, 256-byte aligned); nothing is
@@ -1333,7 +1541,7 @@ int launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const 
     if (pl.total() > cap) pl = plan_sa(M, K, N, false);
     if (pl.total() > cap)
         return fail(LAPLACE_ERR_LIMIT, "gemm: M=%d K=%d needs %zu bytes of scratch, the caller's area holds %zu", M, K, pl.total(), cap);
-    return gemm_sa_on_scratch(scratch, pl, x, w, type, y, M, K, N, st);
+    return gemm_sa_on_scratch(scratch, pl, i8_tiles(type, M, K, &w, 1), x, w, type, y, M, K, N, st);
 }
 
 
@@ -1446,6 +1654,32 @@ __global__ void __launch_bounds__(256) moe_act_quant_sa_kernel(const float* __re
                     op.g + static_cast<size_t>(r >> 1) * (I / 16), r & 1, op.inv_s + r);
 }
 
+// The same two steps for the int8 kernel: rows in its fragment order (lp_i8.cuh).
+__global__ void __launch_bounds__(256) quantize_i8_mapped_kernel(const float* __restrict__ x, int K, const int* __restrict__ src_rows, int src_div,
+                                                                 const int* __restrict__ dst_rows, int lane8, uint32_t act_bytes, uint8_t* __restrict__ img) {
+    const int p = blockIdx.x;
+    const int dr = __ldg(dst_rows + p);
+    if (dr < 0) return;
+    const float* xr = x + static_cast<size_t>(src_rows ? __ldg(src_rows + p) : p / src_div) * K;
+    i8::quantize_row_i8([&](int b, int t8) { return __ldg(reinterpret_cast<const float4*>(xr + b * 32) + t8); }, K, lane8, act_bytes,
+                        img + static_cast<size_t>(dr >> 3) * (K / 256) * act_bytes, dr & 7);
+}
+__global__ void __launch_bounds__(256) moe_act_quant_i8_kernel(const float* __restrict__ gu, int I, int activation, const int* __restrict__ dst_rows,
+                                                               int lane8, uint32_t act_bytes, uint8_t* __restrict__ img, float* __restrict__ h_out) {
+    const int p = blockIdx.x;
+    const int r = __ldg(dst_rows + p);
+    if (r < 0) return;
+    const float* row = gu + static_cast<size_t>(r) * (2 * I);
+    i8::quantize_row_i8([&](int b, int t8) {
+        const float4 g = __ldg(reinterpret_cast<const float4*>(row + b * 32) + t8);
+        const float4 u = __ldg(reinterpret_cast<const float4*>(row + I + b * 32) + t8);
+        const float4 h = activation == 1 ? make_float4(act_geglu(g.x, u.x), act_geglu(g.y, u.y), act_geglu(g.z, u.z), act_geglu(g.w, u.w))
+                                         : make_float4(act_swiglu(g.x, u.x), act_swiglu(g.y, u.y), act_swiglu(g.z, u.z), act_swiglu(g.w, u.w));
+        if (h_out) reinterpret_cast<float4*>(h_out + static_cast<size_t>(p) * I + b * 32)[t8] = h;
+        return h;
+    }, I, lane8, act_bytes, img + static_cast<size_t>(r >> 3) * (I / 256) * act_bytes, r & 7);
+}
+
 // out[t][:] = sum over the token's live pairs, in slot order, of top_w[t][j] * dn[row of pair][:]
 // (the reference's weight of pair j is top_w[j] * down_scale[expert], src/arch_gemma4.cpp:634-638; down_scale may be null)
 __global__ void __launch_bounds__(256) moe_combine_sa_kernel(const float* __restrict__ dn, const int* __restrict__ dst_row,
@@ -1505,11 +1739,49 @@ void release_moe_sa_scratch() { g_moe_scratch.release(); }
 
 bool moe_sa_supports(uint32_t type, int K, int N) { return gemm_sa_supports(type, 9, K, N); }
 
+namespace {
+
+// A few tokens per expert: the int8 kernel, which costs in proportion to the tokens, else the tcgen05 kernels, which cost the
+// same up to 32 tokens and little more up to 128.
+constexpr int I8_PAIRS_PER_EXPERT = 32;
+bool few_per_expert(int P, int E) { return P <= I8_PAIRS_PER_EXPERT * static_cast<long long>(E < P ? E : P); }
+
+size_t image_bytes(uint32_t type, size_t rows, int K) { return align256((rows + 7) / 8 * (K / 256) * gemm_i8_act_bytes(type)); }
+
+int launch_moe_grouped_i8(const float* x, const uint8_t* w, uint32_t type, const int* pair_expert, const int* pair_row, int P, int E, float* y, int K, int N,
+                          int tokens, cudaStream_t st) {
+    Context& c = ctx();
+    const int tiles_n = (N + I8_JOB_ROWS - 1) / I8_JOB_ROWS;
+    const GroupBounds gb = group_bounds(P, E, tokens);
+    const size_t pair_bytes = align256(sizeof(int) * static_cast<size_t>(P)), out_bytes = align256(sizeof(int) * gb.rows);
+    const size_t tab_bytes = align256(sizeof(int4) * gb.groups * tiles_n), img_bytes = image_bytes(type, gb.rows, K);
+    int rc;
+    if ((rc = g_moe_scratch.ensure(img_bytes + pair_bytes + out_bytes + tab_bytes + 256, st))) return rc;
+    uint8_t* s = static_cast<uint8_t*>(g_moe_scratch.p);
+    uint8_t* img = s;                               s += img_bytes;
+    int* dst_row = reinterpret_cast<int*>(s);       s += pair_bytes;
+    int* out_row = reinterpret_cast<int*>(s);       s += out_bytes;
+    int4* tab = reinterpret_cast<int4*>(s);         s += tab_bytes;
+    int* n_tiles = reinterpret_cast<int*>(s);
+    if ((rc = launch_plan(pair_expert, P, E, 8, tokens, I8_JOB_ROWS, static_cast<int>(gb.rows), dst_row, out_row, N, tiles_n, tab, n_tiles, 0, 0, nullptr, nullptr, st)))
+        return rc;
+    quantize_i8_mapped_kernel<<<P, 256, 0, st>>>(x, K, pair_row, 1, dst_row, gemm_i8_lane8(type), gemm_i8_act_bytes(type), img);
+    c.launches++;
+    if ((rc = cuda_check(cudaGetLastError(), "moe quantize launch"))) return rc;
+    rc = launch_gemm_i8_jobs(w, type, static_cast<long long>(E) * N, img, y, K, N, tokens, static_cast<int>(gb.groups * tiles_n), tab, n_tiles, out_row, 0, st);
+    if (rc == LAPLACE_OK) c.last_path = 3;
+    return rc;
+}
+
+}  // namespace
+
 int launch_moe_grouped_sa(const float* x, const uint8_t* w, uint32_t type, const int* pair_expert, const int* pair_row,
                           int P, int E, float* y, int K, int N, cudaStream_t st) {
     if (!moe_sa_supports(type, K, N)) return LAPLACE_UNSUPPORTED;
     if ((reinterpret_cast<uintptr_t>(w) & (type == LAPLACE_TYPE_Q4_K ? 15 : 1)) || (reinterpret_cast<uintptr_t>(x) & 15))
         return fail(LAPLACE_ERR_ARG, "moe_grouped: x (16 bytes) or w (16 bytes for Q4_K, else 2) is misaligned on the device");
+    if (few_per_expert(P, E))
+        if (const int tokens = gemm_i8_job_tokens(type, K, w)) return launch_moe_grouped_i8(x, w, type, pair_expert, pair_row, P, E, y, K, N, tokens, st);
     Context& c = ctx();
     const int tiles_n = (N + TW - 1) / TW;
     const GroupBounds gb = group_bounds(P, E);
@@ -1538,6 +1810,61 @@ int launch_moe_grouped_sa(const float* x, const uint8_t* w, uint32_t type, const
     return rc;
 }
 
+namespace {
+
+int launch_combine(const float* dn, const int* dst_row, const float* top_w, const int* top_idx, const float* down_scale, int T, int top_k, int H, float* out,
+                   cudaStream_t st) {
+    Context& c = ctx();
+    const long long total4 = static_cast<long long>(T) * (H / 4);
+    long long blocks = (total4 + 255) / 256;
+    if (blocks > static_cast<long long>(c.sm_count) * 8) blocks = static_cast<long long>(c.sm_count) * 8;
+    moe_combine_sa_kernel<<<static_cast<int>(blocks < 1 ? 1 : blocks), 256, 0, st>>>(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out);
+    c.launches++;
+    c.last_path = 4;
+    return cuda_check(cudaGetLastError(), "moe_combine launch");
+}
+
+int launch_moe_ffn_i8(const float* x, const uint8_t* w_gate_up, const uint8_t* w_down, uint32_t type_gu, uint32_t type_dn, const int* top_idx, const float* top_w,
+                      const float* down_scale, int T, int top_k, int E, int H, int I, int activation, float* out, float* h_out, int tokens, cudaStream_t st) {
+    Context& c = ctx();
+    const int P = T * top_k;
+    const int tiles_n1 = (2 * I + I8_JOB_ROWS - 1) / I8_JOB_ROWS, tiles_n2 = (H + I8_JOB_ROWS - 1) / I8_JOB_ROWS;
+    const GroupBounds gb = group_bounds(P, E, tokens);
+    const size_t pair_bytes = align256(sizeof(int) * static_cast<size_t>(P)), out_bytes = align256(sizeof(int) * gb.rows);
+    const size_t tab1_bytes = align256(sizeof(int4) * gb.groups * tiles_n1), tab2_bytes = align256(sizeof(int4) * gb.groups * tiles_n2);
+    const size_t gu_bytes = align256(gb.rows * 2 * I * sizeof(float)), dn_bytes = align256(gb.rows * H * sizeof(float));
+    const size_t img1_bytes = image_bytes(type_gu, gb.rows, H), img2_bytes = image_bytes(type_dn, gb.rows, I);
+    int rc;
+    if ((rc = g_moe_scratch.ensure(img1_bytes + img2_bytes + pair_bytes + out_bytes + tab1_bytes + tab2_bytes + gu_bytes + dn_bytes + 256, st))) return rc;
+    uint8_t* s = static_cast<uint8_t*>(g_moe_scratch.p);
+    uint8_t* img1 = s;                              s += img1_bytes;
+    uint8_t* img2 = s;                              s += img2_bytes;
+    int* dst_row = reinterpret_cast<int*>(s);       s += pair_bytes;
+    int* out_row = reinterpret_cast<int*>(s);       s += out_bytes;
+    int4* tab1 = reinterpret_cast<int4*>(s);        s += tab1_bytes;
+    int4* tab2 = reinterpret_cast<int4*>(s);        s += tab2_bytes;
+    float* gu = reinterpret_cast<float*>(s);        s += gu_bytes;
+    float* dn = reinterpret_cast<float*>(s);        s += dn_bytes;
+    int* n_tiles1 = reinterpret_cast<int*>(s);
+    int* n_tiles2 = n_tiles1 + 1;
+    if ((rc = launch_plan(top_idx, P, E, 8, tokens, I8_JOB_ROWS, static_cast<int>(gb.rows), dst_row, out_row, 2 * I, tiles_n1, tab1, n_tiles1, H, tiles_n2, tab2, n_tiles2, st)))
+        return rc;
+    quantize_i8_mapped_kernel<<<P, 256, 0, st>>>(x, H, nullptr, top_k, dst_row, gemm_i8_lane8(type_gu), gemm_i8_act_bytes(type_gu), img1);
+    c.launches++;
+    if ((rc = cuda_check(cudaGetLastError(), "moe quantize launch"))) return rc;
+    // gu and dn stay in activation-row order
+    if ((rc = launch_gemm_i8_jobs(w_gate_up, type_gu, static_cast<long long>(E) * 2 * I, img1, gu, H, 2 * I, tokens, static_cast<int>(gb.groups * tiles_n1), tab1, n_tiles1, out_row, 1, st)))
+        return rc;
+    moe_act_quant_i8_kernel<<<P, 256, 0, st>>>(gu, I, activation, dst_row, gemm_i8_lane8(type_dn), gemm_i8_act_bytes(type_dn), img2, h_out);
+    c.launches++;
+    if ((rc = cuda_check(cudaGetLastError(), "moe_act_quant launch"))) return rc;
+    if ((rc = launch_gemm_i8_jobs(w_down, type_dn, static_cast<long long>(E) * H, img2, dn, I, H, tokens, static_cast<int>(gb.groups * tiles_n2), tab2, n_tiles2, out_row, 1, st)))
+        return rc;
+    return launch_combine(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out, st);
+}
+
+}  // namespace
+
 int launch_moe_ffn_sa(const float* x, const uint8_t* w_gate_up, const uint8_t* w_down, uint32_t type_gu, uint32_t type_dn,
                       const int* top_idx, const float* top_w, const float* down_scale, int T, int top_k, int E, int H, int I,
                       int activation, float* out, float* h_out, cudaStream_t st) {
@@ -1547,6 +1874,11 @@ int launch_moe_ffn_sa(const float* x, const uint8_t* w_gate_up, const uint8_t* w
         (reinterpret_cast<uintptr_t>(w_down) & (type_dn == LAPLACE_TYPE_Q4_K ? 15 : 1)) ||
         (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(out) & 15))
         return fail(LAPLACE_ERR_ARG, "moe_ffn: x, out (16 bytes) or the weights (16 bytes for Q4_K, else 2) are misaligned on the device");
+    if (few_per_expert(T * top_k, E)) {
+        const int t1 = gemm_i8_job_tokens(type_gu, H, w_gate_up), t2 = gemm_i8_job_tokens(type_dn, I, w_down);
+        if (t1 && t2)
+            return launch_moe_ffn_i8(x, w_gate_up, w_down, type_gu, type_dn, top_idx, top_w, down_scale, T, top_k, E, H, I, activation, out, h_out, t1 < t2 ? t1 : t2, st);
+    }
     Context& c = ctx();
     const int P = T * top_k;
     const int tiles_n1 = (2 * I + TW - 1) / TW, tiles_n2 = (H + TW - 1) / TW;
@@ -1617,6 +1949,7 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(const float
     extern __shared__ float probs[];
     const int lane = threadIdx.x & 31, t = blockIdx.x * ROUTE_WARPS + (threadIdx.x >> 5);
     if (t >= T) return;
+    constexpr unsigned ALL = 0xffffffffu;
     const float* l = logits + static_cast<size_t>(t) * E;
     float* p = probs + (threadIdx.x >> 5) * p_ld;
     // running maximum with a strict comparison, started at l[0]: values that are not numbers lose every comparison
@@ -1648,32 +1981,6 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(const float
     for (int k = 0; k < top_k; ++k) {
         float best_p = -1.0f;
         int best = 0x7fffffff;
-// The same two steps for the int8 kernel: rows in its fragment order (lp_i8.cuh).
-__global__ void __launch_bounds__(256) quantize_i8_mapped_kernel(const float* __restrict__ x, int K, const int* __restrict__ src_rows, int src_div,
-                                                                 const int* __restrict__ dst_rows, int lane8, uint32_t act_bytes, uint8_t* __restrict__ img) {
-    const int p = blockIdx.x;
-    const int dr = __ldg(dst_rows + p);
-    if (dr < 0) return;
-    const float* xr = x + static_cast<size_t>(src_rows ? __ldg(src_rows + p) : p / src_div) * K;
-    i8::quantize_row_i8([&](int b, int t8) { return __ldg(reinterpret_cast<const float4*>(xr + b * 32) + t8); }, K, lane8, act_bytes,
-                        img + static_cast<size_t>(dr >> 3) * (K / 256) * act_bytes, dr & 7);
-}
-__global__ void __launch_bounds__(256) moe_act_quant_i8_kernel(const float* __restrict__ gu, int I, int activation, const int* __restrict__ dst_rows,
-                                                               int lane8, uint32_t act_bytes, uint8_t* __restrict__ img, float* __restrict__ h_out) {
-    const int p = blockIdx.x;
-    const int r = __ldg(dst_rows + p);
-    if (r < 0) return;
-    const float* row = gu + static_cast<size_t>(r) * (2 * I);
-    i8::quantize_row_i8([&](int b, int t8) {
-        const float4 g = __ldg(reinterpret_cast<const float4*>(row + b * 32) + t8);
-        const float4 u = __ldg(reinterpret_cast<const float4*>(row + I + b * 32) + t8);
-        const float4 h = activation == 1 ? make_float4(act_geglu(g.x, u.x), act_geglu(g.y, u.y), act_geglu(g.z, u.z), act_geglu(g.w, u.w))
-                                         : make_float4(act_swiglu(g.x, u.x), act_swiglu(g.y, u.y), act_swiglu(g.z, u.z), act_swiglu(g.w, u.w));
-        if (h_out) reinterpret_cast<float4*>(h_out + static_cast<size_t>(p) * I + b * 32)[t8] = h;
-        return h;
-    }, I, lane8, act_bytes, img + static_cast<size_t>(r >> 3) * (I / 256) * act_bytes, r & 7);
-}
-
         for (int e = lane; e < E; e += 32) {
             const float v = p_ld ? p[e] : __fdiv_rn(expf(__fsub_rn(__ldg(l + e), maxl)), suml);
             if ((v < last_p || (v == last_p && e > last_e)) && v > best_p) { best = e; best_p = v; }
@@ -1686,6 +1993,7 @@ __global__ void __launch_bounds__(256) moe_act_quant_i8_kernel(const float* __re
         }
         if (lane == 0) { ti[k] = best; tw[k] = best_p; }
         wsum = __fadd_rn(wsum, best_p);
+        last_p = best_p; last_e = best;
     }
     __syncwarp();
     for (int k = lane; k < top_k; k += 32) tw[k] = __fdiv_rn(tw[k], wsum);
@@ -1733,49 +2041,11 @@ __global__ void moe_unpack_kernel(const float* __restrict__ packed, int T, int H
         if (c < H) x[static_cast<long long>(t) * H + c] = v;
         else if (c < H + k) {
             const int e = __float_as_int(v) - first;
-namespace {
-
-// A few tokens per expert: the int8 kernel, which costs in proportion to the tokens, else the tcgen05 kernels, which cost the
-// same up to 32 tokens and little more up to 128.
-constexpr int I8_PAIRS_PER_EXPERT = 32;
-bool few_per_expert(int P, int E) { return P <= I8_PAIRS_PER_EXPERT * static_cast<long long>(E < P ? E : P); }
-
-size_t image_bytes(uint32_t type, size_t rows, int K) { return align256((rows + 7) / 8 * (K / 256) * gemm_i8_act_bytes(type)); }
-
-int launch_moe_grouped_i8(const float* x, const uint8_t* w, uint32_t type, const int* pair_expert, const int* pair_row, int P, int E, float* y, int K, int N,
-                          int tokens, cudaStream_t st) {
-    Context& c = ctx();
-    const int tiles_n = (N + I8_JOB_ROWS - 1) / I8_JOB_ROWS;
-    const GroupBounds gb = group_bounds(P, E, tokens);
-    const size_t pair_bytes = align256(sizeof(int) * static_cast<size_t>(P)), out_bytes = align256(sizeof(int) * gb.rows);
-    const size_t tab_bytes = align256(sizeof(int4) * gb.groups * tiles_n), img_bytes = image_bytes(type, gb.rows, K);
-    int rc;
-    if ((rc = g_moe_scratch.ensure(img_bytes + pair_bytes + out_bytes + tab_bytes + 256, st))) return rc;
-    uint8_t* s = static_cast<uint8_t*>(g_moe_scratch.p);
-    uint8_t* img = s;                               s += img_bytes;
-    int* dst_row = reinterpret_cast<int*>(s);       s += pair_bytes;
-    int* out_row = reinterpret_cast<int*>(s);       s += out_bytes;
-    int4* tab = reinterpret_cast<int4*>(s);         s += tab_bytes;
-    int* n_tiles = reinterpret_cast<int*>(s);
-    if ((rc = launch_plan(pair_expert, P, E, 8, tokens, I8_JOB_ROWS, static_cast<int>(gb.rows), dst_row, out_row, N, tiles_n, tab, n_tiles, 0, 0, nullptr, nullptr, st)))
-        return rc;
-    quantize_i8_mapped_kernel<<<P, 256, 0, st>>>(x, K, pair_row, 1, dst_row, gemm_i8_lane8(type), gemm_i8_act_bytes(type), img);
-    c.launches++;
-    if ((rc = cuda_check(cudaGetLastError(), "moe quantize launch"))) return rc;
-    rc = launch_gemm_i8_jobs(w, type, static_cast<long long>(E) * N, img, y, K, N, tokens, static_cast<int>(gb.groups * tiles_n), tab, n_tiles, out_row, 0, st);
-    if (rc == LAPLACE_OK) c.last_path = 3;
-    return rc;
-}
-
-}  // namespace
-
             idx_local[t * k + (c - H)] = (e >= 0 && e < count) ? e : -1;
         } else wts[t * k + (c - H - k)] = v;
     }
 }
 
-    if (few_per_expert(P, E))
-        if (const int tokens = gemm_i8_job_tokens(type, K, w)) return launch_moe_grouped_i8(x, w, type, pair_expert, pair_row, P, E, y, K, N, tokens, st);
 }  // namespace
 
 int launch_moe_pack(const float* x, const int* idx, const float* wts, int T, int H, int k, float* packed, cudaStream_t st) {
@@ -1804,61 +2074,6 @@ int launch_moe_unpack(const float* packed, int T, int H, int k, int first, int c
 // path: a serving process that has handed all free HBM to its own pools (KV cache,
 // activations), so that cudaMalloc would fail or fragment them, and latency-bound loops that
 // cannot take the allocator's locks or the implicit device synchronisation that comes with
-namespace {
-
-int launch_combine(const float* dn, const int* dst_row, const float* top_w, const int* top_idx, const float* down_scale, int T, int top_k, int H, float* out,
-                   cudaStream_t st) {
-    Context& c = ctx();
-    const long long total4 = static_cast<long long>(T) * (H / 4);
-    long long blocks = (total4 + 255) / 256;
-    if (blocks > static_cast<long long>(c.sm_count) * 8) blocks = static_cast<long long>(c.sm_count) * 8;
-    moe_combine_sa_kernel<<<static_cast<int>(blocks < 1 ? 1 : blocks), 256, 0, st>>>(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out);
-    c.launches++;
-    c.last_path = 4;
-    return cuda_check(cudaGetLastError(), "moe_combine launch");
-}
-
-int launch_moe_ffn_i8(const float* x, const uint8_t* w_gate_up, const uint8_t* w_down, uint32_t type_gu, uint32_t type_dn, const int* top_idx, const float* top_w,
-                      const float* down_scale, int T, int top_k, int E, int H, int I, int activation, float* out, float* h_out, int tokens, cudaStream_t st) {
-    Context& c = ctx();
-    const int P = T * top_k;
-    const int tiles_n1 = (2 * I + I8_JOB_ROWS - 1) / I8_JOB_ROWS, tiles_n2 = (H + I8_JOB_ROWS - 1) / I8_JOB_ROWS;
-    const GroupBounds gb = group_bounds(P, E, tokens);
-    const size_t pair_bytes = align256(sizeof(int) * static_cast<size_t>(P)), out_bytes = align256(sizeof(int) * gb.rows);
-    const size_t tab1_bytes = align256(sizeof(int4) * gb.groups * tiles_n1), tab2_bytes = align256(sizeof(int4) * gb.groups * tiles_n2);
-    const size_t gu_bytes = align256(gb.rows * 2 * I * sizeof(float)), dn_bytes = align256(gb.rows * H * sizeof(float));
-    const size_t img1_bytes = image_bytes(type_gu, gb.rows, H), img2_bytes = image_bytes(type_dn, gb.rows, I);
-    int rc;
-    if ((rc = g_moe_scratch.ensure(img1_bytes + img2_bytes + pair_bytes + out_bytes + tab1_bytes + tab2_bytes + gu_bytes + dn_bytes + 256, st))) return rc;
-    uint8_t* s = static_cast<uint8_t*>(g_moe_scratch.p);
-    uint8_t* img1 = s;                              s += img1_bytes;
-    uint8_t* img2 = s;                              s += img2_bytes;
-    int* dst_row = reinterpret_cast<int*>(s);       s += pair_bytes;
-    int* out_row = reinterpret_cast<int*>(s);       s += out_bytes;
-    int4* tab1 = reinterpret_cast<int4*>(s);        s += tab1_bytes;
-    int4* tab2 = reinterpret_cast<int4*>(s);        s += tab2_bytes;
-    float* gu = reinterpret_cast<float*>(s);        s += gu_bytes;
-    float* dn = reinterpret_cast<float*>(s);        s += dn_bytes;
-    int* n_tiles1 = reinterpret_cast<int*>(s);
-    int* n_tiles2 = n_tiles1 + 1;
-    if ((rc = launch_plan(top_idx, P, E, 8, tokens, I8_JOB_ROWS, static_cast<int>(gb.rows), dst_row, out_row, 2 * I, tiles_n1, tab1, n_tiles1, H, tiles_n2, tab2, n_tiles2, st)))
-        return rc;
-    quantize_i8_mapped_kernel<<<P, 256, 0, st>>>(x, H, nullptr, top_k, dst_row, gemm_i8_lane8(type_gu), gemm_i8_act_bytes(type_gu), img1);
-    c.launches++;
-    if ((rc = cuda_check(cudaGetLastError(), "moe quantize launch"))) return rc;
-    // gu and dn stay in activation-row order
-    if ((rc = launch_gemm_i8_jobs(w_gate_up, type_gu, static_cast<long long>(E) * 2 * I, img1, gu, H, 2 * I, tokens, static_cast<int>(gb.groups * tiles_n1), tab1, n_tiles1, out_row, 1, st)))
-        return rc;
-    moe_act_quant_i8_kernel<<<P, 256, 0, st>>>(gu, I, activation, dst_row, gemm_i8_lane8(type_dn), gemm_i8_act_bytes(type_dn), img2, h_out);
-    c.launches++;
-    if ((rc = cuda_check(cudaGetLastError(), "moe_act_quant launch"))) return rc;
-    if ((rc = launch_gemm_i8_jobs(w_down, type_dn, static_cast<long long>(E) * H, img2, dn, I, H, tokens, static_cast<int>(gb.groups * tiles_n2), tab2, n_tiles2, out_row, 1, st)))
-        return rc;
-    return launch_combine(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out, st);
-}
-
-}  // namespace
-
 // cudaFree when a buffer has to grow. For them the scratch of the prefill GEMM
 // (the quantized activations) lives in a fixed array inside the library image instead of a
 // growable cudaMalloc'd buffer.
@@ -1868,11 +2083,6 @@ int launch_moe_ffn_i8(const float* x, const uint8_t* w_gate_up, const uint8_t* w
 // address comes from cudaGetSymbolAddress, asked once per device with that device current.
 constexpr size_t NOALLOC_SCRATCH_BYTES = 10u << 20;    // 10 MiB: e.g. M = 512, K = 4096 needs 8.3 MiB
 static __device__ __align__(256) uint8_t g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
-    if (few_per_expert(T * top_k, E)) {
-        const int t1 = gemm_i8_job_tokens(type_gu, H, w_gate_up), t2 = gemm_i8_job_tokens(type_dn, I, w_down);
-        if (t1 && t2)
-            return launch_moe_ffn_i8(x, w_gate_up, w_down, type_gu, type_dn, top_idx, top_w, down_scale, T, top_k, E, H, I, activation, out, h_out, t1 < t2 ? t1 : t2, st);
-    }
 
 namespace {
 uint8_t* g_noalloc_ptr = nullptr;     // device address of g_noalloc_scratch on g_noalloc_dev
@@ -1908,5 +2118,3 @@ extern "C" int laplace_cuda_gemm_noalloc_dev(const float* x, const uint8_t* w, u
     return launch_gemm_sa_prealloc(g_noalloc_ptr, NOALLOC_SCRATCH_BYTES, x, w, type, y, M, K, N,
                                    stream ? static_cast<cudaStream_t>(stream) : c.stream);
 }
-    constexpr unsigned ALL = 0xffffffffu;
-        last_p = best_p; last_e = best;
