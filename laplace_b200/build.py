@@ -1,4 +1,4 @@
-"""Builds liblaplace_cuda.so (sm_100a only) next to this file with nvcc.
+"""Builds liblaplace_cuda.so (sm_100a only) and _native.so, its torch binding, next to this file.
 
 The shared library is the product; Python only loads it through ctypes. The
 build is a plain nvcc invocation per source so that it works without a GPU
@@ -16,6 +16,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 ROOT = PKG.parent
 LIB = PKG / "liblaplace_cuda.so"
+NATIVE = PKG / "_native.so"
 
 SOURCES = ["lp_api.cu", "lp_gemv.cu", "lp_quantize.cu", "lp_gemm_sa.cu", "lp_peak.cu", "lp_gguf.cu", "lp_types.cu", "lp_gemm_i8.cu"]
 
@@ -72,7 +73,26 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     if force or jobs or _stale(LIB, objs):
         cmd = [nvcc, "-shared", "-o", str(LIB), *map(str, objs), "-gencode", "arch=compute_100a,code=sm_100a"]
         run(cmd)
+    build_native(force)
     return LIB
+
+
+def build_native(force: bool = False) -> Path:
+    """The host side of the calls on torch tensors (lp_torch.cpp): a CPython module against torch's own headers."""
+    src = CSRC / "lp_torch.cpp"
+    if force or _stale(NATIVE, [src, ROOT / "include" / "laplace_cuda.h"]):
+        import sysconfig
+
+        import torch
+        t = Path(torch.__file__).resolve().parent
+        cuda = Path(_nvcc()).resolve().parent.parent if os.path.sep in _nvcc() else Path("/usr/local/cuda")
+        cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *(f"-I{d}" for d in (ROOT / "include", t / "include", t / "include" / "torch" / "csrc" / "api" / "include", cuda / "include", sysconfig.get_path("include"))),
+               str(src), "-o", str(NATIVE), f"-L{t / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{t / 'lib'}"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError("the torch binding failed to build:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+    return NATIVE
 
 
 if __name__ == "__main__":

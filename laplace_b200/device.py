@@ -6,6 +6,8 @@ current CUDA stream to the ``*_dev`` entry points of include/laplace_cuda.h.
 """
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import torch
 
@@ -14,17 +16,22 @@ from .ggml import any_row_bytes, blocksums_per_row, row_bytes
 from .matmul import LaplaceCudaError, _check
 
 _ready_on = None
+_native = None                # the calls' host side in native code (csrc/lp_torch.cpp), bound with the library
 
 
 def lib(device: int | None = None):
     """Loads the library and binds it to ``device`` (default: torch's current device)."""
-    global _ready_on
+    global _ready_on, _native
     L = _lib.load()
     if not torch.cuda.is_available():
         raise LaplaceCudaError(-3, "no CUDA device visible to this process; the library has no CPU path")
     dev = torch.cuda.current_device() if device is None else device
     if _ready_on is None:
         _check(L, L.laplace_cuda_init(dev))
+        from . import _native as n
+        n.bind(dev, *(ctypes.cast(getattr(L, "laplace_cuda_" + f), ctypes.c_void_p).value
+                      for f in ("gemm_dev", "gemm_multi_dev", "moe_gemv_dev", "lm_head_dev", "moe_route_dev", "moe_ffn_dev")))
+        _native = n
         _ready_on = dev
         from . import matmul as _m
         _m._initialised = True
@@ -49,6 +56,9 @@ def upload_weights(w: np.ndarray) -> torch.Tensor:
 
 
 def gemm(x: torch.Tensor, w: torch.Tensor, t: int, M: int, K: int, N: int, y: torch.Tensor | None = None) -> torch.Tensor:
+    r = _native and _native.gemm(x, w, t, M, K, N, y)
+    if r is not None:
+        return r
     L = lib()
     assert x.dtype == torch.float32 and x.is_cuda and x.is_contiguous() and x.numel() >= M * K
     assert w.dtype == torch.uint8 and w.is_cuda and w.numel() >= N * any_row_bytes(t, K)
@@ -62,6 +72,9 @@ def gemm_multi(x: torch.Tensor, ws, t: int, M: int, K: int, Ns, norm_weight: tor
                want_x_norm: bool = False):
     """Several matrices of one type against the same (optionally RMS-normalised) activation rows in one launch
     (laplace_cuda_gemm_multi_dev). Returns the list of outputs, and the normalised rows when asked for."""
+    r = _native.gemm_multi(x, ws, t, M, K, Ns, norm_weight, eps) if _native and not want_x_norm else None
+    if r is not None:
+        return r
     L = lib()
     assert x.dtype == torch.float32 and x.is_cuda and x.is_contiguous() and len(ws) == len(Ns)
     ys = [torch.empty((M, n), dtype=torch.float32, device=x.device) for n in Ns]
@@ -74,6 +87,9 @@ def gemm_multi(x: torch.Tensor, ws, t: int, M: int, K: int, Ns, norm_weight: tor
 
 def moe_gemv(x: torch.Tensor, w: torch.Tensor, t: int, expert_idx: torch.Tensor, K: int, N: int,
              per_expert_x: bool, y: torch.Tensor | None = None) -> torch.Tensor:
+    r = _native and _native.moe_gemv(x, w, t, expert_idx, K, N, per_expert_x, y)
+    if r is not None:
+        return r
     L = lib()
     n = expert_idx.numel()
     assert expert_idx.dtype == torch.int32 and expert_idx.is_cuda
@@ -123,6 +139,10 @@ def moe_ffn(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, t_ga
             down_scale: torch.Tensor | None = None) -> torch.Tensor:
     """The fused expert FFN (laplace_cuda_moe_ffn_dev): out[t] = sum over the experts of token t that live here of
     top_w * down(act(gate_up(x[t]))). Raises for types the grouped kernels do not take."""
+    r = _native.moe_ffn(x, w_gate_up, w_down, t_gate_up, t_down, top_idx, top_w, n_experts_total, hidden, inter, activation) if (
+        _native and out is None and h_out is None and down_scale is None) else None
+    if r is not None:
+        return r
     L = lib()
     T, k = top_idx.shape
     assert top_idx.dtype == torch.int32 and top_idx.is_cuda and top_idx.is_contiguous()
@@ -140,6 +160,9 @@ def moe_ffn(x: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, t_ga
 
 def moe_route(logits: torch.Tensor, top_k: int):
     """Softmax, top-k by repeated argmax and renormalisation of router logits [T, E] (laplace_cuda_moe_route_dev)."""
+    r = _native and _native.moe_route(logits, top_k)
+    if r is not None:
+        return r
     L = lib()
     T, E = logits.shape
     assert logits.dtype == torch.float32 and logits.is_cuda and logits.is_contiguous()
@@ -209,6 +232,9 @@ def embed_rows(w: torch.Tensor, t: int, tokens: torch.Tensor, H: int, vocab: int
 
 def lm_head(x: torch.Tensor, w: torch.Tensor, t: int, M: int, K: int, N: int, softcap: float = 0.0) -> torch.Tensor:
     """matmul_lm_head (src/matmul.cpp:439) plus the optional logit soft-cap (src/model.cpp:399-406)."""
+    r = _native and _native.lm_head(x, w, t, M, K, N, softcap)
+    if r is not None:
+        return r
     y = torch.empty((M, N), dtype=torch.float32, device=x.device)
     L = lib()
     _check(L, L.laplace_cuda_lm_head_dev(x.data_ptr(), w.data_ptr(), int(t), y.data_ptr(), M, K, N, float(softcap), _stream()))
