@@ -129,10 +129,12 @@ __device__ __forceinline__ void add_block(float2 (&acc)[2], const int (&c)[4], f
 }
 __device__ __forceinline__ float2 lo2(const uint4& v) { return make_float2(__uint_as_float(v.x), __uint_as_float(v.y)); }
 __device__ __forceinline__ float2 hi2(const uint4& v) { return make_float2(__uint_as_float(v.z), __uint_as_float(v.w)); }
-// four bytes from a shared address that is only 2-byte aligned (reads the two words around it)
-__device__ __forceinline__ uint32_t lds32_align2(uint32_t addr) {
-    const uint32_t base = addr & ~3u;
-    return __funnelshift_r(lds32(base), lds32(base + 4), (addr & 3u) * 8u);
+// four bytes from a shared address that is 2-byte aligned; MIS = the address modulo 4, known where the code is built
+template <int MIS>
+__device__ __forceinline__ uint32_t lds32_mis(uint32_t addr) {
+    static_assert(MIS == 0 || MIS == 2, "2-byte aligned data");
+    if (MIS == 0) return lds32(addr);
+    return __funnelshift_r(lds32(addr - 2), lds32(addr + 2), 16);
 }
 
 // mn . (sum pieces) of 16 weight rows x 8 activation rows over the eight sub-blocks of a super-block: f for the leading pieces, g
@@ -156,8 +158,9 @@ __device__ __forceinline__ uint32_t min_pair(const uint4& h, int tq) {
 // acc[g][tile][0 / 1] += weight rows gq / gq + 8 of 16-row group g (the lane's: gq = lane / 4) against activation rows 2 tq, 2 tq + 1
 // of every tile, for tiles 0 .. live - 1. `row` = shared address of row gq's super-block in the first group; row gq + 8 lies 8
 // PITCHes on, the next group 16. `act` = the super-block of the first tile, tiles `act_stride` apart.
-template <uint32_t TYPE, int PITCH, int MT, int NT>
-__device__ __forceinline__ void super_block(uint32_t row, uint32_t act, uint32_t act_stride, int lane, int live, float2 (&acc)[MT][NT][2]) {
+// MIS = `row` modulo 4 (Q6_K: 2 for odd super-blocks; otherwise 0).
+template <uint32_t TYPE, int PITCH, int MT, int NT, int MIS>
+__device__ __forceinline__ void super_block_at(uint32_t row, uint32_t act, uint32_t act_stride, int lane, int live, float2 (&acc)[MT][NT][2]) {
     const int tq = lane & 3;
     const uint32_t frag = act + lane * 16, dbase = act + 2048 + tq * 16;
     if constexpr (TYPE == LAPLACE_TYPE_Q4_K) {
@@ -224,24 +227,28 @@ __device__ __forceinline__ void super_block(uint32_t row, uint32_t act, uint32_t
         for (int c = 0; c < 4; ++c) {
             uint32_t a[MT][2][4];
             float sc[MT][2][2];                              // [group][block of the pair][row]
+            // quants of an even block (34 or 18 bytes each, the rows 4-byte aligned) lie 2 bytes off a word, those of an odd one on it
+            auto load = [&](auto odd) {
+                constexpr int o = decltype(odd)::value, MIS = o ? 0 : 2;
 #pragma unroll
-            for (int g = 0; g < MT; ++g)
-#pragma unroll
-                for (int o = 0; o < 2; ++o) {
+                for (int g = 0; g < MT; ++g) {
                     const uint32_t ba = row + 16 * g * PITCH + (2 * c + o) * BB, bb = ba + 8 * PITCH;
                     sc[g][o][0] = half_bits_to_float(lds16(ba)); sc[g][o][1] = half_bits_to_float(lds16(bb));
                     if constexpr (TYPE == LAPLACE_TYPE_Q8_0) {
-                        a[g][o][0] = lds32_align2(ba + 2 + 4 * tq); a[g][o][2] = lds32_align2(ba + 18 + 4 * tq);
-                        a[g][o][1] = lds32_align2(bb + 2 + 4 * tq); a[g][o][3] = lds32_align2(bb + 18 + 4 * tq);
+                        a[g][o][0] = lds32_mis<MIS>(ba + 2 + 4 * tq); a[g][o][2] = lds32_mis<MIS>(ba + 18 + 4 * tq);
+                        a[g][o][1] = lds32_mis<MIS>(bb + 2 + 4 * tq); a[g][o][3] = lds32_mis<MIS>(bb + 18 + 4 * tq);
                     } else {
                         // byte l: value l in the low nibble, l + 16 in the high one; the signed byte 16 * (nibble - 8) is the
                         // nibble on top with its first bit flipped
-                        const uint32_t wa = lds32_align2(ba + 2 + 4 * tq), wb = lds32_align2(bb + 2 + 4 * tq);
+                        const uint32_t wa = lds32_mis<MIS>(ba + 2 + 4 * tq), wb = lds32_mis<MIS>(bb + 2 + 4 * tq);
                         a[g][o][0] = ((wa << 4) & 0xf0f0f0f0u) ^ 0x80808080u; a[g][o][2] = (wa & 0xf0f0f0f0u) ^ 0x80808080u;
                         a[g][o][1] = ((wb << 4) & 0xf0f0f0f0u) ^ 0x80808080u; a[g][o][3] = (wb & 0xf0f0f0f0u) ^ 0x80808080u;
                         sc[g][o][0] *= 0.0625f; sc[g][o][1] *= 0.0625f;
                     }
                 }
+            };
+            load(Tag<0>{});
+            load(Tag<1>{});
 #pragma unroll
             for (int t = 0; t < NT; ++t) {
                 if (t >= live) break;
@@ -280,9 +287,9 @@ __device__ __forceinline__ void super_block(uint32_t row, uint32_t act, uint32_t
 #pragma unroll
                     for (int s = 0; s < 2; ++s) {
                         const uint32_t at = base + 16 * s + 4 * tq;
-                        ql[m][r][s][0] = lds32_align2(at + 64 * h);
-                        ql[m][r][s][1] = lds32_align2(at + 64 * h + 32);
-                        qh[m][r][s] = lds32_align2(at + 128 + 32 * h);
+                        ql[m][r][s][0] = lds32_mis<MIS>(at + 64 * h);
+                        ql[m][r][s][1] = lds32_mis<MIS>(at + 64 * h + 32);
+                        qh[m][r][s] = lds32_mis<MIS>(at + 128 + 32 * h);
                     }
                 }
 #pragma unroll
@@ -324,6 +331,12 @@ __device__ __forceinline__ void super_block(uint32_t row, uint32_t act, uint32_t
             }
         }
     }
+}
+
+template <uint32_t TYPE, int PITCH, int MT, int NT>
+__device__ __forceinline__ void super_block(uint32_t row, uint32_t act, uint32_t act_stride, int lane, int live, float2 (&acc)[MT][NT][2]) {
+    if (TYPE == LAPLACE_TYPE_Q6_K && (row & 2)) super_block_at<TYPE, PITCH, MT, NT, 2>(row, act, act_stride, lane, live, acc);
+    else super_block_at<TYPE, PITCH, MT, NT, 0>(row, act, act_stride, lane, live, acc);
 }
 
 // ---- quantized rows in fragment order, for calls whose CTAs do not quantize themselves -----------------------------------
