@@ -149,6 +149,18 @@ int launch_blocksums_q(const int8_t* q, const uint8_t* w, uint32_t type, int32_t
 // ---- device helpers ---------------------------------------------------------
 #ifdef __CUDACC__
 
+// A launch that may overlap the end of the kernel before it in the stream: the kernel waits (griddepcontrol.wait) before it
+// touches what that one reads or writes.
+template <class K, class... A>
+int launch_early(K* kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
+    return cuda_check(cudaLaunchKernelEx(&cfg, kernel, args...), "kernel launch");
+}
+
 // Records a device-side failure in the status word (host-mapped memory).
 __device__ __forceinline__ void report_status(int* err, int code) {
     *reinterpret_cast<volatile int*>(err) = code;

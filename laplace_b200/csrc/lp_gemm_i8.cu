@@ -453,8 +453,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
 __global__ void __launch_bounds__(256) quantize_i8_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps,
                                                           float* __restrict__ x_norm_out, int K, int lane8, uint32_t act_bytes, uint8_t* __restrict__ img) {
     __shared__ float red[8];
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");       // the matmul's copies of weights may start
     asm volatile("griddepcontrol.wait;" ::: "memory");                    // x is there, and the call before has read the scratch
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");       // the matmul's copies of weights may start (all before this call is done)
     const int m = blockIdx.x;
     const float* xr = x + static_cast<size_t>(m) * K;
     uint8_t* tile = img + static_cast<size_t>(m >> 3) * (K / 256) * act_bytes;
@@ -647,14 +647,8 @@ bool gemm_i8_supports(uint32_t type, int M, int K, const uint8_t* const* ws, int
 int launch_quantize_i8(const float* x, const float* norm_w, float eps, float* x_norm_out, uint32_t type, int M, int K, uint8_t* img, cudaStream_t st) {
     TypeGeo g;
     if (!type_geo(type, g)) return LAPLACE_UNSUPPORTED;
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3(M); cfg.blockDim = dim3(256); cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, quantize_i8_kernel, x, norm_w, eps, x_norm_out, K, g.lane8 ? 1 : 0, static_cast<uint32_t>(g.act_bytes), img);
     ctx().launches++;
-    return cuda_check(e, "quantize_i8 launch");
+    return launch_early(quantize_i8_kernel, dim3(M), 256, 0, st, x, norm_w, eps, x_norm_out, K, g.lane8 ? 1 : 0, static_cast<uint32_t>(g.act_bytes), img);
 }
 
 int launch_gemm_i8(const float* x, const float* norm_w, float eps, float* x_norm_out, const uint8_t* const* ws, float* const* ys,

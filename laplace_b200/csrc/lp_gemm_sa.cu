@@ -1,5 +1,6 @@
-// lp_gemm_sa.cu - prefill GEMM (M >= 9 activation rows) and expert-grouped matmul for Q4_K weights on the
-// 5th-generation tensor cores, "scaled activation" formulation. Replaces gemm_int<dot_row_q4_k_int_neon> of
+// lp_gemm_sa.cu - prefill GEMM and expert-grouped matmul: tiles on the 5th-generation tensor cores in a "scaled activation"
+// formulation (this comment, Q4_K; namespace w2 for the two-piece types) or on the warp-level int8 instruction (namespace i8t);
+// which call takes which is said at i8_tiles. Up to 32 activation rows, and experts with few tokens, run in lp_gemm_i8.cu. Replaces gemm_int<dot_row_q4_k_int_neon> of
 // Laplace's NEON back-end (src/matmul_simd.cpp:226-283, 432-455) for large M.
 //
 // The reference's result for one (token m, weight row n) is
@@ -1257,18 +1258,6 @@ bool i8_tiles(uint32_t type, int M, int K, const uint8_t* const* ws, int n_mats)
     return row_bytes(type, K) % 16 == 0;
 }
 
-// A launch that may overlap the end of the kernel before it in the stream: the kernel waits (griddepcontrol.wait) before it
-// touches what that one reads or writes.
-template <class K, class... A>
-int launch_early(K* kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = grid; cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 1;
-    return cuda_check(cudaLaunchKernelEx(&cfg, kernel, args...), "kernel launch");
-}
-
 template <uint32_t TYPE>
 int launch_i8_tiles(const CUtensorMap& map, const SaLaunch& L, const SaParams& p, const SaPeers<true>& pe, cudaStream_t st) {
     using namespace i8t;
@@ -1587,16 +1576,27 @@ __global__ void __launch_bounds__(1024) moe_plan_sa_kernel(const int* __restrict
         dst_row[p] = slot;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
+        // running sums over the experts, 32 at a time
+        const int lane = threadIdx.x;
         int rows = 0, groups = 0;
-        for (int e = 0; e < E; ++e) {
-            base[e] = rows;
-            grp0[e] = groups;
-            rows += (cnt[e] + pad - 1) / pad * pad;
-            groups += (cnt[e] + group - 1) / group;
+        for (int at = 0; at < E; at += 32) {
+            const int e = at + lane, c = e < E ? cnt[e] : 0;
+            const int own_r = (c + pad - 1) / pad * pad, own_g = (c + group - 1) / group;
+            int r = own_r, g = own_g;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int pr = __shfl_up_sync(0xffffffffu, r, o), pg = __shfl_up_sync(0xffffffffu, g, o);
+                if (lane >= o) { r += pr; g += pg; }
+            }
+            if (e < E) { base[e] = rows + r - own_r; grp0[e] = groups + g - own_g; }
+            rows += __shfl_sync(0xffffffffu, r, 31);
+            groups += __shfl_sync(0xffffffffu, g, 31);
         }
-        *n_tiles1 = groups * tiles_n1;
-        if (tiles_n2) *n_tiles2 = groups * tiles_n2;
+        if (lane == 0) {
+            *n_tiles1 = groups * tiles_n1;
+            if (tiles_n2) *n_tiles2 = groups * tiles_n2;
+        }
     }
     __syncthreads();
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
@@ -1662,6 +1662,7 @@ __global__ void __launch_bounds__(256) moe_act_quant_sa_kernel(const float* __re
 // The same two steps for the int8 kernel: rows in its fragment order (lp_i8.cuh).
 __global__ void __launch_bounds__(256) quantize_i8_mapped_kernel(const float* __restrict__ x, int K, const int* __restrict__ src_rows, int src_div,
                                                                  const int* __restrict__ dst_rows, int lane8, uint32_t act_bytes, uint8_t* __restrict__ img) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");        // launched to overlap the kernel before
     const int p = blockIdx.x;
     const int dr = __ldg(dst_rows + p);
     if (dr < 0) return;
@@ -1671,6 +1672,7 @@ __global__ void __launch_bounds__(256) quantize_i8_mapped_kernel(const float* __
 }
 __global__ void __launch_bounds__(256) moe_act_quant_i8_kernel(const float* __restrict__ gu, int I, int activation, const int* __restrict__ dst_rows,
                                                                int lane8, uint32_t act_bytes, uint8_t* __restrict__ img, float* __restrict__ h_out) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");        // launched to overlap the kernel before
     const int p = blockIdx.x;
     const int r = __ldg(dst_rows + p);
     if (r < 0) return;
@@ -1691,6 +1693,7 @@ __global__ void __launch_bounds__(256) moe_combine_sa_kernel(const float* __rest
                                                              const float* __restrict__ top_w, const int* __restrict__ top_idx,
                                                              const float* __restrict__ down_scale, int T, int top_k, int H,
                                                              float* __restrict__ out) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");        // launched to overlap the kernel before
     const int h4 = H / 4;
     const long long total = static_cast<long long>(T) * h4;
     for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -1770,9 +1773,9 @@ int launch_moe_grouped_i8(const float* x, const uint8_t* w, uint32_t type, const
     int* n_tiles = reinterpret_cast<int*>(s);
     if ((rc = launch_plan(pair_expert, P, E, 8, tokens, I8_JOB_ROWS, static_cast<int>(gb.rows), dst_row, out_row, N, tiles_n, tab, n_tiles, 0, 0, nullptr, nullptr, st)))
         return rc;
-    quantize_i8_mapped_kernel<<<P, 256, 0, st>>>(x, K, pair_row, 1, dst_row, gemm_i8_lane8(type), gemm_i8_act_bytes(type), img);
+    rc = launch_early(quantize_i8_mapped_kernel, dim3(P), 256, 0, st, x, K, pair_row, 1, static_cast<const int*>(dst_row), static_cast<int>(gemm_i8_lane8(type)), gemm_i8_act_bytes(type), img);
     c.launches++;
-    if ((rc = cuda_check(cudaGetLastError(), "moe quantize launch"))) return rc;
+    if (rc) return rc;
     rc = launch_gemm_i8_jobs(w, type, static_cast<long long>(E) * N, img, y, K, N, tokens, static_cast<int>(gb.groups * tiles_n), tab, n_tiles, out_row, 0, st);
     if (rc == LAPLACE_OK) c.last_path = 3;
     return rc;
@@ -1823,10 +1826,10 @@ int launch_combine(const float* dn, const int* dst_row, const float* top_w, cons
     const long long total4 = static_cast<long long>(T) * (H / 4);
     long long blocks = (total4 + 255) / 256;
     if (blocks > static_cast<long long>(c.sm_count) * 8) blocks = static_cast<long long>(c.sm_count) * 8;
-    moe_combine_sa_kernel<<<static_cast<int>(blocks < 1 ? 1 : blocks), 256, 0, st>>>(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out);
+    const int rc = launch_early(moe_combine_sa_kernel, dim3(static_cast<unsigned>(blocks < 1 ? 1 : blocks)), 256, 0, st, dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out);
     c.launches++;
     c.last_path = 4;
-    return cuda_check(cudaGetLastError(), "moe_combine launch");
+    return rc;
 }
 
 int launch_moe_ffn_i8(const float* x, const uint8_t* w_gate_up, const uint8_t* w_down, uint32_t type_gu, uint32_t type_dn, const int* top_idx, const float* top_w,
@@ -1854,15 +1857,17 @@ int launch_moe_ffn_i8(const float* x, const uint8_t* w_gate_up, const uint8_t* w
     int* n_tiles2 = n_tiles1 + 1;
     if ((rc = launch_plan(top_idx, P, E, 8, tokens, I8_JOB_ROWS, static_cast<int>(gb.rows), dst_row, out_row, 2 * I, tiles_n1, tab1, n_tiles1, H, tiles_n2, tab2, n_tiles2, st)))
         return rc;
-    quantize_i8_mapped_kernel<<<P, 256, 0, st>>>(x, H, nullptr, top_k, dst_row, gemm_i8_lane8(type_gu), gemm_i8_act_bytes(type_gu), img1);
+    rc = launch_early(quantize_i8_mapped_kernel, dim3(P), 256, 0, st, x, H, static_cast<const int*>(nullptr), top_k, static_cast<const int*>(dst_row),
+                      static_cast<int>(gemm_i8_lane8(type_gu)), gemm_i8_act_bytes(type_gu), img1);
     c.launches++;
-    if ((rc = cuda_check(cudaGetLastError(), "moe quantize launch"))) return rc;
+    if (rc) return rc;
     // gu and dn stay in activation-row order
     if ((rc = launch_gemm_i8_jobs(w_gate_up, type_gu, static_cast<long long>(E) * 2 * I, img1, gu, H, 2 * I, tokens, static_cast<int>(gb.groups * tiles_n1), tab1, n_tiles1, out_row, 1, st)))
         return rc;
-    moe_act_quant_i8_kernel<<<P, 256, 0, st>>>(gu, I, activation, dst_row, gemm_i8_lane8(type_dn), gemm_i8_act_bytes(type_dn), img2, h_out);
+    rc = launch_early(moe_act_quant_i8_kernel, dim3(P), 256, 0, st, static_cast<const float*>(gu), I, activation, static_cast<const int*>(dst_row),
+                      static_cast<int>(gemm_i8_lane8(type_dn)), gemm_i8_act_bytes(type_dn), img2, h_out);
     c.launches++;
-    if ((rc = cuda_check(cudaGetLastError(), "moe_act_quant launch"))) return rc;
+    if (rc) return rc;
     if ((rc = launch_gemm_i8_jobs(w_down, type_dn, static_cast<long long>(E) * H, img2, dn, I, H, tokens, static_cast<int>(gb.groups * tiles_n2), tab2, n_tiles2, out_row, 1, st)))
         return rc;
     return launch_combine(dn, dst_row, top_w, top_idx, down_scale, T, top_k, H, out, st);

@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(256) gemv_f32act_kernel(const float* __restric
 }
 
 __global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ y, long long n, float cap, float inv_cap) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");        // launched to overlap the matmul that makes y
     for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<long long>(gridDim.x) * blockDim.x)
         y[i] = __fmul_rn(tanhf(__fmul_rn(y[i], inv_cap)), cap);
 }
@@ -612,9 +613,8 @@ int launch_softcap(float* y, long long n, float cap, cudaStream_t st) {
     if (!y || n <= 0 || !(cap > 0.0f)) return fail(LAPLACE_ERR_ARG, "softcap: n=%lld cap=%g", n, static_cast<double>(cap));
     long long blocks = (n + 255) / 256;
     if (blocks > static_cast<long long>(ctx().sm_count) * 16) blocks = static_cast<long long>(ctx().sm_count) * 16;
-    softcap_kernel<<<static_cast<int>(blocks), 256, 0, st>>>(y, n, cap, 1.0f / cap);
     ctx().launches++;
-    return cuda_check(cudaGetLastError(), "softcap launch");
+    return launch_early(softcap_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, st, y, n, cap, 1.0f / cap);
 }
 
 }  // namespace lp
