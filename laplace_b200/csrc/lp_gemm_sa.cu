@@ -1749,8 +1749,9 @@ bool moe_sa_supports(uint32_t type, int K, int N) { return gemm_sa_supports(type
 
 namespace {
 
-// A few tokens per expert: the int8 kernel, which costs in proportion to the tokens, else the tcgen05 kernels, which cost the
-// same up to 32 tokens and little more up to 128.
+// Up to 32 pairs per expert on average: the int8 kernel, one pass over an expert's weights (128 experts, hidden 2048, width 768, Q4_K,
+// router included: 16 pairs 168 us against 430, 32 pairs 267 against 515; 32 pairs of 8 Q8_0 experts 50 against 112). Beyond
+// that most experts would take a second pass, while the tcgen05 tiles cost little more up to 128 tokens.
 constexpr int I8_PAIRS_PER_EXPERT = 32;
 bool few_per_expert(int P, int E) { return P <= I8_PAIRS_PER_EXPERT * static_cast<long long>(E < P ? E : P); }
 
