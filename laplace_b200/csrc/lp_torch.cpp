@@ -76,18 +76,26 @@ template <class F>
 PyObject* guarded(F&& f) {
     try {
         return f();
-    } catch (const std::exception&) {        // an allocation that failed, say: the general path meets it again and raises
+    } catch (...) {        // an allocation that failed, a tensor without storage: the general path meets it again and raises
         PyErr_Clear();
         Py_RETURN_NONE;
     }
 }
+// Runs f without the interpreter lock, which is back however f ends. Only the library's own call belongs in f: data_ptr() throws
+// for a tensor without storage (inside torch.vmap, torch.func.grad and the like), so pointers are taken before.
+struct Unlocked {
+    PyThreadState* st = PyEval_SaveThread();
+    Unlocked() = default;
+    Unlocked(const Unlocked&) = delete;
+    Unlocked& operator=(const Unlocked&) = delete;
+    ~Unlocked() { PyEval_RestoreThread(st); }
+};
 template <class F>
 int unlocked(F&& f) {
-    PyThreadState* st = PyEval_SaveThread();
-    const int rc = f();
-    PyEval_RestoreThread(st);
-    return rc;
+    Unlocked lock;
+    return f();
 }
+template <class T> T* ptr(const at::Tensor& t) { return static_cast<T*>(t.data_ptr()); }
 
 // gemm(x, w, type, M, K, N, y or None)
 PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -99,7 +107,11 @@ PyObject* py_gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
             (y && y->numel() < M * N))
             Py_RETURN_NONE;
         const at::Tensor out = y ? *y : fresh({M, N}, at::kFloat);
-        if (unlocked([&] { return g.gemm(static_cast<const float*>(x->data_ptr()), static_cast<const uint8_t*>(w->data_ptr()), type, static_cast<float*>(out.data_ptr()), M, K, N, stream()); }))
+        const auto* px = ptr<const float>(*x);
+        const auto* pw = ptr<const uint8_t>(*w);
+        auto* po = ptr<float>(out);
+        void* st = stream();
+        if (unlocked([&] { return g.gemm(px, pw, type, po, M, K, N, st); }))
             Py_RETURN_NONE;
         if (y) { Py_INCREF(a[6]); return a[6]; }
         return THPVariable_Wrap(out);
@@ -123,9 +135,11 @@ PyObject* py_gemm_multi(PyObject*, PyObject* const* a, Py_ssize_t n) {
             long N;
             if (!tensor(PyList_GET_ITEM(a[1], i), at::kByte, w) || !number(PySequence_Fast_GET_ITEM(a[5], i), N) || !whole_rows(*w, type, K, N)) Py_RETURN_NONE;
             ys[i] = fresh({M, N}, at::kFloat);
-            mats[i] = laplace_cuda_matrix{static_cast<const uint8_t*>(w->data_ptr()), static_cast<float*>(ys[i].data_ptr()), static_cast<int>(N)};
+            mats[i] = laplace_cuda_matrix{ptr<const uint8_t>(*w), ptr<float>(ys[i]), static_cast<int>(N)};
         }
-        if (unlocked([&] { return g.gemm_multi(static_cast<const float*>(x->data_ptr()), norm ? static_cast<const float*>(norm->data_ptr()) : nullptr, static_cast<float>(eps), nullptr, mats, static_cast<int>(count), type, M, K, stream()); }))
+        const auto* px = ptr<const float>(*x), *pn = norm ? ptr<const float>(*norm) : nullptr;
+        void* st = stream();
+        if (unlocked([&] { return g.gemm_multi(px, pn, static_cast<float>(eps), nullptr, mats, static_cast<int>(count), type, M, K, st); }))
             Py_RETURN_NONE;
         PyObject* list = PyList_New(count);
         if (!list) return nullptr;
@@ -151,7 +165,12 @@ PyObject* py_moe_gemv(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const long e = idx->numel();
         if (x->numel() < (per ? e : 1) * K || (y && y->numel() < e * N)) Py_RETURN_NONE;
         const at::Tensor out = y ? *y : fresh({e, N}, at::kFloat);
-        if (unlocked([&] { return g.moe_gemv(static_cast<const float*>(x->data_ptr()), static_cast<const uint8_t*>(w->data_ptr()), type, static_cast<const int*>(idx->data_ptr()), e, static_cast<float*>(out.data_ptr()), K, N, per, stream()); }))
+        const auto* px = ptr<const float>(*x);
+        const auto* pw = ptr<const uint8_t>(*w);
+        const auto* pi = ptr<const int>(*idx);
+        auto* po = ptr<float>(out);
+        void* st = stream();
+        if (unlocked([&] { return g.moe_gemv(px, pw, type, pi, e, po, K, N, per, st); }))
             Py_RETURN_NONE;
         if (y) { Py_INCREF(a[7]); return a[7]; }
         return THPVariable_Wrap(out);
@@ -168,7 +187,11 @@ PyObject* py_lm_head(PyObject*, PyObject* const* a, Py_ssize_t n) {
             !number(a[5], N) || !real(a[6], cap) || x->numel() < M * K || !whole_rows(*w, type, K, N))
             Py_RETURN_NONE;
         const at::Tensor out = fresh({M, N}, at::kFloat);
-        if (unlocked([&] { return g.lm_head(static_cast<const float*>(x->data_ptr()), static_cast<const uint8_t*>(w->data_ptr()), type, static_cast<float*>(out.data_ptr()), M, K, N, static_cast<float>(cap), stream()); }))
+        const auto* px = ptr<const float>(*x);
+        const auto* pw = ptr<const uint8_t>(*w);
+        auto* po = ptr<float>(out);
+        void* st = stream();
+        if (unlocked([&] { return g.lm_head(px, pw, type, po, M, K, N, static_cast<float>(cap), st); }))
             Py_RETURN_NONE;
         return THPVariable_Wrap(out);
     });
@@ -181,7 +204,12 @@ PyObject* py_moe_route(PyObject*, PyObject* const* a, Py_ssize_t n) {
         long k;
         if (n != 2 || !ready() || !tensor(a[0], at::kFloat, l) || l->dim() != 2 || !number(a[1], k)) Py_RETURN_NONE;
         const at::Tensor idx = fresh({l->size(0), k}, at::kInt), wts = fresh({l->size(0), k}, at::kFloat);
-        if (unlocked([&] { return g.moe_route(static_cast<const float*>(l->data_ptr()), l->size(0), l->size(1), k, static_cast<int*>(idx.data_ptr()), static_cast<float*>(wts.data_ptr()), stream()); }))
+        const auto* pl = ptr<const float>(*l);
+        const long T = l->size(0), E = l->size(1);
+        auto* pi = ptr<int>(idx);
+        auto* pw = ptr<float>(wts);
+        void* st = stream();
+        if (unlocked([&] { return g.moe_route(pl, T, E, k, pi, pw, st); }))
             Py_RETURN_NONE;
         return Py_BuildValue("NN", THPVariable_Wrap(idx), THPVariable_Wrap(wts));
     });
@@ -198,7 +226,12 @@ PyObject* py_moe_ffn(PyObject*, PyObject* const* a, Py_ssize_t n) {
             Py_RETURN_NONE;
         const long T = idx->size(0), k = idx->size(1);
         const at::Tensor out = fresh({T, H}, at::kFloat);
-        if (unlocked([&] { return g.moe_ffn(static_cast<const float*>(x->data_ptr()), static_cast<const uint8_t*>(wg->data_ptr()), static_cast<const uint8_t*>(wd->data_ptr()), tg, td, static_cast<const int*>(idx->data_ptr()), static_cast<const float*>(tw->data_ptr()), nullptr, T, k, E, H, I, act, static_cast<float*>(out.data_ptr()), nullptr, stream()); }))
+        const auto* px = ptr<const float>(*x), *pt = ptr<const float>(*tw);
+        const auto* pg = ptr<const uint8_t>(*wg), *pd = ptr<const uint8_t>(*wd);
+        const auto* pi = ptr<const int>(*idx);
+        auto* po = ptr<float>(out);
+        void* st = stream();
+        if (unlocked([&] { return g.moe_ffn(px, pg, pd, tg, td, pi, pt, nullptr, T, k, E, H, I, act, po, nullptr, st); }))
             Py_RETURN_NONE;
         return THPVariable_Wrap(out);
     });

@@ -63,3 +63,38 @@ def test_what_was_refused_is_refused():
     with pytest.raises(LaplaceCudaError):
         device.gemm(torch.zeros(M * K + 1, device="cuda")[1:], w, t, M, K, N)          # x not 16-byte aligned
     device.sync()
+
+
+@pytest.mark.parametrize("transform", ["vmap", "grad", "jvp"])
+@pytest.mark.parametrize("native", [True, False])
+def test_tensors_without_storage_are_refused(transform, native):
+    """Inside a function transform tensors have no storage: every call raises, with the native host side as without it."""
+    import torch
+    from laplace_b200 import device
+    device.lib()
+    t, K, N, E = GGMLType.Q4_K, 256, 8, 2
+    w = torch.zeros(E * 2 * K * 144 + 64, dtype=torch.uint8, device="cuda")
+    idx = torch.zeros((1, 2), dtype=torch.int32, device="cuda")
+    wts = torch.zeros((1, 2), device="cuda")
+    calls = [lambda x: device.gemm(x, w, t, 1, K, N), lambda x: device.gemm_multi(x, [w], t, 1, K, [N]), lambda x: device.moe_gemv(x, w, t, idx[0], K, N, per_expert_x=False),
+             lambda x: device.lm_head(x, w, t, 1, K, N), lambda x: device.moe_route(x.reshape(1, -1), 2), lambda x: device.moe_ffn(x.reshape(1, -1), w, w, t, t, idx, wts, E, K, K)]
+    x = torch.zeros((3, K), device="cuda")
+    kept = device._native
+    try:
+        if not native:
+            device._native = None
+        for call in calls:
+            def f(v):
+                with pytest.raises(RuntimeError, match="data pointer"):
+                    call(v)
+                return v.sum()
+            if transform == "vmap":
+                torch.vmap(f)(x)
+            elif transform == "grad":
+                torch.func.grad(f)(x[0])
+            else:
+                torch.func.jvp(f, (x[0],), (x[0],))
+    finally:
+        device._native = kept
+    assert device.gemm(x, w, t, 3, K, N).shape == (3, N)
+    device.sync()
