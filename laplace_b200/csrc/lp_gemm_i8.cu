@@ -529,6 +529,24 @@ bool plan_dense(uint32_t type, int M, int K, DensePlan& d) {
     return false;
 }
 
+// Rows of a panel that has at most `room` row groups wherever it begins. Rows [a, a + r) that meet b matrices make at most
+// b + (r - b) / 16 groups (every matrix adds one, and one more per 16 further rows), and the fewest rows that meet b matrices are
+// the ones between the first and the last, and two. Little room and many matrices come here (eight matrices, 24 rows, Q4_K, K =
+// 14336: room for eight groups, panels of 112 rows if no matrix has fewer).
+int panel_rows_for(const I8Params& p, int room) {
+    auto most_matrices = [&](int r) {
+        int most = 1;
+        for (int i = 0; i < p.n_mats; ++i)
+            for (int j = i + 1; j < p.n_mats; ++j)
+                if (p.mat_end[j - 1] - p.mat_end[i] + 2 <= r && j - i + 1 > most) most = j - i + 1;
+        return most;
+    };
+    auto fits = [&](int r) { const int b = most_matrices(r); return b + (r - b) / 16 <= room; };
+    int r = 16 * room;
+    while (r > 1 && !fits(r)) r = r > 16 ? (r - 1) / 16 * 16 : r - 1;
+    return fits(r) ? r : 0;
+}
+
 template <uint32_t TYPE, int NT, int C, bool QUANT, bool MOE>
 int launch_as(const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes, size_t smem, cudaStream_t st) {
     auto k = gemm_i8_kernel<TYPE, NT, C, QUANT, MOE>;
@@ -572,7 +590,8 @@ int launch_as(const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes
             const int rows = (p.total_rows + clusters - 1) / clusters, room = static_cast<int>(slab_bytes / (p.kw * 8 * NT * 16 * 4)) / C * C;
             const int round = CW / p.kw;
             if ((rows + 15) / 16 + p.n_mats <= room) p.panel_rows = rows;
-            else p.panel_rows = 16 * (room - p.n_mats >= round ? (room - p.n_mats) / round * round : room - p.n_mats);
+            else if (room - p.n_mats >= round) p.panel_rows = 16 * ((room - p.n_mats) / round * round);
+            else p.panel_rows = panel_rows_for(p, room);
             if (p.panel_rows < 1) return fail(LAPLACE_ERR_STATE, "gemm_i8: internal planning error (no room for partial results)");
             p.slab_groups = room / C;
         }

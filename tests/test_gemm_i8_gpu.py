@@ -60,6 +60,21 @@ def test_matrices_that_share_normalised_rows(oracle, t, M, K, Ns):
         assert np.array_equal(single, y)            # how K is cut does not depend on the rows of a call
 
 
+@pytest.mark.parametrize("t,M,K", [(GGMLType.Q4_K, 16, 11008), (GGMLType.Q4_K, 24, 14336), (GGMLType.Q4_K, 8, 24832), (GGMLType.Q8_0, 24, 8192), (GGMLType.Q6_K, 32, 8192),
+                                   (GGMLType.Q4_0, 32, 11520)])
+def test_eight_matrices_where_partial_results_have_little_room(oracle, t, M, K):
+    """Room for eight row groups in clusters of four and of eight CTAs: panels end inside matrices and hold the ends of several."""
+    Ns = (1500, 1, 700, 16, 5, 1290, 64, 800)
+    ws = [synth.random_blocks(t, K, n, seed=650 + i) for i, n in enumerate(Ns)]
+    x = synth.normal_f32(651, (M, K))
+    ys, _ = _run(t, x, ws, M, K, Ns)
+    for y, w, n in zip(ys, ws, Ns):
+        mass = oracle.gemm(x, w, t, M, K, n, mode=2, threads=THREADS)
+        check_close(y, oracle.gemm(x, w, t, M, K, n, mode=1, threads=THREADS), f"eight matrices {t.name} M={M} K={K} N={n}", mass)
+        (single,), _ = _run(t, x, [w], M, K, [n])
+        assert np.array_equal(single, y)
+
+
 @pytest.mark.parametrize("t", TYPES)
 @pytest.mark.parametrize("M", [5, 20])
 def test_special_rows(oracle, t, M):
