@@ -670,8 +670,10 @@ int launch_quantize_i8(const float* x, const float* norm_w, float eps, float* x_
     return launch_early(quantize_i8_kernel, dim3(M), 256, 0, st, x, norm_w, eps, x_norm_out, K, g.lane8 ? 1 : 0, static_cast<uint32_t>(g.act_bytes), img);
 }
 
+// `scratch`: where more than 8 rows are quantized to (gemm_i8_act_bytes for every 8 rows and 256 values, 16-byte aligned);
+// nullptr: the library's own.
 int launch_gemm_i8(const float* x, const float* norm_w, float eps, float* x_norm_out, const uint8_t* const* ws, float* const* ys,
-                   const int* ns, int n_mats, uint32_t type, int M, int K, cudaStream_t st) {
+                   const int* ns, int n_mats, uint32_t type, int M, int K, cudaStream_t st, uint8_t* scratch) {
     Context& c = ctx();
     DensePlan d;
     TypeGeo g;
@@ -700,8 +702,8 @@ int launch_gemm_i8(const float* x, const float* norm_w, float eps, float* x_norm
     int rc;
     if (!quant) {
         const size_t bytes = static_cast<size_t>(d.nt) * p.nsb * g.act_bytes;
-        if ((rc = gemm_scratch().ensure(bytes, st))) return rc;
-        uint8_t* img = static_cast<uint8_t*>(gemm_scratch().p);
+        if (!scratch && (rc = gemm_scratch().ensure(bytes, st))) return rc;
+        uint8_t* img = scratch ? scratch : static_cast<uint8_t*>(gemm_scratch().p);
         if ((rc = launch_quantize_i8(x, norm_w, eps, x_norm_out, type, M, K, img, st))) return rc;
         p.img = img;
     }

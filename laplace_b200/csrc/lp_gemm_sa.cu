@@ -1524,9 +1524,9 @@ int launch_gemm_sa_peers(const float* x, const uint8_t* w, uint32_t type, const 
     return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, i8_tiles(type, M, K, &w, 1), x, w, type, nullptr, M, K, N, st, &po);
 }
 
-// The same call on scratch memory the caller owns (`cap` bytes at `scratch`, 256-byte aligned); nothing is
-// allocated. The balanced split of launch_gemm_sa is kept when its partial results fit too (the result is then
-// bit-identical to launch_gemm_sa's), otherwise the call runs on whole tiles.
+// laplace_cuda_gemm_dev for more than 8 rows on scratch memory the caller owns (`cap` bytes at `scratch`, 256-byte aligned);
+// nothing is allocated. The same kernel runs as there, and the balanced split of launch_gemm_sa is kept when its partial
+// results fit too (the result is then bit-identical to that call's), otherwise the call runs on whole tiles.
 int launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const uint8_t* w, uint32_t type, float* y,
                             int M, int K, int N, cudaStream_t st) {
     int rc = check_args(x, w, type, M, K, N);
@@ -1535,6 +1535,8 @@ int launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const 
     if (pl.total() > cap) pl = plan_sa(M, K, N, false);
     if (pl.total() > cap)
         return fail(LAPLACE_ERR_LIMIT, "gemm: M=%d K=%d needs %zu bytes of scratch, the caller's area holds %zu", M, K, pl.total(), cap);
+    // a handful of rows: a twelfth of that operand at most, but the limit stays one formula for every row count
+    if (gemm_i8_supports(type, M, K, &w, 1)) return launch_gemm_i8(x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, scratch);
     return gemm_sa_on_scratch(scratch, pl, i8_tiles(type, M, K, &w, 1), x, w, type, y, M, K, N, st);
 }
 
@@ -2124,8 +2126,8 @@ extern "C" int laplace_cuda_gemm_noalloc_dev(const float* x, const uint8_t* w, u
         g_noalloc_ptr = static_cast<uint8_t*>(ptr);
         g_noalloc_dev = c.device;
     }
-    // the same K-split as laplace_cuda_gemm_dev (hence bit-identical results) whenever its partial results fit the
-    // array too; otherwise no split (results then agree to fp32 rounding)
+    // the same kernel as laplace_cuda_gemm_dev and the same K-split (hence bit-identical results) whenever its partial
+    // results fit the array too; otherwise no split (results then agree to fp32 rounding)
     return launch_gemm_sa_prealloc(g_noalloc_ptr, NOALLOC_SCRATCH_BYTES, x, w, type, y, M, K, N,
                                    stream ? static_cast<cudaStream_t>(stream) : c.stream);
 }

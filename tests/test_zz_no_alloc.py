@@ -64,6 +64,18 @@ def test_noalloc_other_plans_and_types(oracle, t, M, K, N):
     check_close(a, oracle.gemm(x, w, t, M, K, N, mode=1, threads=THREADS), f"noalloc vs oracle {t.name} {M}x{K}x{N}")
 
 
+@pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q6_K, GGMLType.Q8_0, GGMLType.Q4_0])
+@pytest.mark.parametrize("M,K,N", [(9, 256, 40), (16, 2048, 130), (24, 14336, 200), (32, 4096, 1024), (33, 2048, 300)])
+def test_noalloc_has_the_bits_of_the_allocating_entry_point(oracle, t, M, K, N):
+    """Both sides of the line between the kernel for a handful of rows and the tiles: the same kernel as in the allocating call."""
+    from laplace_b200 import device
+    w = synth.random_blocks(t, K, N, seed=97)
+    x = synth.normal_f32(98, (M, K))
+    a, b = _call(device.lib(), t, x, w, M, K, N)
+    assert np.array_equal(a, b)
+    check_close(a, oracle.gemm(x, w, t, M, K, N, mode=1, threads=THREADS), f"noalloc {t.name} {M}x{K}x{N}")
+
+
 def test_noalloc_rejects_what_it_cannot_serve():
     import torch
     from laplace_b200 import device
