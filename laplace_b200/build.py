@@ -77,10 +77,25 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIB
 
 
-def build_native(force: bool = False) -> Path:
-    """The host side of the calls on torch tensors (lp_torch.cpp): a CPython module against torch's own headers."""
+def _native_abi() -> str | None:
+    """What _native.so is built against besides its sources: torch's headers and the interpreter. None: torch is not installed."""
+    import sysconfig
+    from importlib import metadata
+    try:
+        return f"torch {metadata.version('torch')}\npython {sysconfig.get_config_var('SOABI')}\n"
+    except metadata.PackageNotFoundError:
+        return None
+
+
+def build_native(force: bool = False) -> Path | None:
+    """The host side of the calls on torch tensors (lp_torch.cpp): a CPython module against torch's own headers. Built again when
+    torch or the interpreter is another one; left out (device.py then makes its calls through ctypes) where torch is not installed."""
     src = CSRC / "lp_torch.cpp"
-    if force or _stale(NATIVE, [src, ROOT / "include" / "laplace_cuda.h"]):
+    abi, stamp = _native_abi(), PKG / "build" / "_native.abi"
+    if abi is None:
+        print("torch is not installed: _native.so is left out, the C library does not need it", file=sys.stderr)
+        return None
+    if force or _stale(NATIVE, [src, ROOT / "include" / "laplace_cuda.h"]) or not stamp.exists() or stamp.read_text() != abi:
         import sysconfig
 
         import torch
@@ -92,6 +107,8 @@ def build_native(force: bool = False) -> Path:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError("the torch binding failed to build:\n" + " ".join(cmd) + "\n" + r.stdout + r.stderr)
+        stamp.parent.mkdir(exist_ok=True)
+        stamp.write_text(abi)
     return NATIVE
 
 

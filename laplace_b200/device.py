@@ -7,6 +7,7 @@ current CUDA stream to the ``*_dev`` entry points of include/laplace_cuda.h.
 from __future__ import annotations
 
 import ctypes
+import warnings
 
 import numpy as np
 import torch
@@ -16,7 +17,7 @@ from .ggml import any_row_bytes, blocksums_per_row, row_bytes
 from .matmul import LaplaceCudaError, _check
 
 _ready_on = None
-_native = None                # the calls' host side in native code (csrc/lp_torch.cpp), bound with the library
+_native = None                # the calls' host side in native code (csrc/lp_torch.cpp), bound with the library; None: ctypes
 
 
 def lib(device: int | None = None):
@@ -28,9 +29,15 @@ def lib(device: int | None = None):
     dev = torch.cuda.current_device() if device is None else device
     if _ready_on is None:
         _check(L, L.laplace_cuda_init(dev))
-        from . import _native as n
-        n.bind(dev, *(ctypes.cast(getattr(L, "laplace_cuda_" + f), ctypes.c_void_p).value
-                      for f in ("gemm_dev", "gemm_multi_dev", "moe_gemv_dev", "lm_head_dev", "moe_route_dev", "moe_ffn_dev")))
+        try:
+            from . import _native as n
+        except ImportError as e:       # not built, or against another torch: the general path makes every call
+            warnings.warn(f"laplace_b200: the native host side of the calls does not load ({e}); every call goes through ctypes, "
+                          "some 10 us slower on the host. `python -m laplace_b200.build` builds it.", RuntimeWarning, stacklevel=2)
+            n = None
+        if n is not None:
+            n.bind(dev, *(ctypes.cast(getattr(L, "laplace_cuda_" + f), ctypes.c_void_p).value
+                          for f in ("gemm_dev", "gemm_multi_dev", "moe_gemv_dev", "lm_head_dev", "moe_route_dev", "moe_ffn_dev")))
         _native = n
         _ready_on = dev
         from . import matmul as _m
