@@ -327,6 +327,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
     int slot = 0;                                       // of this warp's ring, and its barriers' phase
     uint32_t phase = 0;
     const uint32_t ring = ring_of(warp), full0 = bar_full(warp, 0), empty0 = bar_empty(warp, 0);
+    // Up to 8 rows: every super-block is summed on its own, even and odd block pairs apart, and then added, so that no chain of
+    // roundings is longer than a few dozen terms: error against 64 bits at 8 rows, one running sum / this / the dp4a kernel, Q6_K 4096 x
+    // 1024 15.2 / 8.7 / 8.9e-8, 28672 x 1024 27.2 / 14.4 / 15.2e-8, Q8_0 4096 x 14336 11.6 / 8.0 / 8.0e-8. It costs 0.5 % (Q4_K 1.2 %).
+    // More rows are below what the tcgen05 kernels show (4e-7) without it.
+    constexpr int SETS = QUANT ? 2 : 0;
     // one row group: units of super-blocks [s0, s1); `act` = shared address of the activations of super-block s0
     auto run_group = [&](auto nt_tag, int s0, int s1, uint32_t act, uint32_t act_stride, auto& acc) {
         constexpr int NTC = decltype(nt_tag)::value;
@@ -334,9 +339,24 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
             if (!mbar_wait_bounded(full0 + 8 * slot, phase)) { ok = false; return; }
             const uint32_t row = ring + slot * G::UNIT_BYTES + gq * G::PITCH;
 #pragma unroll
-            for (int k = 0; k < G::UNIT_SB; ++k)
-                if (G::UNIT_SB == 1 || sb + k < s1)
-                    super_block<TYPE, G::PITCH, 1, NTC>(row + G::offset_in_unit(sb, k), act + static_cast<uint32_t>(sb - s0 + k) * G::ACT_BYTES, act_stride, lane, NTC, acc);
+            for (int k = 0; k < G::UNIT_SB; ++k) {
+                if (G::UNIT_SB > 1 && sb + k >= s1) break;
+                const uint32_t r = row + G::offset_in_unit(sb, k), a = act + static_cast<uint32_t>(sb - s0 + k) * G::ACT_BYTES;
+                if constexpr (SETS) {
+                    float2 own[SETS][1][NTC][2];
+#pragma unroll
+                    for (int q = 0; q < SETS; ++q)
+#pragma unroll
+                        for (int t = 0; t < NTC; ++t) own[q][0][t][0] = own[q][0][t][1] = make_float2(0.f, 0.f);
+                    super_block<TYPE, G::PITCH, 1, NTC>(r, a, act_stride, lane, NTC, own);
+#pragma unroll
+                    for (int t = 0; t < NTC; ++t)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) acc[0][0][t][h] = __fadd2_rn(acc[0][0][t][h], own[0][0][t][h]);
+                } else {
+                    super_block<TYPE, G::PITCH, 1, NTC>(r, a, act_stride, lane, NTC, acc);
+                }
+            }
             __syncwarp();
             if (lane == 0) mbar_arrive(empty0 + 8 * slot);                   // the slot may be refilled
             if (++slot == p.n_slots) { slot = 0; phase ^= 1; }
@@ -354,9 +374,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
             const uint32_t act = sbase + OFF_ACT + buf * p.act_buf_bytes, act_stride = static_cast<uint32_t>(p.nsb) * G::ACT_BYTES;
             auto tile = [&](auto nt_tag) {
                 constexpr int NTC = decltype(nt_tag)::value;
-                float2 acc[1][NTC][2];
+                float2 acc[1][1][NTC][2];
 #pragma unroll
-                for (int i = 0; i < NTC; ++i) acc[0][i][0] = acc[0][i][1] = make_float2(0.f, 0.f);
+                for (int i = 0; i < NTC; ++i) acc[0][0][i][0] = acc[0][0][i][1] = make_float2(0.f, 0.f);
                 run_group(nt_tag, 0, p.nsb, act, act_stride, acc);
 #pragma unroll
                 for (int i = 0; i < NTC; ++i)
@@ -368,8 +388,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
                         if (orow < 0) continue;
                         if (p.out_identity) orow = t.x + tok;
                         float* y = p.mat_y[0] + static_cast<size_t>(orow) * p.N + row0 + gq;
-                        if (row0 + gq < p.N) y[0] = e ? acc[0][i][0].y : acc[0][i][0].x;
-                        if (row0 + gq + 8 < p.N) y[8] = e ? acc[0][i][1].y : acc[0][i][1].x;
+                        if (row0 + gq < p.N) y[0] = e ? acc[0][0][i][0].y : acc[0][0][i][0].x;
+                        if (row0 + gq + 8 < p.N) y[8] = e ? acc[0][0][i][1].y : acc[0][0][i][1].x;
                     }
             };
             if (row0 < p.N) {
@@ -396,9 +416,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
             if (C > 1 && panel > 0 && !wait_cluster(misc(BAR_SLAB_FREE), (panel - 1) & 1)) ok = false;
             for (int g = gl; g < ng && ok; g += lanes) {
                 const Group gr = panel_group(p, p0, p1, g);
-                float2 acc[1][NT][2];
+                float2 acc[1][1][NT][2];
 #pragma unroll
-                for (int i = 0; i < NT; ++i) acc[0][i][0] = acc[0][i][1] = make_float2(0.f, 0.f);
+                for (int i = 0; i < NT; ++i) acc[0][0][i][0] = acc[0][0][i][1] = make_float2(0.f, 0.f);
                 run_group(Tag<NT>{}, s0, s1, act, act_stride, acc);
                 if constexpr (C == 1) {                          // whole K: straight to y
                     float* y = p.mat_y[gr.mat] + gr.row + gq;
@@ -409,18 +429,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
                         for (int e = 0; e < 2; ++e) {
                             const int tok = 8 * i + 2 * tq + e;
                             if (tok >= p.M) continue;
-                            if (gq < gr.rows) y[static_cast<size_t>(tok) * n] = e ? acc[0][i][0].y : acc[0][i][0].x;
-                            if (gq + 8 < gr.rows) y[static_cast<size_t>(tok) * n + 8] = e ? acc[0][i][1].y : acc[0][i][1].x;
+                            if (gq < gr.rows) y[static_cast<size_t>(tok) * n] = e ? acc[0][0][i][0].y : acc[0][0][i][0].x;
+                            if (gq + 8 < gr.rows) y[static_cast<size_t>(tok) * n + 8] = e ? acc[0][0][i][1].y : acc[0][0][i][1].x;
                         }
                 } else {
                     const int at = ((rank * p.kw + part) * p.slab_groups + g / C) * (8 * NT * 16) + slab_at(2 * tq, gq), at8 = at ^ 8;
                     const uint32_t dst = map_rank(slab + static_cast<uint32_t>(at) * 4, g % C), dst8 = dst + (at8 - at) * 4;
 #pragma unroll
                     for (int i = 0; i < NT; ++i) {
-                        st_remote(dst + (8 * i * 16) * 4, acc[0][i][0].x);
-                        st_remote(dst + (8 * i * 16 + 16) * 4, acc[0][i][0].y);
-                        st_remote(dst8 + (8 * i * 16) * 4, acc[0][i][1].x);
-                        st_remote(dst8 + (8 * i * 16 + 16) * 4, acc[0][i][1].y);
+                        st_remote(dst + (8 * i * 16) * 4, acc[0][0][i][0].x);
+                        st_remote(dst + (8 * i * 16 + 16) * 4, acc[0][0][i][0].y);
+                        st_remote(dst8 + (8 * i * 16) * 4, acc[0][0][i][1].x);
+                        st_remote(dst8 + (8 * i * 16 + 16) * 4, acc[0][0][i][1].y);
                     }
                 }
             }
@@ -434,10 +454,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
                 for (int i = threadIdx.x; i < items; i += CW * 32) {
                     const int row = i & 15, gm = i >> 4, gi = gm / p.M, m = gm - gi * p.M;
                     const float* src = mine + gi * (8 * NT * 16) + slab_at(m, row);
-                    float v = 0.f;
+                    float part[C];                          // of the CTAs, added in pairs
 #pragma unroll
-                    for (int r = 0; r < C; ++r)
-                        for (int k = 0; k < p.kw; ++k) v += src[(r * p.kw + k) * per_src];
+                    for (int r = 0; r < C; ++r) part[r] = p.kw == 2 ? src[2 * r * per_src] + src[(2 * r + 1) * per_src] : src[r * per_src];
+#pragma unroll
+                    for (int o = 1; o < C; o *= 2)
+#pragma unroll
+                        for (int r = 0; r < C; r += 2 * o) part[r] += part[r + o];
+                    const float v = part[0];
                     const Group gr = panel_group(p, p0, p1, gi * C + rank);
                     const int n = p.mat_end[gr.mat] - (gr.mat ? p.mat_end[gr.mat - 1] : 0);
                     if (row < gr.rows) p.mat_y[gr.mat][static_cast<size_t>(m) * n + gr.row + row] = v;

@@ -991,11 +991,11 @@ gemm_i8_tile_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t* __r
         const TileRef tr = seg_ref(p, sg, seg);
         const int nt = (tr.nt + 7) >> 3, first = nt * side / PARTS;                     // 8-token tiles: of the tile, before this warp's
         const int live = nt * (side + 1) / PARTS - first;
-        float2 acc[2][NT][2];
+        float2 acc[1][2][NT][2];
 #pragma unroll
         for (int g = 0; g < 2; ++g)
 #pragma unroll
-            for (int t = 0; t < NT; ++t) acc[g][t][0] = acc[g][t][1] = make_float2(0.f, 0.f);
+            for (int t = 0; t < NT; ++t) acc[0][g][t][0] = acc[0][g][t][1] = make_float2(0.f, 0.f);
         for (int sb = tr.sb0; sb < tr.sb1; ++sb) {
             if (!mbar_wait_bounded(bar_full(s), phase)) { ok = false; break; }
             const uint32_t st = stage0 + s * Lay<TYPE>::STAGE;
@@ -1019,7 +1019,7 @@ gemm_i8_tile_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t* __r
                 const int col = 8 * (first + t) + 2 * tq + e;
                 if (col >= tr.nt) continue;
                 const int row = tr.m0 + col;
-                const float v[4] = {e ? acc[0][t][0].y : acc[0][t][0].x, e ? acc[0][t][1].y : acc[0][t][1].x, e ? acc[1][t][0].y : acc[1][t][0].x, e ? acc[1][t][1].y : acc[1][t][1].x};
+                const float v[4] = {e ? acc[0][0][t][0].y : acc[0][0][t][0].x, e ? acc[0][0][t][1].y : acc[0][0][t][1].x, e ? acc[0][1][t][0].y : acc[0][1][t][0].x, e ? acc[0][1][t][1].y : acc[0][1][t][1].x};
                 if (tr.part >= 0) {
                     float* part = p.y_part + static_cast<size_t>(tr.part) * (TT * TW) + col * TW + 32 * wm + gq;
 #pragma unroll

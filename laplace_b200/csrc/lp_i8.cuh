@@ -155,14 +155,24 @@ __device__ __forceinline__ uint32_t min_pair(const uint4& h, int tq) {
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// acc[g][tile][0 / 1] += weight rows gq / gq + 8 of 16-row group g (the lane's: gq = lane / 4) against activation rows 2 tq, 2 tq + 1
-// of every tile, for tiles 0 .. live - 1. `row` = shared address of row gq's super-block in the first group; row gq + 8 lies 8
+// acc[s][g][tile][0 / 1] stands for weight rows gq / gq + 8 of 16-row group g (the lane's: gq = lane / 4)
+// against activation rows 2 tq, 2 tq + 1 of every tile, for tiles 0 .. live - 1. S = 1: acc[0] += them. S = 2: acc[0] = their sum over
+// the super-block (the caller sets both to zero), the four block pairs in two chains, so that no long chain of roundings arises; Q4_K's
+// min term, as large as the products' sum and mostly taken back by it, comes last. `row` = shared address of row gq's super-block in the first group; row gq + 8 lies 8
 // PITCHes on, the next group 16. `act` = the super-block of the first tile, tiles `act_stride` apart.
 // MIS = `row` modulo 4 (Q6_K: 2 for odd super-blocks; otherwise 0).
-template <uint32_t TYPE, int PITCH, int MT, int NT, int MIS>
-__device__ __forceinline__ void super_block_at(uint32_t row, uint32_t act, uint32_t act_stride, int lane, int live, float2 (&acc)[MT][NT][2]) {
+template <uint32_t TYPE, int PITCH, int MT, int NT, int MIS, int S>
+__device__ __forceinline__ void super_block_at(uint32_t row, uint32_t act, uint32_t act_stride, int lane, int live, float2 (&acc)[S][MT][NT][2]) {
     const int tq = lane & 3;
     const uint32_t frag = act + lane * 16, dbase = act + 2048 + tq * 16;
+    auto join = [&] {                                        // S = 2: the two chains of a super-block
+#pragma unroll
+        for (int g = 0; g < MT; ++g)
+#pragma unroll
+            for (int t = 0; t < NT; ++t)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) acc[0][g][t][h] = __fadd2_rn(acc[0][g][t][h], acc[S - 1][g][t][h]);
+    };
     if constexpr (TYPE == LAPLACE_TYPE_Q4_K) {
         // Scales of sub-blocks tq and tq + 4 of both rows (Laplace src/kernels.h:82-90); the other six come by shuffle. High
         // nibbles stay in place (16 times their value), which the scale of an odd sub-block takes back exactly. The min term
@@ -170,18 +180,33 @@ __device__ __forceinline__ void super_block_at(uint32_t row, uint32_t act, uint3
         // is a contraction over the eight sub-blocks: two small MMAs and one packed multiply-add per row instead of eight.
         float sc[MT][2][2], ndmin[MT][2];
         uint32_t mn[MT][2];
-#pragma unroll
-        for (int g = 0; g < MT; ++g)
-#pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                const uint4 h = lds128(row + (16 * g + 8 * r) * PITCH);
+        auto header = [&](int g, int r, bool scales, bool mins) {
+            const uint4 h = lds128(row + (16 * g + 8 * r) * PITCH);
+            if (scales) {
                 const uint32_t b_lo = (h.y >> (8 * tq)) & 0xff, b_hi = (h.w >> (8 * tq)) & 0xf;
                 const float d = half_bits_to_float(h.x) * ((tq & 1) ? 0.0625f : 1.0f);
                 sc[g][r][0] = d * static_cast<float>(b_lo & 63);
                 sc[g][r][1] = d * static_cast<float>(b_hi | ((b_lo >> 6) << 4));
+            }
+            if (mins) {
                 ndmin[g][r] = -half_bits_to_float(h.x >> 16);
                 mn[g][r] = min_pair(h, tq);
             }
+        };
+        auto min_term = [&](int t) {
+            const uint4 s = lds128(frag + t * act_stride + 2304);
+#pragma unroll
+            for (int g = 0; g < MT; ++g) {
+                float f[4], e[4];
+                mma_mins(f, e, mn[g][0], mn[g][1], s);
+                acc[0][g][t][0] = __ffma2_rn(both(ndmin[g][0]), __fadd2_rn(make_float2(f[0], f[1]), make_float2(e[0], e[1])), acc[0][g][t][0]);
+                acc[0][g][t][1] = __ffma2_rn(both(ndmin[g][1]), __fadd2_rn(make_float2(f[2], f[3]), make_float2(e[2], e[3])), acc[0][g][t][1]);
+            }
+        };
+#pragma unroll
+        for (int g = 0; g < MT; ++g)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) header(g, r, true, S == 1);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             uint2 wa[MT], wb[MT];
@@ -206,19 +231,22 @@ __device__ __forceinline__ void super_block_at(uint32_t row, uint32_t act, uint3
                     int u[4], v[4];
                     mma_us(u, wa[g].x & 0x0f0f0f0fu, wb[g].x & 0x0f0f0f0fu, wa[g].y & 0x0f0f0f0fu, wb[g].y & 0x0f0f0f0fu, x.x, x.y);
                     mma_us(v, wa[g].x & 0xf0f0f0f0u, wb[g].x & 0xf0f0f0f0u, wa[g].y & 0xf0f0f0f0u, wb[g].y & 0xf0f0f0f0u, x.z, x.w);
-                    add_block(acc[g][t], u, s0[g][0], s0[g][1], lo2(d));
-                    add_block(acc[g][t], v, s1[g][0], s1[g][1], hi2(d));
+                    add_block(acc[c % S][g][t], u, s0[g][0], s0[g][1], lo2(d));
+                    add_block(acc[c % S][g][t], v, s1[g][0], s1[g][1], hi2(d));
                 }
-                if (c == 0) {
-                    const uint4 s = lds128(frag + t * act_stride + 2304);
+                if (S == 1 && c == 0) min_term(t);
+            }
+        }
+        if constexpr (S == 2) {
+            join();
 #pragma unroll
-                    for (int g = 0; g < MT; ++g) {
-                        float f[4], e[4];
-                        mma_mins(f, e, mn[g][0], mn[g][1], s);
-                        acc[g][t][0] = __ffma2_rn(both(ndmin[g][0]), __fadd2_rn(make_float2(f[0], f[1]), make_float2(e[0], e[1])), acc[g][t][0]);
-                        acc[g][t][1] = __ffma2_rn(both(ndmin[g][1]), __fadd2_rn(make_float2(f[2], f[3]), make_float2(e[2], e[3])), acc[g][t][1]);
-                    }
-                }
+            for (int g = 0; g < MT; ++g)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) header(g, r, false, true);           // read again: registers held over the loop would spill
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                if (t >= live) break;
+                min_term(t);
             }
         }
     } else if constexpr (TYPE == LAPLACE_TYPE_Q8_0 || TYPE == LAPLACE_TYPE_Q4_0) {
@@ -258,11 +286,12 @@ __device__ __forceinline__ void super_block_at(uint32_t row, uint32_t act, uint3
                     int u[4], v[4];
                     mma_ss(u, a[g][0][0], a[g][0][1], a[g][0][2], a[g][0][3], x.x, x.y);
                     mma_ss(v, a[g][1][0], a[g][1][1], a[g][1][2], a[g][1][3], x.z, x.w);
-                    add_block(acc[g][t], u, sc[g][0][0], sc[g][0][1], lo2(d));
-                    add_block(acc[g][t], v, sc[g][1][0], sc[g][1][1], hi2(d));
+                    add_block(acc[c % S][g][t], u, sc[g][0][0], sc[g][0][1], lo2(d));
+                    add_block(acc[c % S][g][t], v, sc[g][1][0], sc[g][1][1], hi2(d));
                 }
             }
         }
+        if constexpr (S == 2) join();
     } else {
         // Q6_K (Laplace src/kernels.h:46-54, src/matmul.cpp:180-195): half h, group g of 32 values, s = which 16 of them: low four
         // bits from ql[64 h + 32 (g & 1) + l], nibble g / 2, two more from qh[32 h + l] at bit 2 g, scale sc[8 h + 2 g + s].
@@ -320,23 +349,24 @@ __device__ __forceinline__ void super_block_at(uint32_t row, uint32_t act, uint3
                         int u[4], v[4];
                         mma_ss16(u, a[m][0][0][0], a[m][0][0][1], x.x);
                         mma_ss16(v, a[m][0][1][0], a[m][0][1][1], x.y);
-                        add_block(acc[m][t], u, sc[m][0][0][0], sc[m][0][0][1], lo2(d));
-                        add_block(acc[m][t], v, sc[m][0][1][0], sc[m][0][1][1], lo2(d));
+                        add_block(acc[c % S][m][t], u, sc[m][0][0][0], sc[m][0][0][1], lo2(d));
+                        add_block(acc[c % S][m][t], v, sc[m][0][1][0], sc[m][0][1][1], lo2(d));
                         mma_ss16(u, a[m][1][0][0], a[m][1][0][1], x.z);
                         mma_ss16(v, a[m][1][1][0], a[m][1][1][1], x.w);
-                        add_block(acc[m][t], u, sc[m][1][0][0], sc[m][1][0][1], hi2(d));
-                        add_block(acc[m][t], v, sc[m][1][1][0], sc[m][1][1][1], hi2(d));
+                        add_block(acc[c % S][m][t], u, sc[m][1][0][0], sc[m][1][0][1], hi2(d));
+                        add_block(acc[c % S][m][t], v, sc[m][1][1][0], sc[m][1][1][1], hi2(d));
                     }
                 }
             }
         }
+        if constexpr (S == 2) join();
     }
 }
 
-template <uint32_t TYPE, int PITCH, int MT, int NT>
-__device__ __forceinline__ void super_block(uint32_t row, uint32_t act, uint32_t act_stride, int lane, int live, float2 (&acc)[MT][NT][2]) {
-    if (TYPE == LAPLACE_TYPE_Q6_K && (row & 2)) super_block_at<TYPE, PITCH, MT, NT, 2>(row, act, act_stride, lane, live, acc);
-    else super_block_at<TYPE, PITCH, MT, NT, 0>(row, act, act_stride, lane, live, acc);
+template <uint32_t TYPE, int PITCH, int MT, int NT, int S>
+__device__ __forceinline__ void super_block(uint32_t row, uint32_t act, uint32_t act_stride, int lane, int live, float2 (&acc)[S][MT][NT][2]) {
+    if (TYPE == LAPLACE_TYPE_Q6_K && (row & 2)) super_block_at<TYPE, PITCH, MT, NT, 2, S>(row, act, act_stride, lane, live, acc);
+    else super_block_at<TYPE, PITCH, MT, NT, 0, S>(row, act, act_stride, lane, live, acc);
 }
 
 // ---- quantized rows in fragment order, for calls whose CTAs do not quantize themselves -----------------------------------

@@ -76,6 +76,19 @@ def test_eight_matrices_where_partial_results_have_little_room(oracle, t, M, K):
 
 
 @pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("K,N", [(4096, 2048), (14336, 1024)])
+def test_no_further_from_64_bits_than_one_row_calls(oracle, t, K, N):
+    """Eight rows in one call against eight calls of one row, which run on the dp4a kernel: other sums of the same products, no
+    larger error. 8 x N independent errors put 1 / sqrt(16 N) = 0.8 % of spread on either norm; 8 % between the two is ten of it."""
+    w, x = synth.weights(t, K, N, seed=660, how="affine"), synth.normal_f32(661, (8, K))
+    ref = oracle.gemm(x, w, t, 8, K, N, mode=1, threads=THREADS)
+    (y,), _ = _run(t, x, [w], 8, K, [N])
+    one = np.concatenate([_run(t, x[m:m + 1], [w], 1, K, [N])[0][0] for m in range(8)])
+    err, err_one = (np.linalg.norm(v.astype(np.float64) - ref) for v in (y, one))
+    assert err <= 1.08 * err_one, f"{err / np.linalg.norm(ref):.3e} against {err_one / np.linalg.norm(ref):.3e}"
+
+
 @pytest.mark.parametrize("M", [5, 20])
 def test_special_rows(oracle, t, M):
     """A row of zeros gives zeros, a value that is not a number takes its own row only, so does an infinity."""
