@@ -347,8 +347,8 @@ int laplace_cuda_debug_blocksums_dev(const float* x, const uint8_t* w, uint32_t 
  * Synchronous (a few milliseconds). */
 int laplace_cuda_debug_tensor_peak(int kind, double* tops);
 
-/* Which kernel family the last *_dev gemm call used: 1 = streaming dp4a GEMV,
- * 2 = tensor-core GEMM, 3 = expert-grouped tensor-core GEMM, 4 = fused expert FFN. For tests and the benchmark's launch count. */
+/* What the last *_dev matmul call was: 1 = up to 8 activation rows, 2 = more of them, 3 = expert-grouped, 4 = fused expert
+ * FFN or fp32 activations. For tests and the benchmark's launch count. */
 int laplace_cuda_last_path(void);
 /* Kernel launches issued by this library since the counter was last reset. */
 long long laplace_cuda_launch_count(int reset);
@@ -357,3 +357,6 @@ long long laplace_cuda_launch_count(int reset);
 }
 #endif
 #endif
+/* Which kernel the last matmul launched ran on: 1 = dp4a streaming, 2 = int8 MMA for a handful of rows and for experts
+ * (mma.sync), 3 = int8 MMA tiles, 4 = tcgen05, 5 = tcgen05 with weights in two pieces, 6 = fp32 activations. For tests. */
+int laplace_cuda_last_kernel(void);

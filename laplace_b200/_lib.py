@@ -54,6 +54,7 @@ SYMBOLS = {
     "laplace_cuda_gguf_meta_str": (C.c_char_p, [_vp, C.c_char_p]),
     "laplace_cuda_gguf_close": (None, [_vp]),
     "laplace_cuda_last_path": (_i, []),
+    "laplace_cuda_last_kernel": (_i, []),
     "laplace_cuda_launch_count": (C.c_longlong, [_i]),
 }
 

@@ -295,6 +295,7 @@ const char* laplace_cuda_last_error(void) { return g_err; }
 int laplace_cuda_sm_count(void) { return g_ctx.ready ? g_ctx.sm_count : 0; }
 
 int laplace_cuda_last_path(void) { return g_ctx.last_path; }
+int laplace_cuda_last_kernel(void) { return g_ctx.last_kernel; }
 
 long long laplace_cuda_launch_count(int reset) {
     long long v = g_ctx.launches;

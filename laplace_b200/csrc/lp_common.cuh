@@ -48,8 +48,10 @@ struct Context {
     int*         d_err = nullptr;      // device view of the status word, 0 = fine
     int*         h_err = nullptr;      // host view of the same word (mapped pinned memory)
     int          last_path = 0;
+    int          last_kernel = 0;      // KERNEL_*
     long long    launches = 0;
 };
+enum : int { KERNEL_DP4A = 1, KERNEL_INT8 = 2, KERNEL_INT8_TILES = 3, KERNEL_TCGEN05 = 4, KERNEL_TCGEN05_TWO_PIECE = 5, KERNEL_F32ACT = 6 };      // laplace_cuda_last_kernel
 Context& ctx();
 int  fail(int code, const char* fmt, ...);   // records the message, returns code
 int  cuda_check(cudaError_t e, const char* what);

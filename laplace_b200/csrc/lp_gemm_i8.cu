@@ -625,6 +625,7 @@ int launch_as(const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes
     const cudaError_t e = cudaLaunchKernelEx(&cfg, k, maps, p);
     ctx().launches++;
     return cuda_check(e, "gemm_i8 launch");
+    ctx().last_kernel = KERNEL_INT8;
 }
 
 template <uint32_t TYPE, int NT, bool QUANT>

@@ -1142,6 +1142,7 @@ int launch_gemv_stream(const GemvArgs& a, cudaStream_t st) {
     }
     c.launches++;
     c.last_path = 1;
+    c.last_kernel = KERNEL_DP4A;
     return cuda_check(e, "gemv_stream launch");
 }
 

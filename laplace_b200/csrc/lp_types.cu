@@ -577,6 +577,7 @@ int launch_gemm_f32act(const float* x, const uint8_t* w, uint32_t type, float* y
         }
         c.launches++;
         c.last_path = 4;
+        c.last_kernel = KERNEL_F32ACT;
         if (e != cudaSuccess) return cuda_check(e, "gemv_f32act launch");
     }
     return LAPLACE_OK;

@@ -39,8 +39,9 @@ def test_small_batches(oracle, t, M, K, N):
 
 @pytest.mark.parametrize("M", [8, 24])
 def test_more_rows_than_one_panel(oracle, M):
-    """A cluster's share of the rows goes through shared memory in several panels."""
-    t, K, N = GGMLType.Q4_K, 4096, 33000
+    """A cluster's share of the rows goes through shared memory in several panels: about 2100 rows of 33 clusters' with room for 64
+    row groups (8 rows) or 32 (24 rows), the last panel ragged."""
+    t, K, N = GGMLType.Q4_K, 4096, 70001
     w = synth.weights(t, K, N, seed=610, how="affine")
     x = synth.normal_f32(611, (M, K))
     (y,), _ = _run(t, x, [w], M, K, [N])
