@@ -350,6 +350,9 @@ int laplace_cuda_debug_tensor_peak(int kind, double* tops);
 /* What the last *_dev matmul call was: 1 = up to 8 activation rows, 2 = more of them, 3 = expert-grouped, 4 = fused expert
  * FFN or fp32 activations. For tests and the benchmark's launch count. */
 int laplace_cuda_last_path(void);
+/* Which kernel the last matmul launched ran on: 1 = dp4a streaming, 2 = int8 MMA for a handful of rows and for experts
+ * (mma.sync), 3 = int8 MMA tiles, 4 = tcgen05, 5 = tcgen05 with weights in two pieces, 6 = fp32 activations. For tests. */
+int laplace_cuda_last_kernel(void);
 /* Kernel launches issued by this library since the counter was last reset. */
 long long laplace_cuda_launch_count(int reset);
 
@@ -357,6 +360,3 @@ long long laplace_cuda_launch_count(int reset);
 }
 #endif
 #endif
-/* Which kernel the last matmul launched ran on: 1 = dp4a streaming, 2 = int8 MMA for a handful of rows and for experts
- * (mma.sync), 3 = int8 MMA tiles, 4 = tcgen05, 5 = tcgen05 with weights in two pieces, 6 = fp32 activations. For tests. */
-int laplace_cuda_last_kernel(void);

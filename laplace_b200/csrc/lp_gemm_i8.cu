@@ -624,8 +624,8 @@ int launch_as(const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes
     cfg.dynamicSmemBytes = smem;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, k, maps, p);
     ctx().launches++;
-    return cuda_check(e, "gemm_i8 launch");
     ctx().last_kernel = KERNEL_INT8;
+    return cuda_check(e, "gemm_i8 launch");
 }
 
 template <uint32_t TYPE, int NT, bool QUANT>

@@ -1292,10 +1292,10 @@ int run_i8_kernel(const SaLaunch& L, const SaParams& p, const SaPeers<true>& pe,
         case LAPLACE_TYPE_Q6_K: rc = launch_i8_tiles<LAPLACE_TYPE_Q6_K>(map, L, p, pe, st); break;
         default: return LAPLACE_UNSUPPORTED;
     }
-    ctx().last_kernel = KERNEL_INT8_TILES;
     if (rc) return rc;
     ctx().launches++;
     ctx().last_path = 2;
+    ctx().last_kernel = KERNEL_INT8_TILES;
     return cuda_check(cudaGetLastError(), "gemm_i8_tile launch");
 }
 
@@ -1367,10 +1367,10 @@ int run_sa_kernel(const SaLaunch& L, cudaStream_t st) {
             else w2::gemm_w2_sa_kernel<LAPLACE_TYPE_Q6_K, false><<<L.grid, THREADS, w2::SMEM_BYTES, st>>>(maps, p, none);
             break;
         default: return LAPLACE_UNSUPPORTED;
-    c.last_kernel = L.type == LAPLACE_TYPE_Q4_K ? KERNEL_TCGEN05 : KERNEL_TCGEN05_TWO_PIECE;
     }
     c.launches++;
     c.last_path = 2;
+    c.last_kernel = L.type == LAPLACE_TYPE_Q4_K ? KERNEL_TCGEN05 : KERNEL_TCGEN05_TWO_PIECE;
     return cuda_check(cudaGetLastError(), "gemm_sa launch");
 }
 

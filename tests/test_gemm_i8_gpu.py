@@ -77,7 +77,6 @@ def test_eight_matrices_where_partial_results_have_little_room(oracle, t, M, K):
 
 
 @pytest.mark.parametrize("t", TYPES)
-@pytest.mark.parametrize("t", TYPES)
 @pytest.mark.parametrize("K,N", [(4096, 2048), (14336, 1024)])
 def test_no_further_from_64_bits_than_one_row_calls(oracle, t, K, N):
     """Eight rows in one call against eight calls of one row, which run on the dp4a kernel: other sums of the same products, no
@@ -90,6 +89,7 @@ def test_no_further_from_64_bits_than_one_row_calls(oracle, t, K, N):
     assert err <= 1.08 * err_one, f"{err / np.linalg.norm(ref):.3e} against {err_one / np.linalg.norm(ref):.3e}"
 
 
+@pytest.mark.parametrize("t", TYPES)
 @pytest.mark.parametrize("M", [5, 20])
 def test_special_rows(oracle, t, M):
     """A row of zeros gives zeros, a value that is not a number takes its own row only, so does an infinity."""
