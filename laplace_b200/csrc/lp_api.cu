@@ -150,7 +150,7 @@ int dispatch_gemm_dev(const float* x, const uint8_t* w, uint32_t type, float* y,
     if (M <= 0 || N <= 0 || K <= 0) return fail(LAPLACE_ERR_ARG, "gemm: M=%d K=%d N=%d", M, K, N);
     if (K % block_elems(type)) return fail(LAPLACE_ERR_ARG, "gemm: K=%d is not a multiple of %d", K, block_elems(type));
     // A handful of rows: the int8 kernel that streams the weights once.
-    if (M >= 2 && gemm_i8_supports(type, M, K, &w, 1)) return launch_gemm_i8(x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st);
+    if (M >= 2 && gemm_i8_supports(type, M, K, &w, 1, N)) return launch_gemm_i8(x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st);
     // Prefill: tensor-core GEMM where one exists for the type.
     if (gemm_sa_supports(type, M, K, N)) return launch_gemm_sa(x, w, type, y, M, K, N, st);
     // Small M (or a K that is not a multiple of 256): one streaming pass per group of up to 8 activation rows.
@@ -438,8 +438,9 @@ int laplace_cuda_gemm_multi_dev(const float* x, const float* norm_weight, float 
     const uint8_t* ws[8]; float* ys[8]; int ns[8];
     for (int i = 0; i < n_mats; ++i) { ws[i] = mats[i].w; ys[i] = mats[i].y; ns[i] = mats[i].N; }
     bool whole = true;
-    for (int i = 0; i < n_mats; ++i) whole = whole && ws[i] && ys[i] && ns[i] > 0;
-    if (M >= 2 && whole && gemm_i8_supports(type, M, K, ws, n_mats))
+    long long rows = 0;
+    for (int i = 0; i < n_mats; ++i) { whole = whole && ws[i] && ys[i] && ns[i] > 0; rows += ns[i]; }
+    if (M >= 2 && whole && gemm_i8_supports(type, M, K, ws, n_mats, rows, norm_weight != nullptr))
         return launch_gemm_i8(x, norm_weight, norm_eps, x_norm_out, ws, ys, ns, n_mats, type, M, K,
                               stream ? static_cast<cudaStream_t>(stream) : g_ctx.stream);
     if (M > 8) {

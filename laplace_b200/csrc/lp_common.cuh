@@ -97,7 +97,7 @@ struct PeerOut {
 };
 int launch_gemv_stream(const GemvArgs& a, cudaStream_t st);
 // 2..32 activation rows on mma.sync int8 (lp_gemm_i8.cu): one or several matrices, optional RMSNorm in front
-bool gemm_i8_supports(uint32_t type, int M, int K, const uint8_t* const* ws, int n_mats);
+bool gemm_i8_supports(uint32_t type, int M, int K, const uint8_t* const* ws, int n_mats, long long rows, bool norm = false);
 int  launch_gemm_i8(const float* x, const float* norm_w, float eps, float* x_norm_out, const uint8_t* const* ws, float* const* ys,
                     const int* ns, int n_mats, uint32_t type, int M, int K, cudaStream_t st, uint8_t* scratch = nullptr);
 int  launch_quantize_i8(const float* x, const float* norm_w, float eps, float* x_norm_out, uint32_t type, int M, int K, uint8_t* img, cudaStream_t st);

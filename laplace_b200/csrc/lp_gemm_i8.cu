@@ -11,8 +11,8 @@
 //
 // Shape of the kernel (one CTA per SM, sixteen consumer warps and two copy warps):
 //   * K is cut over a cluster of up to eight CTAs, so that a CTA needs its part of the quantized activations only (they stay
-//     in shared memory for the whole call) and a long-K matrix with few rows still occupies every SM. The cut depends on K
-//     alone, so a matrix gives the same bits in a call of its own and in a call with others;
+//     in shared memory for the whole call) and a long-K matrix with few rows still occupies every SM. The cut depends on
+//     K, type and row count (see plan_dense), so a matrix has the same bits alone and beside others on this kernel;
 //   * every consumer warp takes groups of 16 weight rows for itself (two warps share a group when the CTA's part of K is
 //     eight super-blocks or more): its copies are 2-D tensor-map tiles of 16 rows x one or two super-blocks into a ring of
 //     its own, so that warps never wait for one another while they stream;
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
     const uint32_t ring = ring_of(warp), full0 = bar_full(warp, 0), empty0 = bar_empty(warp, 0);
     // Up to 8 rows: every super-block is summed on its own, even and odd block pairs apart, and then added, so that no chain of
     // roundings is longer than a few dozen terms: error against 64 bits at 8 rows, one running sum / this / the dp4a kernel, Q6_K 4096 x
-    // 1024 15.2 / 8.7 / 8.9e-8, 28672 x 1024 27.2 / 14.4 / 15.2e-8, Q8_0 4096 x 14336 11.6 / 8.0 / 8.0e-8. It costs 0.5 % (Q4_K 1.2 %).
+    // 1024 15.2 / 8.7 / 9.0e-8, 28672 x 1024 27.2 / 10.9 / 14.9e-8, Q8_0 4096 x 14336 11.6 / 8.1 / 8.0e-8. It costs 0.5 % (Q4_K 1.2 %).
     // More rows are below what the tcgen05 kernels show (4e-7) without it.
     constexpr int SETS = QUANT ? 2 : 0;
     // one row group: units of super-blocks [s0, s1); `act` = shared address of the activations of super-block s0
@@ -523,17 +523,18 @@ bool type_geo(uint32_t type, TypeGeo& g) {
 constexpr int MAX_NT = 4;
 struct DensePlan { int nt, c, kw, smax, n_slots; uint32_t act, slab_budget; };
 
-// How K is cut: by K, type and row count alone. A CTA of the cluster gets two super-blocks or more; eight CTAs where the
-// activations of four would not leave room for two ring slots a warp. False: the plan does not fit, the call takes another kernel.
-bool plan_dense(uint32_t type, int M, int K, DensePlan& d) {
+// How K is cut: by K, type and row count, except for Q4_K with 3 to 8 rows and few weight rows. A CTA of the cluster gets two super-blocks
+// or more; eight CTAs where the activations of four would not leave room for two ring slots a warp. False: the plan does not fit,
+// the call takes another kernel.
+// Q4_K, K = 4096..8192, up to 2048 weight rows: eight CTAs, whose shorter prologue is worth more than their weight rows (8 rows: 4096 x 1024
+// 6.6 -> 5.8 us, 6144 x 1024 8.4 -> 6.9, 8192 x 2048 9.2 -> 8.1; 6144 x 4096 9.7 -> 9.7, 4096 x 16384 13.9 -> 16.6).
+bool plan_dense(uint32_t type, int M, int K, long long rows, DensePlan& d) {
     TypeGeo g;
     if (!type_geo(type, g) || M < 2 || M > 8 * MAX_NT || K <= 0 || K % 256) return false;
     const int nsb = K / 256;
-    // short rows, and two activation rows unless the rows are long: the dp4a kernel's shorter prologue wins (4096 x 4096, 2 rows:
-    // 6.7 us against 7.6 for Q4_K, 8.5 against 9.5 for Q6_K; 14336 x 4096: 21.3 against 14.7, 26.7 against 20.2)
-    if (M <= 8 && (nsb < 4 || (M == 2 && nsb < 32))) return false;
     d.nt = (M + 7) / 8;
-    for (int c = nsb >= 8 ? 4 : nsb >= 4 ? 2 : 1; c <= 8; c = c < 4 ? 4 : 2 * c) {
+    const bool wide = type == LAPLACE_TYPE_Q4_K && M <= 8 && rows <= 2048 && nsb >= 16 && nsb <= 32;
+    for (int c = wide ? 8 : nsb >= 8 ? 4 : nsb >= 4 ? 2 : 1; c <= 8; c = c < 4 ? 4 : 2 * c) {
         d.c = c;
         d.smax = (nsb + c - 1) / c;
         d.kw = d.smax >= 8 ? 2 : 1;
@@ -678,10 +679,34 @@ bool map_weights(CUtensorMap* m, const uint8_t* w, uint32_t type, int K, uint64_
 
 }  // namespace
 
-// Matrices the kernel takes: 16-byte aligned rows (the copies are tensor-map tiles) and a plan that fits.
-bool gemm_i8_supports(uint32_t type, int M, int K, const uint8_t* const* ws, int n_mats) {
+// Up to 8 rows: where the dp4a kernel is the faster one. It starts sooner (no cluster, no exchange; with a norm in front the
+// difference grows, since here the row sums cross the cluster) but its time grows with rows x values, so the line is one on their
+// product and, because that growth is per activation value, one on M x super-blocks. `rows`: weight rows of the whole call. Measured,
+// dp4a against this kernel (us):
+//   two rows: 4096 x 4096 Q4_K 6.7 / 7.6, Q6_K 8.5 / 9.5; 14336 x 4096 21.3 / 14.7, 26.7 / 20.2;
+//   Q8_0, three rows, K = 1024: 1024 rows 3.3 / 4.6, 4096 4.3 / 4.9, 8192 5.6 / 5.4; K = 2048: 1024 4.2 / 4.9, 4096 6.4 / 5.8;
+//   K = 3072: 5.5 / 5.5; eight rows, K = 1024: 512 rows 4.7 / 4.0; with a norm, three rows, K = 2048: 3072 rows 8.5 / 9.4, 6144 11.3 / 10.9;
+//   Q6_K, three rows, 4096 x 1024: 6.8 / 7.1, x 2048 8.4 / 7.5; four rows, 2048 x 1024: 5.2 / 5.7, x 4096 8.1 / 6.5;
+//   Q4_K, three rows, K = 1024: 2048 rows 4.6 / 5.1, 4096 5.6 / 5.1; with a norm, 6144 rows 8.8 / 9.4, 16384 15.7 / 10.3.
+// Rows of one to three super-blocks: Q4_K eight rows 768 x 16384 24.0 / 5.6; the other types have not been taken off the dp4a kernel.
+bool dp4a_wins(uint32_t type, int M, int nsb, long long rows, bool norm) {
+    if (M == 2) return nsb < 32;
+    const long long work = rows * M * nsb * 256;
+    if (type == LAPLACE_TYPE_Q4_K) {
+        if (nsb < 4) return norm ? M <= 4 && rows * M <= 12000 : M * nsb <= 6 && work <= 1000000;
+        return norm ? M <= 4 && M * nsb <= 30 && work <= 20000000 : M == 3 && nsb <= 8 && work <= 9000000;
+    }
+    if (nsb < 4) return true;
+    if (type == LAPLACE_TYPE_Q6_K) return M <= 4 && M * nsb <= 48 && work <= 20000000;
+    return M * nsb <= 32 && (norm ? M <= 4 && work <= 28000000 : M <= 6 && work <= 20000000);
+}
+
+// Matrices the kernel takes: 16-byte aligned rows (the copies are tensor-map tiles), a plan that fits, and not faster elsewhere.
+// `rows`: of all matrices.
+bool gemm_i8_supports(uint32_t type, int M, int K, const uint8_t* const* ws, int n_mats, long long rows, bool norm) {
     DensePlan d;
-    if (n_mats < 1 || n_mats > MAX_MATS || !plan_dense(type, M, K, d) || row_bytes(type, K) % 16) return false;
+    if (n_mats < 1 || n_mats > MAX_MATS || !plan_dense(type, M, K, rows, d) || row_bytes(type, K) % 16) return false;
+    if (M <= 8 && dp4a_wins(type, M, K / 256, rows, norm)) return false;
     for (int i = 0; i < n_mats; ++i)
         if (reinterpret_cast<uintptr_t>(ws[i]) & 15) return false;
     return true;
@@ -702,19 +727,20 @@ int launch_gemm_i8(const float* x, const float* norm_w, float eps, float* x_norm
     Context& c = ctx();
     DensePlan d;
     TypeGeo g;
-    if (!plan_dense(type, M, K, d) || !type_geo(type, g)) return LAPLACE_UNSUPPORTED;
+    long long total = 0;
+    for (int i = 0; i < n_mats; ++i) total += ns[i];
+    if (total >= (1LL << 30)) return fail(LAPLACE_ERR_LIMIT, "gemm: more than 2^30 weight rows");
+    if (!plan_dense(type, M, K, total, d) || !type_geo(type, g)) return LAPLACE_UNSUPPORTED;
     if (reinterpret_cast<uintptr_t>(x) & 15) return fail(LAPLACE_ERR_ARG, "gemm: x not 16-byte aligned");
     if (norm_w && ((reinterpret_cast<uintptr_t>(norm_w) & 15) || (x_norm_out && (reinterpret_cast<uintptr_t>(x_norm_out) & 15))))
         return fail(LAPLACE_ERR_ARG, "gemm_multi: the norm weights (and the optional output) must be 16-byte aligned");
     I8Maps maps;
     I8Params p{};
-    long long total = 0;
-    for (int i = 0; i < n_mats; ++i) {
+    for (int i = 0, end = 0; i < n_mats; ++i) {
         if (!map_weights(&maps.w[i], ws[i], type, K, static_cast<uint64_t>(ns[i]), g)) return LAPLACE_ERR_CUDA;
-        total += ns[i];
-        if (total >= (1LL << 30)) return fail(LAPLACE_ERR_LIMIT, "gemm: more than 2^30 weight rows");
+        end += ns[i];
         p.mat_y[i] = ys[i];
-        p.mat_end[i] = static_cast<int>(total);
+        p.mat_end[i] = end;
     }
     for (int i = n_mats; i < MAX_MATS; ++i) maps.w[i] = maps.w[0];
     p.x = x; p.norm_w = norm_w; p.norm_eps = eps; p.x_norm_out = x_norm_out; p.err = c.d_err;

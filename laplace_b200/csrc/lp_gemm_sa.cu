@@ -1538,7 +1538,7 @@ int launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const 
     if (pl.total() > cap)
         return fail(LAPLACE_ERR_LIMIT, "gemm: M=%d K=%d needs %zu bytes of scratch, the caller's area holds %zu", M, K, pl.total(), cap);
     // a handful of rows: a twelfth of that operand at most, but the limit stays one formula for every row count
-    if (gemm_i8_supports(type, M, K, &w, 1)) return launch_gemm_i8(x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, scratch);
+    if (gemm_i8_supports(type, M, K, &w, 1, N)) return launch_gemm_i8(x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, scratch);
     return gemm_sa_on_scratch(scratch, pl, i8_tiles(type, M, K, &w, 1), x, w, type, y, M, K, N, st);
 }
 

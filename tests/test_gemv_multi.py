@@ -47,12 +47,12 @@ def test_multi_matrix_gemv(oracle, t, M, K, Ns, norm):
     for y, w, n in zip(ys, ws, Ns):
         mass = oracle.gemm(x_in, w, t, M, K, n, mode=2)
         check_close(y.cpu().numpy(), oracle.gemm(x_in, w, t, M, K, n, mode=1), f"multi {t.name} M={M} K={K} N={n} norm={norm}", mass)
-        # and bit-identical to a single-matrix call on the same activations (the same kernel), except where the single
-        # call takes another kernel (Q4_K with 3..8 rows runs on mma.sync tiles: another fp32 summation order)
+        # and bit-identical to a single-matrix call on the same activations (the same kernel), except for Q4_K with 3..8 rows, where
+        # a call of few weight rows may take another kernel than one of more (another fp32 summation order)
         single = device.gemm(torch.from_numpy(np.ascontiguousarray(x_in)).cuda(), device.upload_weights(w), t, M, K, n)
         device.sync()
         if t == GGMLType.Q4_K and 3 <= M <= 8 and K % 256 == 0:
-            check_close(single.cpu().numpy(), y.cpu().numpy().astype(np.float64), "single (mma kernel) vs multi (dp4a kernel)", mass)
+            check_close(single.cpu().numpy(), y.cpu().numpy().astype(np.float64), "single vs multi", mass)
         else:
             assert np.array_equal(single.cpu().numpy(), y.cpu().numpy())
 

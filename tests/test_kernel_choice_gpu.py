@@ -37,13 +37,46 @@ def _gemm(t, x, w, M, K, N, off=0):
 
 
 @pytest.mark.parametrize("t,M,K,off,kernel", [
-    (Q4_K, 1, 4096, 0, DP4A), (Q4_K, 9, 256, 0, INT8), (Q4_K, 32, 4096, 0, INT8), (Q4_K, 33, 4096, 0, INT8_TILES), (Q4_K, 80, 2048, 0, INT8_TILES), (Q4_K, 81, 2048, 0, TCGEN05),
+    (Q4_K, 1, 4096, 0, DP4A), (Q4_K, 2, 7936, 0, DP4A), (Q4_K, 2, 8192, 0, INT8), (Q4_K, 3, 512, 0, DP4A), (Q4_K, 3, 768, 0, INT8), (Q4_K, 3, 2048, 0, DP4A), (Q4_K, 3, 2304, 0, INT8),
+    (Q6_K, 3, 4096, 0, DP4A), (Q6_K, 4, 4096, 0, INT8), (Q8_0, 4, 2048, 0, DP4A), (Q8_0, 4, 2304, 0, INT8), (Q4_0, 7, 1024, 0, INT8), (Q8_0, 8, 768, 0, DP4A), (Q4_K, 9, 256, 0, INT8), (Q4_K, 32, 4096, 0, INT8), (Q4_K, 33, 4096, 0, INT8_TILES), (Q4_K, 80, 2048, 0, INT8_TILES), (Q4_K, 81, 2048, 0, TCGEN05),
     (Q6_K, 32, 2048, 0, INT8), (Q6_K, 112, 2048, 0, INT8_TILES), (Q6_K, 113, 2048, 0, TCGEN05_TWO_PIECE), (Q6_K, 24, 2816, 0, TCGEN05_TWO_PIECE),
     (Q8_0, 16, 512, 0, INT8), (Q8_0, 130, 512, 0, INT8_TILES), (Q8_0, 16, 512, 2, TCGEN05_TWO_PIECE), (Q4_0, 200, 768, 0, INT8_TILES), (Q4_0, 200, 768, 2, TCGEN05_TWO_PIECE),
     (Q8_0, 20, 544, 0, DP4A)])
 def test_lines_between_the_kernels(t, M, K, off, kernel):
     w, x = synth.weights(t, K, 40, seed=860, how="random"), synth.normal_f32(861, (M, K))
     assert _gemm(t, x, w, M, K, 40, off)[1] == kernel
+
+
+@pytest.mark.parametrize("t,M,K,N", [(Q8_0, 3, 1024, 6511), (Q4_K, 3, 1024, 2930), (Q6_K, 4, 2048, 2442), (Q4_K, 4, 256, 1000)])
+def test_line_on_the_weight_rows(oracle, t, M, K, N):
+    """The last row count of the dp4a kernel and the first of the int8 one, with room for neither's rounding in between."""
+    w, x = synth.weights(t, K, N, seed=874, how="random"), synth.normal_f32(875, (M, K))
+    ref = oracle.gemm(x, w, t, M, K, N, mode=1, threads=THREADS)
+    kernels = []
+    for n in (N - N // 8, N):
+        y, kernel = _gemm(t, x, w[:n], M, K, n)
+        kernels.append(kernel)
+        check_close(y, ref[:, :n], f"{t.name} {M} x {K} x {n}")
+    assert kernels == [DP4A, INT8]
+
+
+@pytest.mark.parametrize("t,M,K,Ns", [(Q4_K, 8, 4096, (1024, 1000, 24)), (Q4_K, 5, 6144, (17,)), (Q4_K, 3, 8192, (700, 1349)), (Q4_K, 8, 256, (40, 9)), (Q4_K, 6, 768, (1000, 33)),
+                                      (Q4_K, 3, 512, (5000, 16))])
+@pytest.mark.parametrize("norm", [False, True])
+def test_q4k_plans_of_up_to_eight_rows(oracle, t, M, K, Ns, norm):
+    """Clusters of eight up to 2048 weight rows and of four beyond, single CTAs for rows of one to three super-blocks."""
+    import torch
+    from laplace_b200 import device
+    ws = [synth.random_blocks(t, K, n, seed=876 + i) for i, n in enumerate(Ns)]
+    x = synth.normal_f32(877, (M, K))
+    nw = torch.from_numpy((1.0 + 0.1 * synth.normal_f32(878, (K,))).astype(np.float32)).cuda() if norm else None
+    ys, xn = device.gemm_multi(torch.from_numpy(x).cuda(), [_upload(w) for w in ws], t, M, K, list(Ns), norm_weight=nw, eps=1e-5, want_x_norm=True)
+    device.sync()
+    assert device.lib().laplace_cuda_last_kernel() == INT8
+    x_in = xn.cpu().numpy() if norm else x
+    for y, w, n in zip(ys, ws, Ns):
+        mass = oracle.gemm(x_in, w, t, M, K, n, mode=2, threads=THREADS)
+        check_close(y.cpu().numpy(), oracle.gemm(x_in, w, t, M, K, n, mode=1, threads=THREADS), f"Q4_K M={M} K={K} N={n}", mass)
 
 
 @pytest.mark.parametrize("t,off", [(Q6_K, 2), (Q8_0, 2), (Q4_0, 2), (Q6_K, 0)])
