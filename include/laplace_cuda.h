@@ -23,6 +23,13 @@
  * (src/threadpool.h:236-257 has a single dispatch slot). Host-pointer entry
  * points are synchronous. *_dev entry points only enqueue work on the given
  * stream.
+ *
+ * Overlap: a call's first kernel may start while the kernel before it in the
+ * stream is ending. It waits for that kernel before it touches activations,
+ * norm weights, indices, scratch or results; with up to 8 activation rows it
+ * copies WEIGHTS before it waits. A program that writes weights with a kernel
+ * of its own on the same stream lets that kernel finish before it makes such a
+ * call (a memory copy or a stream synchronisation in between does).
  */
 #ifndef LAPLACE_CUDA_H
 #define LAPLACE_CUDA_H
@@ -84,13 +91,13 @@ int laplace_cuda_unregister_weights(const void* base);
  * reference is single-device). */
 void laplace_cuda_nsplit(int N, int rank, int world, int* row_begin, int* row_end);
 
-/* Scratch memory and CUDA graphs. laplace_cuda_gemm_dev (more than 8 activation rows), laplace_cuda_moe_grouped_dev,
- * laplace_cuda_moe_ffn_dev and laplace_cuda_gemm_peers_dev keep their quantized operands in scratch buffers that grow to
+/* Scratch memory and CUDA graphs. laplace_cuda_gemm_dev and laplace_cuda_gemm_multi_dev (more than 8 activation rows),
+ * laplace_cuda_moe_grouped_dev, laplace_cuda_moe_ffn_dev and laplace_cuda_gemm_peers_dev keep their quantized operands in scratch buffers that grow to
  * the largest call seen. A buffer that was handed to a launch is never freed before laplace_cuda_shutdown (a captured
  * graph may hold its address), but growing calls the allocator, which is illegal while the call's stream is being
  * captured: such a call returns LAPLACE_ERR_STATE and leaves the capture valid. Make every call shape once before
  * capturing it. Calls that share a scratch buffer must not overlap on the GPU (one stream, or the caller's own
- * ordering). laplace_cuda_gemm_dev with 3 to 8 rows of Q4_K uses a fixed array inside the library in the same way. */
+ * ordering). Calls of up to 8 rows use no scratch. */
 
 /* ---- the three back-end entry points (host pointers) -------------------- */
 
@@ -99,7 +106,8 @@ void laplace_cuda_nsplit(int N, int rank, int world, int* row_begin, int* row_en
  * Q4_0, Q5_0, Q8_0, Q4_K and Q6_K are computed as that back-end computes them (activations quantized to Q8 per 32
  * values, integer block sums, fp32 scales); the three MoE entry points below take the same five types. More than 8
  * rows run on the tensor cores for Q4_0 / Q8_0 / Q4_K / Q6_K when K % 256 == 0, otherwise (and for Q5_0) in passes
- * of 8 rows through the streaming kernel. */
+ * of 8 rows through the streaming kernel. The device-pointer twin takes the tensor cores from 2 or 3 rows on where the
+ * rows' bytes are a multiple of 16 and the base is 16-byte aligned. */
 int laplace_cuda_gemm(const float* x, const uint8_t* w, uint32_t type,
                       float* y, int M, int K, int N);
 
@@ -131,8 +139,9 @@ int laplace_cuda_moe_gemv_dev(const float* x, const uint8_t* w, uint32_t type,
  * x_norm = x * 1/sqrt(mean(x^2) + norm_eps) * norm_weight, fp32) and quantized ONCE inside the kernel's prologue and
  * every matrix streams past it: y_i[m*N_i + j] = dot(quantize(x_norm[m]), row j of matrix i). x_norm_out (optional)
  * receives the normalised rows [M][K]. 1..8 matrices. Device pointers. With M <= 8 (decode) everything is one launch;
- * with more rows (prefill; K a multiple of 256) one quantizer launch normalises and quantizes the rows once and every
- * matrix then runs as a tensor-core GEMM on that shared operand. */
+ * with more rows (prefill; K a multiple of 256) one quantizer launch normalises and quantizes the rows once, and the
+ * matrices then run as tensor-core GEMMs on that shared operand: all in one launch with up to 32 rows (weights as
+ * for laplace_cuda_gemm_dev above), one by one with more. */
 typedef struct { const uint8_t* w; float* y; int N; } laplace_cuda_matrix;
 int laplace_cuda_gemm_multi_dev(const float* x, const float* norm_weight, float norm_eps, float* x_norm_out,
                                 const laplace_cuda_matrix* mats, int n_mats, uint32_t type, int M, int K, void* stream);

@@ -911,7 +911,7 @@ gemm_w2_sa_kernel(const __grid_constant__ SaMaps maps, const SaParams p, const S
 
 // ---- the same tiles on the warp-level int8 instruction ------------------------------------------------------------
 // Integer block sums of 128 weight rows x up to 128 tokens from mma.sync (super_block in lp_i8.cuh: one super-block of 32 weight
-// rows x 64 tokens per consumer warp), the fp32 scale chain in registers, results, pieces and tables as in the kernels above.
+// rows x 64 tokens per consumer warp), the fp32 scale chain in registers, results and pieces as in the kernels above. Dense calls only.
 // Bound by the FP32 pipe: the chain costs 12 cycles of it per 16 x 8 x 32 products, the MMA 8 cycles of the tensor pipe beside
 // it. The two-piece tcgen05 form needs four fp16 products a value and eight fp16 values written per packed one, which its
 // converter warps cannot feed. A producer warp fills three stages of one super-block: the packed rows by one tensor-map tile,
@@ -942,7 +942,7 @@ gemm_i8_tile_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t* __r
         fence_barrier_init();
     }
     __syncthreads();
-    // the quantized tokens (and a job table) are the kernel's before this one, which this one's launch and set-up overlap
+    // the quantized tokens are the kernel's before this one, which this one's launch and set-up overlap
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const Segments sg = segments(p);
     const int nsb = p.K / 256;
@@ -1033,6 +1033,8 @@ gemm_i8_tile_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t* __r
                         for (int k = 0; k < 4; ++k)
                             if (n + 8 * k < p.N) pe.y[r][static_cast<size_t>(row) * pe.ld + pe.col0 + n + 8 * k] = v[k];
                 } else {
+                    // a dense call has no out_row; without these lines the compiler orders the loop above so that Q4_0 at 64 to 96 rows
+                    // takes 4 to 6 % longer (4096 x 14336, 96 rows: 50.0 -> 53.1 us)
                     int orow = p.out_row ? __ldg(p.out_row + row) : row;
                     if (p.out_identity && orow >= 0) orow = row;
                     if (orow < 0) continue;
@@ -1315,7 +1317,7 @@ int run_sa_kernel(const SaLaunch& L, cudaStream_t st) {
         pe.n = L.peers->world; pe.ld = L.peers->ld; pe.col0 = L.peers->col0;
     }
     if (L.peers && (L.out_row || L.tile_tab)) return fail(LAPLACE_ERR_STATE, "gemm_sa: the peer-store form takes a plain dense call");
-    if (L.i8) return run_i8_kernel(L, p, pe, st);
+    if (L.i8) return L.out_row || L.tile_tab ? fail(LAPLACE_ERR_STATE, "gemm_sa: the int8 tiles take a plain dense call") : run_i8_kernel(L, p, pe, st);
     SaMaps maps;
     for (int bk = 0; bk < 4; ++bk) {
         if (!make_map_2d(&maps.a[bk], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, L.op.a, static_cast<uint64_t>(K), 2ull * L.op.m_pad,
@@ -1724,7 +1726,7 @@ struct GroupBounds { size_t rows, groups; };
 GroupBounds group_bounds(int P, int E, int group = TT) {
     const size_t live = static_cast<size_t>(E < P ? E : P);
     GroupBounds b;
-    b.rows = ((static_cast<size_t>(P) + 15 * live + TT - 1) / TT + 1) * TT;       // every expert pads to 16 rows; one box of slack
+    b.rows = ((static_cast<size_t>(P) + 15 * live + TT - 1) / TT + 1) * TT;       // every expert pads to 16 rows (int8 jobs: to 8); one box of slack
     b.groups = static_cast<size_t>(P) / group + live;
     return b;
 }
@@ -1753,9 +1755,12 @@ bool moe_sa_supports(uint32_t type, int K, int N) { return gemm_sa_supports(type
 
 namespace {
 
-// Up to 32 pairs per expert on average: the int8 kernel, one pass over an expert's weights (128 experts, hidden 2048, width 768, Q4_K,
-// router included: 16 pairs 168 us against 430, 32 pairs 267 against 515; 32 pairs of 8 Q8_0 experts 50 against 112). Beyond
-// that most experts would take a second pass, while the tcgen05 tiles cost little more up to 128 tokens.
+// Up to 32 pairs per expert on average: jobs of the int8 kernel. A job holds as many tokens as fit beside two ring slots a warp (32, 16
+// or 8; Q4_K rows of 2048 values 16, of 4096 values 8; a fused layer takes the smaller of its two matmuls' counts), so an expert
+// with more is read more than once, from L2. The jobs win up to the line all the same (fused layer, 128 experts, Q4_K, tcgen05 > int8
+// at 8 / 16 / 32 pairs: hidden 2048, width 768 396 > 121, 419 > 165, 507 > 263 us; hidden 4096, width 1536 1279 > 358, 1330 > 586,
+// 1489 > 1030; hidden 6144, width 1024 1299 > 351, 1355 > 574, 1545 > 1031; 8 experts, Q8_0, hidden 4096, 32 pairs 273 > 90). Their
+// time grows with the pairs and the tcgen05 tiles' hardly does up to 128 tokens: the line stays where they were compared.
 constexpr int I8_PAIRS_PER_EXPERT = 32;
 bool few_per_expert(int P, int E) { return P <= I8_PAIRS_PER_EXPERT * static_cast<long long>(E < P ? E : P); }
 
