@@ -1486,6 +1486,10 @@ int gemm_sa_on_scratch(uint8_t* scratch, const SaPlan& pl, bool i8, const float*
 int launch_gemm_sa(const float* x, const uint8_t* w, uint32_t type, float* y, int M, int K, int N, cudaStream_t st) {
     int rc = check_args(x, w, type, M, K, N);
     if (rc) return rc;
+    if (gemm_pair_supports(type, M)) {
+        if ((rc = g_scratch.ensure(gemm_pair_scratch(type, M, K, &N, 1, true), st))) return rc;
+        return launch_gemm_pair(static_cast<uint8_t*>(g_scratch.p), true, x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, nullptr);
+    }
     const SaPlan pl = plan_sa(M, K, N, true);
     if ((rc = g_scratch.ensure(pl.total(), st))) return rc;
     return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, i8_tiles(type, M, K, &w, 1), x, w, type, y, M, K, N, st);
@@ -1504,6 +1508,10 @@ int launch_gemm_sa_multi(const float* x, const float* norm_w, float eps, float* 
     }
     if (norm_w && ((reinterpret_cast<uintptr_t>(norm_w) & 15) || (x_norm_out && (reinterpret_cast<uintptr_t>(x_norm_out) & 15))))
         return fail(LAPLACE_ERR_ARG, "gemm_multi: the norm weights (and the optional output) must be 16-byte aligned");
+    if (gemm_pair_supports(type, M)) {
+        if ((rc = g_scratch.ensure(gemm_pair_scratch(type, M, K, ns, n_mats, true), st))) return rc;
+        return launch_gemm_pair(static_cast<uint8_t*>(g_scratch.p), true, x, norm_w, eps, x_norm_out, ws, ys, ns, n_mats, type, M, K, st, nullptr);
+    }
     if ((rc = g_scratch.ensure(need, st))) return rc;
     uint8_t* scratch = static_cast<uint8_t*>(g_scratch.p);
     const bool i8 = i8_tiles(type, M, K, ws, n_mats);
@@ -1523,6 +1531,10 @@ int launch_gemm_sa_multi(const float* x, const float* norm_w, float eps, float* 
 int launch_gemm_sa_peers(const float* x, const uint8_t* w, uint32_t type, const PeerOut& po, int M, int K, int N, cudaStream_t st) {
     int rc = check_args(x, w, type, M, K, N);
     if (rc) return rc;
+    if (gemm_pair_supports(type, M)) {
+        if ((rc = g_scratch.ensure(gemm_pair_scratch(type, M, K, &N, 1, true), st))) return rc;
+        return launch_gemm_pair(static_cast<uint8_t*>(g_scratch.p), true, x, nullptr, 0.f, nullptr, &w, nullptr, &N, 1, type, M, K, st, &po);
+    }
     const SaPlan pl = plan_sa(M, K, N, true);
     if ((rc = g_scratch.ensure(pl.total(), st))) return rc;
     return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, i8_tiles(type, M, K, &w, 1), x, w, type, nullptr, M, K, N, st, &po);
@@ -1539,6 +1551,11 @@ int launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const 
     if (pl.total() > cap) pl = plan_sa(M, K, N, false);
     if (pl.total() > cap)
         return fail(LAPLACE_ERR_LIMIT, "gemm: M=%d K=%d needs %zu bytes of scratch, the caller's area holds %zu", M, K, pl.total(), cap);
+    if (gemm_pair_supports(type, M)) {
+        const bool cut = gemm_pair_scratch(type, M, K, &N, 1, true) <= cap;
+        if (gemm_pair_scratch(type, M, K, &N, 1, cut) <= cap)       // always: its operand is smaller than the one above
+            return launch_gemm_pair(scratch, cut, x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, nullptr);
+    }
     // a handful of rows: a twelfth of that operand at most, but the limit stays one formula for every row count
     if (gemm_i8_supports(type, M, K, &w, 1, N)) return launch_gemm_i8(x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, scratch);
     return gemm_sa_on_scratch(scratch, pl, i8_tiles(type, M, K, &w, 1), x, w, type, y, M, K, N, st);
