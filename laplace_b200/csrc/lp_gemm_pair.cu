@@ -27,6 +27,7 @@
 // All waits are bounded; a wait that gives up raises the status word and the CTA's roles leave their loops.
 #include <cuda_bf16.h>
 
+#include "lp_i8.cuh"
 #include "lp_scratch.cuh"
 #include "lp_tc.cuh"
 
@@ -575,20 +576,56 @@ struct PairOperand {
     int     m_pad;
 };
 
+// Four lanes per 32-value block, 64 blocks at a time. NIT: rounds that a row takes; its values then stay in registers over the norm, the
+// row's maximum and the quantization, all loads in flight at once (512 rows of 4096: 9.5 us with three passes over the row, 5 so). 0: rows of
+// any length, read again for every pass.
+template <int NIT>
 __global__ void __launch_bounds__(256) quantize_pair_kernel(const float* __restrict__ x, const float* __restrict__ norm_w, float eps,
                                                             float* __restrict__ x_norm_out, int K, PairOperand op, int sums) {
     __shared__ float red[8], red2[8];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const int m = blockIdx.x, bpr = K / 32, grp = threadIdx.x >> 3, t8 = threadIdx.x & 7, warp = threadIdx.x >> 5;
-    const float* xr = x + static_cast<size_t>(m) * K;
+    const int m = blockIdx.x, bpr = K / 32, grp = threadIdx.x >> 2, t4 = threadIdx.x & 3, warp = threadIdx.x >> 5;
+    const int rounds = NIT ? NIT : (bpr + 63) / 64;
+    const float4* xr = reinterpret_cast<const float4*>(x + static_cast<size_t>(m) * K) + 2 * t4;
+    const float4* nr = reinterpret_cast<const float4*>(norm_w) + 2 * t4;
+    float4 v[NIT ? NIT : 1][2];
+    auto fetch = [&](int r, float4 (&o)[2]) {
+        const int b = r * 64 + grp;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) o[e] = b < bpr ? __ldg(xr + b * 8 + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    if constexpr (NIT > 0) {
+#pragma unroll
+        for (int r = 0; r < NIT; ++r) fetch(r, v[r]);
+    }
+    // f(round, the lane's eight values), values as they are in the row or normalised
     float inv = 1.f;
+    bool norm = false;
+    auto each = [&](auto f) {
+#pragma unroll
+        for (int r = 0; r < (NIT ? NIT : 1 << 30); ++r) {
+            if (NIT == 0 && r >= rounds) break;
+            float4 (&o)[2] = v[NIT ? r : 0];
+            if (NIT == 0) fetch(r, o);
+            if (norm) {
+                const int b = r * 64 + grp;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const float4 w = b < bpr ? __ldg(nr + b * 8 + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    o[e] = make_float4(__fmul_rn(__fmul_rn(o[e].x, inv), w.x), __fmul_rn(__fmul_rn(o[e].y, inv), w.y), __fmul_rn(__fmul_rn(o[e].z, inv), w.z),
+                                       __fmul_rn(__fmul_rn(o[e].w, inv), w.w));
+                }
+            }
+            f(r, o);
+        }
+    };
     if (norm_w) {
         float ss = 0.f;
-        for (int i = threadIdx.x; i < K / 4; i += blockDim.x) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(xr) + i);
-            ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
-        }
+        each([&](int, const float4 (&o)[2]) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) ss = fmaf(o[e].x, o[e].x, fmaf(o[e].y, o[e].y, fmaf(o[e].z, o[e].z, fmaf(o[e].w, o[e].w, ss))));
+        });
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         if ((threadIdx.x & 31) == 0) red2[warp] = ss;
@@ -597,20 +634,17 @@ __global__ void __launch_bounds__(256) quantize_pair_kernel(const float* __restr
         for (int w = 0; w < 8; ++w) t += red2[w];
         inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(t, static_cast<float>(K)), eps)));
     }
-    auto load = [&](int b) {
-        float4 v = __ldg(reinterpret_cast<const float4*>(xr + b * 32) + t8);
-        if (norm_w) {
-            const float4 w = __ldg(reinterpret_cast<const float4*>(norm_w + b * 32) + t8);
-            v = make_float4(__fmul_rn(__fmul_rn(v.x, inv), w.x), __fmul_rn(__fmul_rn(v.y, inv), w.y), __fmul_rn(__fmul_rn(v.z, inv), w.z), __fmul_rn(__fmul_rn(v.w, inv), w.w));
-        }
-        return v;
-    };
+    norm = norm_w != nullptr;
     float amax = 0.f;
-    for (int b = grp; b < bpr; b += 32) {
-        const float4 v = load(b);
-        if (x_norm_out) reinterpret_cast<float4*>(x_norm_out + static_cast<size_t>(m) * K + b * 32)[t8] = v;
-        amax = max_nan(amax, max_nan(max_nan(fabsf(v.x), fabsf(v.y)), max_nan(fabsf(v.z), fabsf(v.w))));
-    }
+    each([&](int r, const float4 (&o)[2]) {
+        const int b = r * 64 + grp;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            if (x_norm_out && b < bpr) reinterpret_cast<float4*>(x_norm_out + static_cast<size_t>(m) * K + b * 32)[2 * t4 + e] = o[e];
+            amax = max_nan(amax, max_nan(max_nan(fabsf(o[e].x), fabsf(o[e].y)), max_nan(fabsf(o[e].z), fabsf(o[e].w))));
+        }
+    });
+    norm = norm && NIT == 0;               // values in registers are normalised by now
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     if ((threadIdx.x & 31) == 0) red[warp] = amax;
@@ -624,37 +658,37 @@ __global__ void __launch_bounds__(256) quantize_pair_kernel(const float* __restr
     field = field < 1 ? 1 : (field > 253 ? 253 : field);
     const float s = __uint_as_float(static_cast<uint32_t>(field) << 23);
     if (threadIdx.x == 0) op.inv_s[m] = __uint_as_float(static_cast<uint32_t>(254 - field) << 23);
-    for (int base = 0; base < bpr; base += 32) {                    // whole warps iterate together: the 8-lane shuffles stay converged
-        const int b = base + grp;
-        const bool live = b < bpr;
-        const float4 v = live ? load(b) : make_float4(0.f, 0.f, 0.f, 0.f);
-        uint32_t packed; int hs;
-        const float d = quantize_block_8lanes(v, packed, hs);
-        const int hs_hi = __shfl_down_sync(0xffffffffu, hs, 4);
-        if (!live) continue;
-        float f[4];
-        __half h[4], l[4];
+    __half* hi = op.a + static_cast<size_t>(m) * K;
+    __half* lo = hi + static_cast<size_t>(op.m_pad) * K;
+    each([&](int r, const float4 (&o)[2]) {                         // whole warps: the shuffles stay converged
+        const int b = r * 64 + grp;
+        uint32_t w[2];
+        int isum;
+        const float d = i8::quantize_block_4lanes(o[0], o[1], w[0], w[1], isum);
+        if (b >= bpr) return;
+        uint32_t h[4], l[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            f[i] = __fmul_rn(__fmul_rn(d, static_cast<float>(static_cast<int8_t>((packed >> (8 * i)) & 0xff))), s);
-            h[i] = __float2half_rn(f[i]);
-            l[i] = __float2half_rn(f[i] - __half2float(h[i]));
+        for (int e = 0; e < 4; ++e) {                               // values e / 2 * 4 + (e & 1) and two further on
+            const uint32_t q = w[e >> 1] >> (8 * (e & 1));
+            const float fa = __fmul_rn(__fmul_rn(d, static_cast<float>(static_cast<int8_t>(q & 0xff))), s), fb = __fmul_rn(__fmul_rn(d, static_cast<float>(static_cast<int8_t>((q >> 16) & 0xff))), s);
+            const __half2 x2 = __floats2half2_rn(fa, fb);
+            h[e] = h2_bits(x2);
+            l[e] = h2_bits(__floats2half2_rn(fa - __low2float(x2), fb - __high2float(x2)));
         }
-        __half* hi = op.a + static_cast<size_t>(m) * K + b * 32;
-        reinterpret_cast<uint2*>(hi)[t8] = make_uint2(h2_bits(__halves2half2(h[0], h[2])), h2_bits(__halves2half2(h[1], h[3])));
-        reinterpret_cast<uint2*>(hi + static_cast<size_t>(op.m_pad) * K)[t8] = make_uint2(h2_bits(__halves2half2(l[0], l[2])), h2_bits(__halves2half2(l[1], l[3])));
-        if (t8 == 0) {
-            if (sums) {
-                const short slo = static_cast<short>(hs), shi = static_cast<short>(hs_hi);
-                const float sum = __fmul_rn(__fmul_rn(d, static_cast<float>(static_cast<int>(slo) + static_cast<int>(shi))), s);
-                __nv_bfloat16* sp = op.s + static_cast<size_t>(m) * (K / 4) + (b >> 3) * 64 + (b & 7);
-                const __nv_bfloat16 p1 = __float2bfloat16_rn(sum);
-                const float r1 = sum - __bfloat162float(p1);
-                const __nv_bfloat16 p2 = __float2bfloat16_rn(r1);
-                sp[0] = sp[8] = sp[32] = p1; sp[16] = sp[24] = p2; sp[40] = __float2bfloat16_rn(r1 - __bfloat162float(p2));
+        reinterpret_cast<uint4*>(hi + b * 32)[t4] = make_uint4(h[0], h[1], h[2], h[3]);
+        reinterpret_cast<uint4*>(lo + b * 32)[t4] = make_uint4(l[0], l[1], l[2], l[3]);
+        if (sums) {
+            const float sum = __fmul_rn(__fmul_rn(d, static_cast<float>(isum)), s);
+            const __nv_bfloat16 p1 = __float2bfloat16_rn(sum);
+            const float r1 = sum - __bfloat162float(p1);
+            const __nv_bfloat16 p2 = __float2bfloat16_rn(r1);
+            __nv_bfloat16* sp = op.s + static_cast<size_t>(m) * (K / 4) + (b >> 3) * 64 + (b & 7) + 16 * t4;      // g1 g1 | g2 g2 | g1 g3
+            if (t4 < 3) {
+                sp[0] = t4 == 1 ? p2 : p1;
+                sp[8] = t4 == 0 ? p1 : t4 == 1 ? p2 : __float2bfloat16_rn(r1 - __bfloat162float(p2));
             }
         }
-    }
+    });
 }
 
 // Adds up the pieces of every cut tile in k order. Block (t, j): tokens 16 j .. 16 j + 15 of cut tile t, four at a time; a thread has four rows.
@@ -836,7 +870,11 @@ int launch_gemm_pair(uint8_t* scratch, bool cut, const float* x, const float* no
             return LAPLACE_ERR_CUDA;
     }
     ctx().launches++;
-    int rc = launch_early(quantize_pair_kernel, dim3(M), 256, 0, st, x, norm_w, eps, x_norm_out, K, op, type == LAPLACE_TYPE_Q4_K ? 1 : 0);
+    const int sums = type == LAPLACE_TYPE_Q4_K ? 1 : 0;
+    int rc = K <= 4096 ? launch_early(quantize_pair_kernel<2>, dim3(M), 256, 0, st, x, norm_w, eps, x_norm_out, K, op, sums)
+           : K <= 8192 ? launch_early(quantize_pair_kernel<4>, dim3(M), 256, 0, st, x, norm_w, eps, x_norm_out, K, op, sums)
+           : K <= 16384 ? launch_early(quantize_pair_kernel<8>, dim3(M), 256, 0, st, x, norm_w, eps, x_norm_out, K, op, sums)
+                        : launch_early(quantize_pair_kernel<0>, dim3(M), 256, 0, st, x, norm_w, eps, x_norm_out, K, op, sums);
     if (rc) return rc;
     if (peers) {
         PairPeers<true> pe{};
