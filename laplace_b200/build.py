@@ -18,7 +18,7 @@ ROOT = PKG.parent
 LIB = PKG / "liblaplace_cuda.so"
 NATIVE = PKG / "_native.so"
 
-SOURCES = ["lp_api.cu", "lp_gemv.cu", "lp_quantize.cu", "lp_gemm_sa.cu", "lp_peak.cu", "lp_gguf.cu", "lp_types.cu", "lp_gemm_i8.cu", "lp_gemm_pair.cu"]
+SOURCES = ["lp_api.cu", "lp_gemv.cu", "lp_quantize.cu", "lp_gemm_sa.cu", "lp_peak.cu", "lp_gguf.cu", "lp_types.cu", "lp_gemm_i8.cu", "lp_gemm_pair.cu", "lp_gemm_i8_tiles.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -129,6 +129,10 @@ int  launch_gemm_sa(const float* x, const uint8_t* w, uint32_t type, float* y, i
 int  launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const uint8_t* w, uint32_t type, float* y,
                              int M, int K, int N, cudaStream_t st);
 void release_gemm_sa_scratch();
+// Tiles of 128 weight rows x up to 128 tokens on mma.sync int8 (lp_gemm_i8_tiles.cu)
+size_t gemm_i8_tiles_scratch(uint32_t type, int M, int K, const int* ns, int n_mats, bool cut);
+int    launch_gemm_i8_tiles(uint8_t* scratch, bool cut, const float* x, const float* norm_w, float eps, float* x_norm_out, const uint8_t* const* ws, float* const* ys,
+                            const int* ns, int n_mats, uint32_t type, int M, int K, cudaStream_t st, const PeerOut* peers);
 // The same for Q4_K and Q6_K with more than 128 rows on pairs of SMs (lp_gemm_pair.cu)
 bool   gemm_pair_supports(uint32_t type, int M);
 size_t gemm_pair_scratch(uint32_t type, int M, int K, const int* ns, int n_mats, bool cut);

@@ -909,147 +909,6 @@ gemm_w2_sa_kernel(const __grid_constant__ SaMaps maps, const SaParams p, const S
 }  // namespace w2
 
 
-// ---- the same tiles on the warp-level int8 instruction ------------------------------------------------------------
-// Integer block sums of 128 weight rows x up to 128 tokens from mma.sync (super_block in lp_i8.cuh: one super-block of 32 weight
-// rows x 64 tokens per consumer warp), the fp32 scale chain in registers, results and pieces as in the kernels above. Dense calls only.
-// Bound by the FP32 pipe: the chain costs 12 cycles of it per 16 x 8 x 32 products, the MMA 8 cycles of the tensor pipe beside
-// it. The two-piece tcgen05 form needs four fp16 products a value and eight fp16 values written per packed one, which its
-// converter warps cannot feed. A producer warp fills three stages of one super-block: the packed rows by one tensor-map tile,
-// the quantized tokens by one bulk copy per eight.
-namespace i8t {
-
-constexpr int STAGES = 3, CONSUMERS = 8, THREADS = (CONSUMERS + 1) * 32;
-constexpr int PARTS = CONSUMERS / 4, NT = (TT / 8 + PARTS - 1) / PARTS;      // consumer warps side by side along the tokens, 8-token tiles of each
-template <uint32_t TYPE> using Geo = i8::GeoWide<TYPE>;
-template <uint32_t TYPE> struct Lay {
-    static constexpr uint32_t RAW = TW * Geo<TYPE>::PITCH, STAGE = RAW + TT / 8 * i8::Geo<TYPE>::ACT_BYTES,
-                              SMEM = 128 + STAGES * STAGE + 16;                        // + read-ahead of the unaligned loads
-};
-
-template <uint32_t TYPE, bool PEERS>
-__global__ void __launch_bounds__(THREADS, 1)
-gemm_i8_tile_kernel(const __grid_constant__ CUtensorMap wmap, const uint8_t* __restrict__ img, const SaParams p, const SaPeers<PEERS> pe) {
-    using G = Geo<TYPE>;
-    constexpr int PITCH = G::PITCH;
-    extern __shared__ __align__(128) uint8_t smem[];
-    static_assert(Lay<TYPE>::SMEM <= 227 * 1024, "shared memory budget");
-    const uint32_t sbase = smem_u32(smem), stage0 = sbase + 128;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    auto bar_full = [&](int s) { return sbase + 8 * s; };
-    auto bar_empty = [&](int s) { return sbase + 32 + 8 * s; };
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) { mbar_init(bar_full(s), 1); mbar_init(bar_empty(s), CONSUMERS); }
-        fence_barrier_init();
-    }
-    __syncthreads();
-    // the quantized tokens are the kernel's before this one, which this one's launch and set-up overlap
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const Segments sg = segments(p);
-    const int nsb = p.K / 256;
-
-    if (warp == CONSUMERS) {
-        int s = 0, issued = 0;
-        uint32_t phase = 0;
-        bool gave_up = false;
-        for (int seg = 0; seg < sg.n && !gave_up; ++seg) {
-            const TileRef tr = seg_ref(p, sg, seg);
-            const int nt = (tr.nt + 7) >> 3;
-            const uint8_t* act = img + static_cast<size_t>(tr.m0 >> 3) * nsb * G::ACT_BYTES;
-            for (int sb = tr.sb0; sb < tr.sb1; ++sb) {
-                bool free = true;
-                if (issued >= STAGES && lane == 0) free = mbar_wait_bounded(bar_empty(s), phase ^ 1);
-                if (!__shfl_sync(0xffffffffu, free, 0)) { gave_up = true; break; }
-                const uint32_t st = stage0 + s * Lay<TYPE>::STAGE;
-                if (lane == 0) {
-                    mbar_expect_tx(bar_full(s), Lay<TYPE>::RAW + nt * G::ACT_BYTES);
-                    tma_load_2d(st, &wmap, G::first_word(sb), tr.wrow0 + tr.n0, bar_full(s));
-                }
-                __syncwarp();
-                if (lane < nt)
-                    bulk_g2s(st + Lay<TYPE>::RAW + lane * G::ACT_BYTES, act + (static_cast<size_t>(lane) * nsb + sb) * G::ACT_BYTES, G::ACT_BYTES, bar_full(s));
-                ++issued;
-                if (++s == STAGES) { s = 0; phase ^= 1; }
-            }
-        }
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        if (gave_up && lane == 0) report_status(p.err, DEV_TIMEOUT_EMPTY);
-        // the copies in flight land before the CTA gives its shared memory back
-        const int pending = issued < STAGES ? issued : STAGES;
-        for (int k = 0; k < pending; ++k) {
-            if (s == 0) { s = STAGES; phase ^= 1; }
-            --s;
-            if (!mbar_wait_bounded(bar_full(s), phase) && lane == 0) report_status(p.err, DEV_TIMEOUT_DRAIN);
-        }
-        return;
-    }
-
-    const int wm = warp & 3, side = warp >> 2, gq = lane >> 2, tq = lane & 3;
-    int s = 0;
-    uint32_t phase = 0;
-    bool ok = true;
-    for (int seg = 0; seg < sg.n && ok; ++seg) {
-        const TileRef tr = seg_ref(p, sg, seg);
-        const int nt = (tr.nt + 7) >> 3, first = nt * side / PARTS;                     // 8-token tiles: of the tile, before this warp's
-        const int live = nt * (side + 1) / PARTS - first;
-        float2 acc[1][2][NT][2];
-#pragma unroll
-        for (int g = 0; g < 2; ++g)
-#pragma unroll
-            for (int t = 0; t < NT; ++t) acc[0][g][t][0] = acc[0][g][t][1] = make_float2(0.f, 0.f);
-        for (int sb = tr.sb0; sb < tr.sb1; ++sb) {
-            if (!mbar_wait_bounded(bar_full(s), phase)) { ok = false; break; }
-            const uint32_t st = stage0 + s * Lay<TYPE>::STAGE;
-            const uint32_t row = st + (32 * wm + gq) * PITCH + G::offset_in_unit(sb, 0), act = st + Lay<TYPE>::RAW + first * G::ACT_BYTES;
-            // a full tile's count known where the code is built lets the MMAs of one 8-token tile run under the chain of another
-            // (512 rows 2816 x 8448 Q8_0 84 -> 76 us); only for the types that run full tiles here, and not for every count: the
-            // instruction fetches cost more than it gives (Q4_K, 64 rows: 44.9 against 47.3 us)
-            if ((TYPE == LAPLACE_TYPE_Q8_0 || TYPE == LAPLACE_TYPE_Q4_0) && live == NT) i8::super_block<TYPE, PITCH, 2, NT>(row, act, G::ACT_BYTES, lane, NT, acc);
-            else i8::super_block<TYPE, PITCH, 2, NT>(row, act, G::ACT_BYTES, lane, live, acc);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_empty(s));
-            if (++s == STAGES) { s = 0; phase ^= 1; }
-        }
-        if (!ok) break;
-        // lane: weight rows gq and gq + 8 of two groups of 16, tokens 2 tq and 2 tq + 1 of every eight
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            if (t >= live) break;
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int col = 8 * (first + t) + 2 * tq + e;
-                if (col >= tr.nt) continue;
-                const int row = tr.m0 + col;
-                const float v[4] = {e ? acc[0][0][t][0].y : acc[0][0][t][0].x, e ? acc[0][0][t][1].y : acc[0][0][t][1].x, e ? acc[0][1][t][0].y : acc[0][1][t][0].x, e ? acc[0][1][t][1].y : acc[0][1][t][1].x};
-                if (tr.part >= 0) {
-                    float* part = p.y_part + static_cast<size_t>(tr.part) * (TT * TW) + col * TW + 32 * wm + gq;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) part[8 * k] = v[k];
-                    continue;
-                }
-                const int n = tr.n0 + 32 * wm + gq;
-                if constexpr (PEERS) {
-                    for (int r = 0; r < pe.n; ++r)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (n + 8 * k < p.N) pe.y[r][static_cast<size_t>(row) * pe.ld + pe.col0 + n + 8 * k] = v[k];
-                } else {
-                    // a dense call has no out_row; without these lines the compiler orders the loop above so that Q4_0 at 64 to 96 rows
-                    // takes 4 to 6 % longer (4096 x 14336, 96 rows: 50.0 -> 53.1 us)
-                    int orow = p.out_row ? __ldg(p.out_row + row) : row;
-                    if (p.out_identity && orow >= 0) orow = row;
-                    if (orow < 0) continue;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (n + 8 * k < p.N) p.y[static_cast<size_t>(orow) * p.N + n + 8 * k] = v[k];
-                }
-            }
-        }
-    }
-    if (!ok && lane == 0) report_status(p.err, DEV_TIMEOUT_FULL);       // the producer drains the copies
-}
-
-}  // namespace i8t
-
 // ---- activation quantizer ------------------------------------------------------------------
 // One CTA per activation row. The int8 values q and the block scales d are the reference's (Laplace
 // src/matmul_simd.cpp:348-410: d = amax / 127, q = rne(x * (1 / d)), sums from the unclamped integers); what is
@@ -1123,8 +982,6 @@ struct SaOperand {          // operand buffers of one matmul
     float*  g;              // [m_pad / 2][K / 16]: block sums of a pair of rows, interleaved
     float*  inv_s;          // [m_pad]
     int     m_pad;
-    // the int8 kernel's operand instead, in the same place (a third of its size): quantized rows in fragment order (lp_i8.cuh)
-    uint8_t* img() const { return reinterpret_cast<uint8_t*>(a); }
 };
 
 __global__ void __launch_bounds__(256) quantize_sa_kernel(const float* __restrict__ x, int K, SaOperand op) {
@@ -1247,7 +1104,6 @@ struct SaLaunch {
     int tiles_m, tiles_n, grid;
     long long sk_units; float* y_part;
     const PeerOut* peers;        // nullptr, or: the result goes to every GPU's buffer
-    bool i8;                     // on the int8 kernel (op.img())
 };
 
 // Which kernel a call's tiles run on. The int8 kernel needs rows that a tensor-map copy can address. Q4_0 and Q8_0 run on it for any
@@ -1258,47 +1114,6 @@ bool i8_tiles(uint32_t type, int M, int K, const uint8_t* const* ws, int n_mats)
     for (int i = 0; i < n_mats; ++i)
         if (reinterpret_cast<uintptr_t>(ws[i]) & 15) return false;
     return row_bytes(type, K) % 16 == 0;
-}
-
-template <uint32_t TYPE>
-int launch_i8_tiles(const CUtensorMap& map, const SaLaunch& L, const SaParams& p, const SaPeers<true>& pe, cudaStream_t st) {
-    using namespace i8t;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_i8_tile_kernel<TYPE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Lay<TYPE>::SMEM));
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_i8_tile_kernel<TYPE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(Lay<TYPE>::SMEM));
-        if (e != cudaSuccess) return cuda_check(e, "cudaFuncSetAttribute gemm_i8_tile");
-        configured = true;
-    }
-    const uint8_t* img = L.op.img();
-    return L.peers ? launch_early(gemm_i8_tile_kernel<TYPE, true>, dim3(L.grid), i8t::THREADS, Lay<TYPE>::SMEM, st, map, img, p, pe)
-                   : launch_early(gemm_i8_tile_kernel<TYPE, false>, dim3(L.grid), i8t::THREADS, Lay<TYPE>::SMEM, st, map, img, p, SaPeers<false>{});
-}
-int run_i8_kernel(const SaLaunch& L, const SaParams& p, const SaPeers<true>& pe, cudaStream_t st) {
-    const uint64_t rb = row_bytes(L.type, L.K);
-    int pitch;
-    switch (L.type) {
-        case LAPLACE_TYPE_Q4_K: pitch = i8t::Geo<LAPLACE_TYPE_Q4_K>::PITCH; break;
-        case LAPLACE_TYPE_Q4_0: pitch = i8t::Geo<LAPLACE_TYPE_Q4_0>::PITCH; break;
-        case LAPLACE_TYPE_Q8_0: pitch = i8t::Geo<LAPLACE_TYPE_Q8_0>::PITCH; break;
-        default: pitch = i8t::Geo<LAPLACE_TYPE_Q6_K>::PITCH; break;
-    }
-    CUtensorMap map;
-    if (!make_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, L.w, rb / 4, static_cast<uint64_t>(L.w_rows), rb, pitch / 4, TW, CU_TENSOR_MAP_SWIZZLE_NONE, "weights"))
-        return LAPLACE_ERR_CUDA;
-    int rc;
-    switch (L.type) {
-        case LAPLACE_TYPE_Q4_K: rc = launch_i8_tiles<LAPLACE_TYPE_Q4_K>(map, L, p, pe, st); break;
-        case LAPLACE_TYPE_Q4_0: rc = launch_i8_tiles<LAPLACE_TYPE_Q4_0>(map, L, p, pe, st); break;
-        case LAPLACE_TYPE_Q8_0: rc = launch_i8_tiles<LAPLACE_TYPE_Q8_0>(map, L, p, pe, st); break;
-        case LAPLACE_TYPE_Q6_K: rc = launch_i8_tiles<LAPLACE_TYPE_Q6_K>(map, L, p, pe, st); break;
-        default: return LAPLACE_UNSUPPORTED;
-    }
-    if (rc) return rc;
-    ctx().launches++;
-    ctx().last_path = 2;
-    ctx().last_kernel = KERNEL_INT8_TILES;
-    return cuda_check(cudaGetLastError(), "gemm_i8_tile launch");
 }
 
 int run_sa_kernel(const SaLaunch& L, cudaStream_t st) {
@@ -1317,7 +1132,6 @@ int run_sa_kernel(const SaLaunch& L, cudaStream_t st) {
         pe.n = L.peers->world; pe.ld = L.peers->ld; pe.col0 = L.peers->col0;
     }
     if (L.peers && (L.out_row || L.tile_tab)) return fail(LAPLACE_ERR_STATE, "gemm_sa: the peer-store form takes a plain dense call");
-    if (L.i8) return L.out_row || L.tile_tab ? fail(LAPLACE_ERR_STATE, "gemm_sa: the int8 tiles take a plain dense call") : run_i8_kernel(L, p, pe, st);
     SaMaps maps;
     for (int bk = 0; bk < 4; ++bk) {
         if (!make_map_2d(&maps.a[bk], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, L.op.a, static_cast<uint64_t>(K), 2ull * L.op.m_pad,
@@ -1436,9 +1250,8 @@ int check_args(const float* x, const uint8_t* w, uint32_t type, int M, int K, in
     return LAPLACE_OK;
 }
 
-// The quantized (optionally normalised) rows as the operand of the kernel that the call runs on.
-int launch_operand(bool i8, const float* x, const float* norm_w, float eps, float* x_norm_out, uint32_t type, int M, int K, const SaOperand& op, cudaStream_t st) {
-    if (i8) return launch_quantize_i8(x, norm_w, eps, x_norm_out, type, M, K, op.img(), st);
+// The quantized (optionally normalised) rows as the kernel's operand.
+int launch_operand(const float* x, const float* norm_w, float eps, float* x_norm_out, int M, int K, const SaOperand& op, cudaStream_t st) {
     if (norm_w) quantize_sa_norm_kernel<<<M, 256, 0, st>>>(x, norm_w, eps, x_norm_out, K, op);
     else quantize_sa_kernel<<<M, 256, 0, st>>>(x, K, op);
     ctx().launches++;
@@ -1446,17 +1259,16 @@ int launch_operand(bool i8, const float* x, const float* norm_w, float eps, floa
 }
 
 // Quantizes x into `scratch` (device memory of at least pl.total() bytes, 256-byte aligned) and runs the kernel.
-int gemm_sa_on_scratch(uint8_t* scratch, const SaPlan& pl, bool i8, const float* x, const uint8_t* w, uint32_t type, float* y, int M, int K, int N,
+int gemm_sa_on_scratch(uint8_t* scratch, const SaPlan& pl, const float* x, const uint8_t* w, uint32_t type, float* y, int M, int K, int N,
                        cudaStream_t st, const PeerOut* peers = nullptr) {
     Context& c = ctx();
     int rc;
     uint8_t* s = scratch;
     const SaOperand op = carve_operand(s, pl.m_pad, K);
     if (x) {                          // nullptr: the operand is in place already (several matrices share one input)
-        if ((rc = launch_operand(i8, x, nullptr, 0.f, nullptr, type, M, K, op, st))) return rc;
+        if ((rc = launch_operand(x, nullptr, 0.f, nullptr, M, K, op, st))) return rc;
     }
     SaLaunch L{};
-    L.i8 = i8;
     L.w = w; L.type = type; L.y = y; L.M = M; L.K = K; L.N = N; L.w_rows = N; L.op = op;
     L.tiles_m = pl.tiles_m; L.tiles_n = pl.tiles_n;
     L.sk_units = pl.sp.units;
@@ -1486,13 +1298,17 @@ int gemm_sa_on_scratch(uint8_t* scratch, const SaPlan& pl, bool i8, const float*
 int launch_gemm_sa(const float* x, const uint8_t* w, uint32_t type, float* y, int M, int K, int N, cudaStream_t st) {
     int rc = check_args(x, w, type, M, K, N);
     if (rc) return rc;
+    if (i8_tiles(type, M, K, &w, 1)) {
+        if ((rc = g_scratch.ensure(gemm_i8_tiles_scratch(type, M, K, &N, 1, true), st))) return rc;
+        return launch_gemm_i8_tiles(static_cast<uint8_t*>(g_scratch.p), true, x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, nullptr);
+    }
     if (gemm_pair_supports(type, M)) {
         if ((rc = g_scratch.ensure(gemm_pair_scratch(type, M, K, &N, 1, true), st))) return rc;
         return launch_gemm_pair(static_cast<uint8_t*>(g_scratch.p), true, x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, nullptr);
     }
     const SaPlan pl = plan_sa(M, K, N, true);
     if ((rc = g_scratch.ensure(pl.total(), st))) return rc;
-    return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, i8_tiles(type, M, K, &w, 1), x, w, type, y, M, K, N, st);
+    return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, x, w, type, y, M, K, N, st);
 }
 
 // Several matrices of one type and K against the same input rows (q / k / v, gate / up of src/arch_llama.cpp:475-499): the
@@ -1508,20 +1324,23 @@ int launch_gemm_sa_multi(const float* x, const float* norm_w, float eps, float* 
     }
     if (norm_w && ((reinterpret_cast<uintptr_t>(norm_w) & 15) || (x_norm_out && (reinterpret_cast<uintptr_t>(x_norm_out) & 15))))
         return fail(LAPLACE_ERR_ARG, "gemm_multi: the norm weights (and the optional output) must be 16-byte aligned");
+    if (i8_tiles(type, M, K, ws, n_mats)) {
+        if ((rc = g_scratch.ensure(gemm_i8_tiles_scratch(type, M, K, ns, n_mats, true), st))) return rc;
+        return launch_gemm_i8_tiles(static_cast<uint8_t*>(g_scratch.p), true, x, norm_w, eps, x_norm_out, ws, ys, ns, n_mats, type, M, K, st, nullptr);
+    }
     if (gemm_pair_supports(type, M)) {
         if ((rc = g_scratch.ensure(gemm_pair_scratch(type, M, K, ns, n_mats, true), st))) return rc;
         return launch_gemm_pair(static_cast<uint8_t*>(g_scratch.p), true, x, norm_w, eps, x_norm_out, ws, ys, ns, n_mats, type, M, K, st, nullptr);
     }
     if ((rc = g_scratch.ensure(need, st))) return rc;
     uint8_t* scratch = static_cast<uint8_t*>(g_scratch.p);
-    const bool i8 = i8_tiles(type, M, K, ws, n_mats);
     {
         uint8_t* s = scratch;
         const SaOperand op = carve_operand(s, plan_sa(M, K, ns[0], true).m_pad, K);
-        if ((rc = launch_operand(i8, x, norm_w, eps, x_norm_out, type, M, K, op, st))) return rc;
+        if ((rc = launch_operand(x, norm_w, eps, x_norm_out, M, K, op, st))) return rc;
     }
     for (int i = 0; i < n_mats; ++i)
-        if ((rc = gemm_sa_on_scratch(scratch, plan_sa(M, K, ns[i], true), i8, nullptr, ws[i], type, ys[i], M, K, ns[i], st))) return rc;
+        if ((rc = gemm_sa_on_scratch(scratch, plan_sa(M, K, ns[i], true), nullptr, ws[i], type, ys[i], M, K, ns[i], st))) return rc;
     return LAPLACE_OK;
 }
 
@@ -1531,13 +1350,17 @@ int launch_gemm_sa_multi(const float* x, const float* norm_w, float eps, float* 
 int launch_gemm_sa_peers(const float* x, const uint8_t* w, uint32_t type, const PeerOut& po, int M, int K, int N, cudaStream_t st) {
     int rc = check_args(x, w, type, M, K, N);
     if (rc) return rc;
+    if (i8_tiles(type, M, K, &w, 1)) {
+        if ((rc = g_scratch.ensure(gemm_i8_tiles_scratch(type, M, K, &N, 1, true), st))) return rc;
+        return launch_gemm_i8_tiles(static_cast<uint8_t*>(g_scratch.p), true, x, nullptr, 0.f, nullptr, &w, nullptr, &N, 1, type, M, K, st, &po);
+    }
     if (gemm_pair_supports(type, M)) {
         if ((rc = g_scratch.ensure(gemm_pair_scratch(type, M, K, &N, 1, true), st))) return rc;
         return launch_gemm_pair(static_cast<uint8_t*>(g_scratch.p), true, x, nullptr, 0.f, nullptr, &w, nullptr, &N, 1, type, M, K, st, &po);
     }
     const SaPlan pl = plan_sa(M, K, N, true);
     if ((rc = g_scratch.ensure(pl.total(), st))) return rc;
-    return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, i8_tiles(type, M, K, &w, 1), x, w, type, nullptr, M, K, N, st, &po);
+    return gemm_sa_on_scratch(static_cast<uint8_t*>(g_scratch.p), pl, x, w, type, nullptr, M, K, N, st, &po);
 }
 
 // laplace_cuda_gemm_dev for more than 8 rows on scratch memory the caller owns (`cap` bytes at `scratch`, 256-byte aligned);
@@ -1551,14 +1374,18 @@ int launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const 
     if (pl.total() > cap) pl = plan_sa(M, K, N, false);
     if (pl.total() > cap)
         return fail(LAPLACE_ERR_LIMIT, "gemm: M=%d K=%d needs %zu bytes of scratch, the caller's area holds %zu", M, K, pl.total(), cap);
+    // a handful of rows: a twelfth of that operand at most, but the limit stays one formula for every row count
+    if (gemm_i8_supports(type, M, K, &w, 1, N)) return launch_gemm_i8(x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, scratch);
+    if (i8_tiles(type, M, K, &w, 1)) {
+        const bool cut = gemm_i8_tiles_scratch(type, M, K, &N, 1, true) <= cap;       // the operand alone always fits: a quarter of the one above
+        return launch_gemm_i8_tiles(scratch, cut, x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, nullptr);
+    }
     if (gemm_pair_supports(type, M)) {
         const bool cut = gemm_pair_scratch(type, M, K, &N, 1, true) <= cap;
         if (gemm_pair_scratch(type, M, K, &N, 1, cut) <= cap)       // always: its operand is smaller than the one above
             return launch_gemm_pair(scratch, cut, x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, nullptr);
     }
-    // a handful of rows: a twelfth of that operand at most, but the limit stays one formula for every row count
-    if (gemm_i8_supports(type, M, K, &w, 1, N)) return launch_gemm_i8(x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, scratch);
-    return gemm_sa_on_scratch(scratch, pl, i8_tiles(type, M, K, &w, 1), x, w, type, y, M, K, N, st);
+    return gemm_sa_on_scratch(scratch, pl, x, w, type, y, M, K, N, st);
 }
 
 
