@@ -9,15 +9,19 @@
 // two activation rows per packed instruction. The accumulator operand of the MMA is the bit pattern of 1.5 * 2^23, so that the
 // integer result read as a float is 1.5 * 2^23 + U exactly (|U| < 2^22): one packed subtraction instead of two conversions.
 //
-// Shape of the kernel (one CTA per SM, sixteen consumer warps and two copy warps):
+// Shape of the kernel (one CTA per SM, sixteen consumer warps, two copy warps, two that add up):
 //   * K is cut over a cluster of up to eight CTAs, so that a CTA needs its part of the quantized activations only (they stay
 //     in shared memory for the whole call) and a long-K matrix with few rows still occupies every SM. The cut depends on
 //     K, type and row count (see plan_dense), so a matrix has the same bits alone and beside others on this kernel;
 //   * every consumer warp takes groups of 16 weight rows for itself (two warps share a group when the CTA's part of K is
 //     eight super-blocks or more): its copies are 2-D tensor-map tiles of 16 rows x one or two super-blocks into a ring of
 //     its own, so that warps never wait for one another while they stream;
-//   * the partial results of a cluster meet in shared memory, are added in a fixed order through distributed shared
-//     memory and written once, coalesced. No scratch in device memory and no second launch;
+//   * the partial results of a row group go to one CTA of the cluster by asynchronous stores that a barrier there counts (no fence,
+//     no wait on the sender's side); two warps of that CTA add them up in a fixed order and write them once, while the others
+//     stream on. With all warps of the cluster meeting after every sixteen to thirty-two row groups instead, a quarter of the
+//     warps' time went into that (24 rows, Q4_K 4096 x 28672: 36 % of the issue slots used): 46.1 -> 32.9 us, 16 rows 36.5 -> 25.7,
+//     8 rows 20.1 -> 18.8, Q6_K 14336 x 4096, 24 rows 40.6 -> 38.2. One adding warp: 34.3, 27.3 and 21.1 us. No scratch in device
+//     memory and no second launch;
 //   * with up to 8 activation rows every CTA quantizes its part of the rows itself (with the RMSNorm in front when asked for,
 //     the row sums meeting through distributed shared memory); with more rows, and for experts, a small kernel writes the
 //     quantized rows in fragment order into device scratch and the CTAs fetch their part with bulk copies.
@@ -36,15 +40,18 @@ constexpr int PW = 2;                      // copy warps: lane l of warp i serve
 constexpr int THREADS = (CW + PW) * 32;
 constexpr int MAX_SLOTS = 8;
 constexpr int MAX_MATS = 8;
-// partial results of a row group: [activation row][16 weight rows], every second pair of activation rows with its halves swapped
-// (the stores of a warp then meet two-way bank conflicts, not four-way)
-__device__ __forceinline__ int slab_at(int tok, int row) { return tok * 16 + (row ^ ((tok & 2) << 2)); }
+constexpr int MAX_PARTS = 8;               // row groups whose partial results a CTA of a cluster holds at a time
+constexpr int RW = 2;                      // warps of a CTA that add up, group i of the CTA's by warp i mod RW
+constexpr int PART_BYTES = 512;            // partial results of 16 weight rows x 8 activation rows, in the order in which the lanes hold them
 
 // Shared memory: barriers, row sums of the norm, then the activations, the partial results, the rings.
 constexpr uint32_t OFF_BAR_FULL = 0, OFF_BAR_EMPTY = OFF_BAR_FULL + CW * MAX_SLOTS * 8, OFF_BAR_MISC = OFF_BAR_EMPTY + CW * MAX_SLOTS * 8,
-                   OFF_RED = OFF_BAR_MISC + 128, OFF_ACT = OFF_RED + 128;
+                   OFF_RED = OFF_BAR_MISC + 256, OFF_ACT = OFF_RED + 128;
 static_assert(OFF_ACT % 128 == 0, "bulk copies land on 128-byte boundaries");
-constexpr uint32_t BAR_ACT = 0, BAR_ACT_EMPTY = 16, BAR_NORM = 32, BAR_SLAB_FULL = 40, BAR_SLAB_FREE = 48;       // inside OFF_BAR_MISC; BAR_ACT*: two each
+// inside OFF_BAR_MISC; BAR_ACT*: two each, BAR_PART: MAX_PARTS, TAKEN: RW words for every CTA of the cluster
+constexpr uint32_t BAR_ACT = 0, BAR_ACT_EMPTY = 16, BAR_NORM = 32, BAR_NORM_READ = 40, BAR_PART = 64, TAKEN = BAR_PART + 8 * MAX_PARTS;
+static_assert(RW == 2 && MAX_PARTS % RW == 0, "places are dealt to the adding warps");
+static_assert(TAKEN + 8 * RW * 4 <= 256, "barrier area");
 
 struct I8Params {
     const float*   x;              // M <= 8: fp32 rows, quantized by every CTA
@@ -59,9 +66,8 @@ struct I8Params {
     int            mat_end[MAX_MATS];      // rows of the matrices one behind the other: where each ends
     int            total_rows;
     int            kw;                     // warps that share a row group
-    int            panel_rows;             // rows whose partial results shared memory holds
-    int            slab_groups;            // row groups of a panel that one CTA adds up, at most
-    uint32_t       off_slab, off_ring;
+    int            n_parts;                // row groups whose partial results shared memory holds: 1 or a multiple of RW, at most MAX_PARTS
+    uint32_t       off_part, off_ring;
     int            n_slots;
     // experts
     const int4*    tile_tab;               // {first activation row, first weight row inside the expert, the expert's first row, tokens}
@@ -88,7 +94,11 @@ __device__ __forceinline__ float ld_remote(uint32_t addr) {
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_remote(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(addr), "f"(v) : "memory"); }
+// 16 bytes into another CTA's shared memory, counted by a barrier there: no fence, nothing to wait for on this side
+__device__ __forceinline__ void st_remote_counted(uint32_t addr, uint32_t bar, float a, float b, float c, float d) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%2, %3, %4, %5}, [%1];"
+                 :: "r"(addr), "r"(bar), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
 __device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity) {
     for (uint32_t it = 0; it < (1u << 22); ++it) {
         uint32_t ok;
@@ -99,33 +109,48 @@ __device__ __forceinline__ bool wait_cluster(uint32_t bar, uint32_t parity) {
     return false;
 }
 
-// The row groups of a panel [p0, p1) of the concatenated rows, 16 rows each, cut at matrix boundaries.
-struct Group { int mat, row, rows, at; };          // matrix, first row inside it, live rows, first row among the concatenated ones
-__device__ __forceinline__ int panel_groups(const I8Params& p, int p0, int p1) {
+__device__ __forceinline__ bool wait_taken(uint32_t addr, int count) {
+    for (uint32_t it = 0; it < (1u << 22); ++it) {
+        int v;
+        asm volatile("ld.acquire.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+        if (v >= count) return true;
+        if (it > 16) __nanosleep(200);
+    }
+    return false;
+}
+__device__ __forceinline__ float4 lds_f4(uint32_t addr) {
+    const uint4 v = lds128(addr);
+    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+// The row groups of rows [r0, r1) of the concatenated ones, 16 rows each, cut at matrix boundaries.
+struct Group { int mat, row, rows; };              // matrix, first row inside it, live rows
+__device__ __forceinline__ int row_groups(const I8Params& p, int r0, int r1) {
     int n = 0;
     for (int i = 0, b = 0; i < p.n_mats; ++i) {
-        const int lo = p0 > b ? p0 : b, hi = p1 < p.mat_end[i] ? p1 : p.mat_end[i];
+        const int lo = r0 > b ? r0 : b, hi = r1 < p.mat_end[i] ? r1 : p.mat_end[i];
         if (hi > lo) n += (hi - lo + 15) >> 4;
         b = p.mat_end[i];
     }
     return n;
 }
-__device__ __forceinline__ Group panel_group(const I8Params& p, int p0, int p1, int g) {
+__device__ __forceinline__ Group row_group(const I8Params& p, int r0, int r1, int g) {
     for (int i = 0, b = 0; i < p.n_mats; ++i) {
-        const int lo = p0 > b ? p0 : b, hi = p1 < p.mat_end[i] ? p1 : p.mat_end[i];
+        const int lo = r0 > b ? r0 : b, hi = r1 < p.mat_end[i] ? r1 : p.mat_end[i];
         if (hi > lo) {
             const int n = (hi - lo + 15) >> 4;
-            if (g < n) { const int at = lo + 16 * g; return {i, at - b, hi - at < 16 ? hi - at : 16, at}; }
+            if (g < n) { const int at = lo + 16 * g; return {i, at - b, hi - at < 16 ? hi - at : 16}; }
             g -= n;
         }
         b = p.mat_end[i];
     }
-    return {0, 0, 0, 0};
+    return {0, 0, 0};
 }
 
 // QUANT: the CTA quantizes the (at most 8) activation rows itself. MOE: jobs from the table, whole K, results straight to y.
 template <uint32_t TYPE, int NT, int C, bool QUANT, bool MOE>
-__global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_constant__ I8Maps maps, const I8Params p) {
+__global__ void __launch_bounds__(THREADS + (C > 1 ? 32 * RW : 0), 1) gemm_i8_kernel(const __grid_constant__ I8Maps maps, const I8Params p) {
     using G = Geo<TYPE>;
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t sbase = smem_u32(smem);
@@ -142,8 +167,9 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
     if (threadIdx.x == CW) {
         for (int b = 0; b < 2; ++b) { mbar_init(misc(BAR_ACT + 8 * b), 1); mbar_init(misc(BAR_ACT_EMPTY + 8 * b), CW); }
         mbar_init(misc(BAR_NORM), C);
-        mbar_init(misc(BAR_SLAB_FULL), C * CW);
-        mbar_init(misc(BAR_SLAB_FREE), C * CW);
+        mbar_init(misc(BAR_NORM_READ), C);
+        for (int b = 0; b < MAX_PARTS; ++b) mbar_init(misc(BAR_PART + 8 * b), 1);
+        for (int r = 0; r < C * RW; ++r) reinterpret_cast<volatile uint32_t*>(smem + OFF_BAR_MISC + TAKEN)[r] = 0u;
     }
     fence_barrier_init();
     __syncthreads();
@@ -159,6 +185,66 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
     const int sb0 = p.nsb * rank / C, sb1 = p.nsb * (rank + 1) / C;
     const int lanes = CW / p.kw;                                   // row groups in work at a time
 
+    if (C > 1 && warp >= CW + PW) {
+        // ------------------------------ adds up the partial results of the cluster: row groups rank, rank + C, ... ------------------------------
+        // [group in work][rank and warp they come from][tile][lane]; a barrier counts a group's bytes. The consumer warps go on meanwhile.
+        const int ng = row_groups(p, r0, r1), n = ng > rank ? (ng - rank + C - 1) / C : 0, n_src = C * p.kw;
+        const uint32_t src_bytes = NT * PART_BYTES, group_bytes = static_cast<uint32_t>(n_src) * src_bytes;
+        const int gq = lane >> 2, tq = lane & 3, rw = warp - (CW + PW), step = p.n_parts == 1 ? 1 : RW;
+        // a place always belongs to the same warp, which meets every phase of its barrier
+        if (lane < p.n_parts && lane < n && lane % step == rw) mbar_expect_tx(misc(BAR_PART + 8 * lane), group_bytes);
+        __syncwarp();
+        asm volatile("griddepcontrol.wait;" ::: "memory");             // y may be read by the kernel before this one
+        bool ok = true;
+        for (int i = rw, at = rw, phase = 0; rw < step && i < n; i += step) {
+            const uint32_t src = sbase + p.off_part + static_cast<uint32_t>(at) * group_bytes + lane * 16;
+            const Group gr = row_group(p, r0, r1, i * C + rank);
+            const size_t ld = p.mat_end[gr.mat] - (gr.mat ? p.mat_end[gr.mat - 1] : 0);
+            float* y = p.mat_y[gr.mat] + gr.row + gq;
+            if (!wait_cluster(misc(BAR_PART + 8 * at), phase)) { ok = false; break; }
+            float4 v[NT];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                float4 part[C];                                        // of the CTAs, added in pairs
+#pragma unroll
+                for (int r = 0; r < C; ++r) {
+                    const uint32_t a = src + t * PART_BYTES + (p.kw == 2 ? 2 * r : r) * src_bytes;
+                    part[r] = lds_f4(a);
+                    if (p.kw == 2) part[r] = add4(part[r], lds_f4(a + src_bytes));
+                }
+#pragma unroll
+                for (int o = 1; o < C; o *= 2)
+#pragma unroll
+                    for (int r = 0; r < C; r += 2 * o) part[r] = add4(part[r], part[r + o]);
+                v[t] = part[0];
+            }
+            __syncwarp();
+            if (i + p.n_parts < n) {                                   // the place may take a group further on
+                if (lane == 0) mbar_expect_tx(misc(BAR_PART + 8 * at), group_bytes);
+                __syncwarp();
+                if (lane < C)
+                    asm volatile("st.release.cluster.shared::cluster.u32 [%0], %1;" :: "r"(map_rank(misc(TAKEN + 4 * (rank * RW + rw)), lane)), "r"(i + 1) : "memory");
+            }
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const int m = 8 * t + 2 * tq;
+                float* ym = y + m * ld;
+                if (m < p.M) {
+                    if (gq < gr.rows) ym[0] = v[t].x;
+                    if (gq + 8 < gr.rows) ym[8] = v[t].z;
+                }
+                if (m + 1 < p.M) {
+                    if (gq < gr.rows) ym[ld] = v[t].y;
+                    if (gq + 8 < gr.rows) ym[ld + 8] = v[t].w;
+                }
+            }
+            if ((at += step) >= p.n_parts) { at = rw; phase ^= 1; }
+        }
+        // the other CTAs have read this one's row sums
+        if (QUANT && rw == 0 && p.norm_w && !wait_cluster(misc(BAR_NORM_READ), 0)) ok = false;
+        if (!ok && lane == 0) report_status(p.err, DEV_TIMEOUT_FULL);
+        return;
+    }
     if (warp >= CW) {
         // ------------------------------ copy warps: a lane walks the units of one consumer warp ------------------------------
         if constexpr (MOE) asm volatile("griddepcontrol.wait;" ::: "memory");        // the job table is written by the kernel before
@@ -188,13 +274,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
             } else {
                 const int part = w / lanes, gl = w - part * lanes, len = sb1 - sb0;
                 const int s0 = sb0 + len * part / p.kw, s1 = sb0 + len * (part + 1) / p.kw;
-                for (int p0 = r0; p0 < r1 && !gave_up; p0 += p.panel_rows) {
-                    const int p1 = p0 + p.panel_rows < r1 ? p0 + p.panel_rows : r1;
-                    const int ng = panel_groups(p, p0, p1);
-                    for (int g = gl; g < ng && !gave_up; g += lanes) {
-                        const Group gr = panel_group(p, p0, p1, g);
-                        for (int sb = s0; sb < s1 && !gave_up; sb += G::UNIT_SB) copy(&maps.w[gr.mat], sb, gr.row);
-                    }
+                const int ng = row_groups(p, r0, r1);
+                for (int g = gl; g < ng && !gave_up; g += lanes) {
+                    const Group gr = row_group(p, r0, r1, g);
+                    for (int sb = s0; sb < s1 && !gave_up; sb += G::UNIT_SB) copy(&maps.w[gr.mat], sb, gr.row);
                 }
             }
         } else if (act_lane) {
@@ -320,6 +403,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
             }
         }
         named_bar_sync(1, CW * 32);
+        if (C > 1 && p.norm_w && threadIdx.x < C) arrive_remote(map_rank(misc(BAR_NORM_READ), threadIdx.x));
     } else if constexpr (!MOE) {
         if (!mbar_wait_bounded(misc(BAR_ACT), 0)) ok = false;
     }
@@ -406,68 +490,37 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_i8_kernel(const __grid_consta
         const int s0 = sb0 + len * part / p.kw, s1 = sb0 + len * (part + 1) / p.kw;
         const uint32_t act_stride = static_cast<uint32_t>(len) * G::ACT_BYTES;
         const uint32_t act = sbase + OFF_ACT + static_cast<uint32_t>(s0 - sb0) * G::ACT_BYTES;
-        // Partial results go to the CTA of the cluster that adds them up, row group g of a panel to rank g mod C:
-        // [rank they come from][warp of the group][g / C][slab_at].
-        const uint32_t slab = sbase + p.off_slab;
-        int panel = 0;
-        for (int p0 = r0; p0 < r1; p0 += p.panel_rows, ++panel) {
-            const int p1 = p0 + p.panel_rows < r1 ? p0 + p.panel_rows : r1;
-            const int ng = panel_groups(p, p0, p1);
-            if (C > 1 && panel > 0 && !wait_cluster(misc(BAR_SLAB_FREE), (panel - 1) & 1)) ok = false;
-            for (int g = gl; g < ng && ok; g += lanes) {
-                const Group gr = panel_group(p, p0, p1, g);
-                float2 acc[1][1][NT][2];
+        // Partial results go to the CTA of the cluster that adds them up, row group g to rank g mod C.
+        const uint32_t src_at = static_cast<uint32_t>((rank * p.kw + part) * NT * PART_BYTES + lane * 16), group_bytes = static_cast<uint32_t>(C * p.kw * NT * PART_BYTES);
+        const int ng = row_groups(p, r0, r1);
+        for (int g = gl; g < ng && ok; g += lanes) {
+            float2 acc[1][1][NT][2];
 #pragma unroll
-                for (int i = 0; i < NT; ++i) acc[0][0][i][0] = acc[0][0][i][1] = make_float2(0.f, 0.f);
-                run_group(Tag<NT>{}, s0, s1, act, act_stride, acc);
-                if constexpr (C == 1) {                          // whole K: straight to y
-                    float* y = p.mat_y[gr.mat] + gr.row + gq;
-                    const int n = p.mat_end[gr.mat] - (gr.mat ? p.mat_end[gr.mat - 1] : 0);
+            for (int i = 0; i < NT; ++i) acc[0][0][i][0] = acc[0][0][i][1] = make_float2(0.f, 0.f);
+            run_group(Tag<NT>{}, s0, s1, act, act_stride, acc);
+            if constexpr (C == 1) {                          // whole K: straight to y
+                const Group gr = row_group(p, r0, r1, g);
+                float* y = p.mat_y[gr.mat] + gr.row + gq;
+                const int n = p.mat_end[gr.mat] - (gr.mat ? p.mat_end[gr.mat - 1] : 0);
 #pragma unroll
-                    for (int i = 0; i < NT; ++i)
+                for (int i = 0; i < NT; ++i)
 #pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const int tok = 8 * i + 2 * tq + e;
-                            if (tok >= p.M) continue;
-                            if (gq < gr.rows) y[static_cast<size_t>(tok) * n] = e ? acc[0][0][i][0].y : acc[0][0][i][0].x;
-                            if (gq + 8 < gr.rows) y[static_cast<size_t>(tok) * n + 8] = e ? acc[0][0][i][1].y : acc[0][0][i][1].x;
-                        }
-                } else {
-                    const int at = ((rank * p.kw + part) * p.slab_groups + g / C) * (8 * NT * 16) + slab_at(2 * tq, gq), at8 = at ^ 8;
-                    const uint32_t dst = map_rank(slab + static_cast<uint32_t>(at) * 4, g % C), dst8 = dst + (at8 - at) * 4;
-#pragma unroll
-                    for (int i = 0; i < NT; ++i) {
-                        st_remote(dst + (8 * i * 16) * 4, acc[0][0][i][0].x);
-                        st_remote(dst + (8 * i * 16 + 16) * 4, acc[0][0][i][0].y);
-                        st_remote(dst8 + (8 * i * 16) * 4, acc[0][0][i][1].x);
-                        st_remote(dst8 + (8 * i * 16 + 16) * 4, acc[0][0][i][1].y);
+                    for (int e = 0; e < 2; ++e) {
+                        const int tok = 8 * i + 2 * tq + e;
+                        if (tok >= p.M) continue;
+                        if (gq < gr.rows) y[static_cast<size_t>(tok) * n] = e ? acc[0][0][i][0].y : acc[0][0][i][0].x;
+                        if (gq + 8 < gr.rows) y[static_cast<size_t>(tok) * n + 8] = e ? acc[0][0][i][1].y : acc[0][0][i][1].x;
                     }
-                }
-            }
-            if constexpr (C > 1) {
-                // every warp of the cluster is done with the panel; each CTA adds up and writes its row groups
-                __syncwarp();
-                if (lane < C) arrive_remote(map_rank(misc(BAR_SLAB_FULL), lane));
-                if (!wait_cluster(misc(BAR_SLAB_FULL), panel & 1)) ok = false;
-                const float* mine = reinterpret_cast<const float*>(smem + p.off_slab);
-                const int per_src = p.slab_groups * 8 * NT * 16, items = (ng > rank ? (ng - rank + C - 1) / C : 0) * p.M * 16;
-                for (int i = threadIdx.x; i < items; i += CW * 32) {
-                    const int row = i & 15, gm = i >> 4, gi = gm / p.M, m = gm - gi * p.M;
-                    const float* src = mine + gi * (8 * NT * 16) + slab_at(m, row);
-                    float part[C];                          // of the CTAs, added in pairs
+            } else {
+                if (!ok) break;
+                const int owner = g % C, gi = g / C, at = gi % p.n_parts;
+                // the place is free once that CTA has taken the group n_parts before (it takes them in order)
+                if (gi >= p.n_parts && !wait_taken(misc(TAKEN + 4 * (owner * RW + (p.n_parts == 1 ? 0 : at % RW))), gi - p.n_parts + 1)) { ok = false; break; }
+                const uint32_t dst = map_rank(sbase + p.off_part + static_cast<uint32_t>(at) * group_bytes + src_at, owner);
+                const uint32_t bar = map_rank(misc(BAR_PART + 8 * at), owner);
 #pragma unroll
-                    for (int r = 0; r < C; ++r) part[r] = p.kw == 2 ? src[2 * r * per_src] + src[(2 * r + 1) * per_src] : src[r * per_src];
-#pragma unroll
-                    for (int o = 1; o < C; o *= 2)
-#pragma unroll
-                        for (int r = 0; r < C; r += 2 * o) part[r] += part[r + o];
-                    const float v = part[0];
-                    const Group gr = panel_group(p, p0, p1, gi * C + rank);
-                    const int n = p.mat_end[gr.mat] - (gr.mat ? p.mat_end[gr.mat - 1] : 0);
-                    if (row < gr.rows) p.mat_y[gr.mat][static_cast<size_t>(m) * n + gr.row + row] = v;
-                }
-                __syncwarp();
-                if (p1 < r1 && lane < C) arrive_remote(map_rank(misc(BAR_SLAB_FREE), lane));       // the area may take the next panel
+                for (int i = 0; i < NT; ++i)
+                    st_remote_counted(dst + i * PART_BYTES, bar, acc[0][0][i][0].x, acc[0][0][i][0].y, acc[0][0][i][1].x, acc[0][0][i][1].y);
             }
         }
     }
@@ -521,7 +574,7 @@ bool type_geo(uint32_t type, TypeGeo& g) {
 }
 
 constexpr int MAX_NT = 4;
-struct DensePlan { int nt, c, kw, smax, n_slots; uint32_t act, slab_budget; };
+struct DensePlan { int nt, c, kw, smax, n_slots; uint32_t act, part_budget; };
 
 // How K is cut: by K, type and row count, except for Q4_K with 3 to 8 rows and few weight rows. A CTA of the cluster gets two super-blocks
 // or more; eight CTAs where the activations of four would not leave room for two ring slots a warp. False: the plan does not fit,
@@ -540,13 +593,13 @@ bool plan_dense(uint32_t type, int M, int K, long long rows, DensePlan& d) {
         d.kw = d.smax >= 8 ? 2 : 1;
         d.act = (static_cast<uint32_t>(d.nt * d.smax * g.act_bytes) + 127u) & ~127u;
         // Two ring slots a warp; then partial results, a row group taking kw x 8 nt x 16 floats: two rounds of row groups, at least
-        // half a round, and more groups than matrices; then more slots.
+        // half a round and one place in every CTA; then more slots.
         const long long slot = static_cast<long long>(CW) * 16 * g.pitch, group = d.kw * 8 * d.nt * 16 * 4, round = CW / d.kw * group;
-        long long rest = static_cast<long long>(ctx().smem_optin) - OFF_ACT - d.act - 256 - 2 * slot;
+        long long rest = static_cast<long long>(ctx().smem_optin) - OFF_ACT - d.act - 128 - 2 * slot;
         const long long least = c == 1 ? 0 : (round / 2 > (MAX_MATS + 1) * group ? round / 2 : (MAX_MATS + 1) * group), most = c == 1 ? 0 : 2 * round > 32 * 1024 ? 2 * round : 32 * 1024;
         if (rest < least) continue;
-        d.slab_budget = static_cast<uint32_t>(rest < most ? rest : most) & ~127u;
-        rest -= d.slab_budget;
+        d.part_budget = static_cast<uint32_t>(rest < most ? rest : most) & ~127u;
+        rest -= d.part_budget;
         d.n_slots = 2 + static_cast<int>(rest / slot);
         if (d.n_slots > MAX_SLOTS) d.n_slots = MAX_SLOTS;
         return true;
@@ -554,26 +607,8 @@ bool plan_dense(uint32_t type, int M, int K, long long rows, DensePlan& d) {
     return false;
 }
 
-// Rows of a panel that has at most `room` row groups wherever it begins. Rows [a, a + r) that meet b matrices make at most
-// b + (r - b) / 16 groups (every matrix adds one, and one more per 16 further rows), and the fewest rows that meet b matrices are
-// the ones between the first and the last, and two. Little room and many matrices come here (eight matrices, 24 rows, Q4_K, K =
-// 14336: room for eight groups, panels of 112 rows if no matrix has fewer).
-int panel_rows_for(const I8Params& p, int room) {
-    auto most_matrices = [&](int r) {
-        int most = 1;
-        for (int i = 0; i < p.n_mats; ++i)
-            for (int j = i + 1; j < p.n_mats; ++j)
-                if (p.mat_end[j - 1] - p.mat_end[i] + 2 <= r && j - i + 1 > most) most = j - i + 1;
-        return most;
-    };
-    auto fits = [&](int r) { const int b = most_matrices(r); return b + (r - b) / 16 <= room; };
-    int r = 16 * room;
-    while (r > 1 && !fits(r)) r = r > 16 ? (r - 1) / 16 * 16 : r - 1;
-    return fits(r) ? r : 0;
-}
-
 template <uint32_t TYPE, int NT, int C, bool QUANT, bool MOE>
-int launch_as(const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes, size_t smem, cudaStream_t st) {
+int launch_as(const I8Maps& maps, I8Params& p, int work_items, size_t part_bytes, size_t smem, cudaStream_t st) {
     auto k = gemm_i8_kernel<TYPE, NT, C, QUANT, MOE>;
     static int max_clusters = 0;
     cudaLaunchConfig_t cfg{};
@@ -584,7 +619,7 @@ int launch_as(const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes
     attr[1].val.clusterDim.x = C; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = C > 1 ? 2 : 1;
-    cfg.blockDim = dim3(THREADS);
+    cfg.blockDim = dim3(THREADS + (C > 1 ? 32 * RW : 0));
     cfg.stream = st;
     if (!max_clusters) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(ctx().smem_optin));
@@ -606,20 +641,11 @@ int launch_as(const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes
         max_clusters = n;
     }
     const int clusters = work_items < max_clusters ? work_items : max_clusters;
-    if constexpr (!MOE) {
-        // panels of as many row groups as the partial results have room for (a panel that begins inside a matrix, or holds the
-        // ends of several, has up to n_mats groups more than rows / 16)
-        p.panel_rows = p.total_rows;
-        p.slab_groups = 0;
-        if (C > 1) {
-            const int rows = (p.total_rows + clusters - 1) / clusters, room = static_cast<int>(slab_bytes / (p.kw * 8 * NT * 16 * 4)) / C * C;
-            const int round = CW / p.kw;
-            if ((rows + 15) / 16 + p.n_mats <= room) p.panel_rows = rows;
-            else if (room - p.n_mats >= round) p.panel_rows = 16 * ((room - p.n_mats) / round * round);
-            else p.panel_rows = panel_rows_for(p, room);
-            if (p.panel_rows < 1) return fail(LAPLACE_ERR_STATE, "gemm_i8: internal planning error (no room for partial results)");
-            p.slab_groups = room / C;
-        }
+    if constexpr (C > 1) {
+        p.n_parts = static_cast<int>(part_bytes / (C * p.kw * NT * PART_BYTES));
+        if (p.n_parts > MAX_PARTS) p.n_parts = MAX_PARTS;
+        if (p.n_parts > 1) p.n_parts = p.n_parts / RW * RW;
+        if (p.n_parts < 1) return fail(LAPLACE_ERR_STATE, "gemm_i8: internal planning error (no room for partial results)");
     }
     cfg.gridDim = dim3(clusters * C);
     cfg.dynamicSmemBytes = smem;
@@ -630,21 +656,21 @@ int launch_as(const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes
 }
 
 template <uint32_t TYPE, int NT, bool QUANT>
-int launch_c(int c, const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes, size_t smem, cudaStream_t st) {
+int launch_c(int c, const I8Maps& maps, I8Params& p, int work_items, size_t part_bytes, size_t smem, cudaStream_t st) {
     switch (c) {
-        case 1: return launch_as<TYPE, NT, 1, QUANT, false>(maps, p, work_items, slab_bytes, smem, st);
-        case 2: return launch_as<TYPE, NT, 2, QUANT, false>(maps, p, work_items, slab_bytes, smem, st);
-        case 4: return launch_as<TYPE, NT, 4, QUANT, false>(maps, p, work_items, slab_bytes, smem, st);
-        default: return launch_as<TYPE, NT, 8, QUANT, false>(maps, p, work_items, slab_bytes, smem, st);
+        case 1: return launch_as<TYPE, NT, 1, QUANT, false>(maps, p, work_items, part_bytes, smem, st);
+        case 2: return launch_as<TYPE, NT, 2, QUANT, false>(maps, p, work_items, part_bytes, smem, st);
+        case 4: return launch_as<TYPE, NT, 4, QUANT, false>(maps, p, work_items, part_bytes, smem, st);
+        default: return launch_as<TYPE, NT, 8, QUANT, false>(maps, p, work_items, part_bytes, smem, st);
     }
 }
 template <uint32_t TYPE>
-int launch_nt(int nt, bool quant, int c, const I8Maps& maps, I8Params& p, int work_items, size_t slab_bytes, size_t smem, cudaStream_t st) {
-    if (quant) return launch_c<TYPE, 1, true>(c, maps, p, work_items, slab_bytes, smem, st);
+int launch_nt(int nt, bool quant, int c, const I8Maps& maps, I8Params& p, int work_items, size_t part_bytes, size_t smem, cudaStream_t st) {
+    if (quant) return launch_c<TYPE, 1, true>(c, maps, p, work_items, part_bytes, smem, st);
     switch (nt) {
-        case 2: return launch_c<TYPE, 2, false>(c, maps, p, work_items, slab_bytes, smem, st);
-        case 3: return launch_c<TYPE, 3, false>(c, maps, p, work_items, slab_bytes, smem, st);
-        default: return launch_c<TYPE, 4, false>(c, maps, p, work_items, slab_bytes, smem, st);
+        case 2: return launch_c<TYPE, 2, false>(c, maps, p, work_items, part_bytes, smem, st);
+        case 3: return launch_c<TYPE, 3, false>(c, maps, p, work_items, part_bytes, smem, st);
+        default: return launch_c<TYPE, 4, false>(c, maps, p, work_items, part_bytes, smem, st);
     }
 }
 
@@ -662,7 +688,7 @@ bool plan_jobs(const TypeGeo& g, int K, int nt, I8Params& p, size_t& smem) {
     const uint32_t buf = (static_cast<uint32_t>(nt * (K / 256) * g.act_bytes) + 127u) & ~127u;
     for (p.act_bufs = 2; p.act_bufs >= 1; --p.act_bufs) {
         p.act_buf_bytes = buf;
-        p.off_slab = p.off_ring = OFF_ACT + p.act_bufs * buf;
+        p.off_part = p.off_ring = OFF_ACT + p.act_bufs * buf;
         const long long ring = static_cast<long long>(ctx().smem_optin) - p.off_ring - 16;
         p.n_slots = static_cast<int>(ring / (static_cast<long long>(CW) * 16 * g.pitch));
         if (p.n_slots > MAX_SLOTS) p.n_slots = MAX_SLOTS;
@@ -745,8 +771,8 @@ int launch_gemm_i8(const float* x, const float* norm_w, float eps, float* x_norm
     for (int i = n_mats; i < MAX_MATS; ++i) maps.w[i] = maps.w[0];
     p.x = x; p.norm_w = norm_w; p.norm_eps = eps; p.x_norm_out = x_norm_out; p.err = c.d_err;
     p.M = M; p.K = K; p.nsb = K / 256; p.n_mats = n_mats; p.total_rows = static_cast<int>(total); p.kw = d.kw;
-    p.off_slab = OFF_ACT + d.act;
-    p.off_ring = (p.off_slab + d.slab_budget + 127u) & ~127u;
+    p.off_part = OFF_ACT + d.act;
+    p.off_ring = (p.off_part + d.part_budget + 127u) & ~127u;
     p.n_slots = d.n_slots;
     const size_t smem = p.off_ring + static_cast<size_t>(CW) * d.n_slots * 16 * g.pitch + 16;      // + read-ahead of the unaligned loads
     const bool quant = M <= 8;
@@ -760,10 +786,10 @@ int launch_gemm_i8(const float* x, const float* norm_w, float eps, float* x_norm
     }
     const int items = static_cast<int>((total + 15) / 16);
     switch (type) {
-        case LAPLACE_TYPE_Q4_K: rc = launch_nt<LAPLACE_TYPE_Q4_K>(d.nt, quant, d.c, maps, p, items, d.slab_budget, smem, st); break;
-        case LAPLACE_TYPE_Q8_0: rc = launch_nt<LAPLACE_TYPE_Q8_0>(d.nt, quant, d.c, maps, p, items, d.slab_budget, smem, st); break;
-        case LAPLACE_TYPE_Q4_0: rc = launch_nt<LAPLACE_TYPE_Q4_0>(d.nt, quant, d.c, maps, p, items, d.slab_budget, smem, st); break;
-        default: rc = launch_nt<LAPLACE_TYPE_Q6_K>(d.nt, quant, d.c, maps, p, items, d.slab_budget, smem, st); break;
+        case LAPLACE_TYPE_Q4_K: rc = launch_nt<LAPLACE_TYPE_Q4_K>(d.nt, quant, d.c, maps, p, items, d.part_budget, smem, st); break;
+        case LAPLACE_TYPE_Q8_0: rc = launch_nt<LAPLACE_TYPE_Q8_0>(d.nt, quant, d.c, maps, p, items, d.part_budget, smem, st); break;
+        case LAPLACE_TYPE_Q4_0: rc = launch_nt<LAPLACE_TYPE_Q4_0>(d.nt, quant, d.c, maps, p, items, d.part_budget, smem, st); break;
+        default: rc = launch_nt<LAPLACE_TYPE_Q6_K>(d.nt, quant, d.c, maps, p, items, d.part_budget, smem, st); break;
     }
     c.last_path = M <= 8 ? 1 : 2;
     return rc;
