@@ -1,6 +1,7 @@
 // lp_gemm_sa.cu - prefill GEMM and expert-grouped matmul: tiles on the 5th-generation tensor cores in a "scaled activation"
-// formulation (this comment, Q4_K; namespace w2 for the two-piece types) or on the warp-level int8 instruction (namespace i8t);
-// which call takes which is said at i8_tiles. Up to 32 activation rows, and experts with few tokens, run in lp_gemm_i8.cu. Replaces gemm_int<dot_row_q4_k_int_neon> of
+// formulation (this comment, Q4_K; namespace w2 for the two-piece types), and the choice of kernel for calls with more than 8 rows.
+// Up to 32 activation rows, and experts with few tokens, run in lp_gemm_i8.cu, the tiles on the warp-level int8 instruction in
+// lp_gemm_i8_tiles.cu (see i8_tiles), Q4_K and Q6_K above 128 rows in lp_gemm_pair.cu. Replaces gemm_int<dot_row_q4_k_int_neon> of
 // Laplace's NEON back-end (src/matmul_simd.cpp:226-283, 432-455) for large M.
 //
 // The reference's result for one (token m, weight row n) is
@@ -1364,8 +1365,8 @@ int launch_gemm_sa_peers(const float* x, const uint8_t* w, uint32_t type, const 
 }
 
 // laplace_cuda_gemm_dev for more than 8 rows on scratch memory the caller owns (`cap` bytes at `scratch`, 256-byte aligned);
-// nothing is allocated. The same kernel runs as there, and the balanced split of launch_gemm_sa is kept when its partial
-// results fit too (the result is then bit-identical to that call's), otherwise the call runs on whole tiles.
+// nothing is allocated. The same kernel runs as there when its operand fits (a call close to the limit may not fit the pair kernel's),
+// and cut tiles are kept when their partial results fit too (the result is then bit-identical to that call's).
 int launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const uint8_t* w, uint32_t type, float* y,
                             int M, int K, int N, cudaStream_t st) {
     int rc = check_args(x, w, type, M, K, N);
@@ -1382,7 +1383,7 @@ int launch_gemm_sa_prealloc(uint8_t* scratch, size_t cap, const float* x, const 
     }
     if (gemm_pair_supports(type, M)) {
         const bool cut = gemm_pair_scratch(type, M, K, &N, 1, true) <= cap;
-        if (gemm_pair_scratch(type, M, K, &N, 1, cut) <= cap)       // always: its operand is smaller than the one above
+        if (gemm_pair_scratch(type, M, K, &N, 1, cut) <= cap)       // its operand is 4.5 bytes a value: close to the limit the kernels below run
             return launch_gemm_pair(scratch, cut, x, nullptr, 0.f, nullptr, &w, &y, &N, 1, type, M, K, st, nullptr);
     }
     return gemm_sa_on_scratch(scratch, pl, x, w, type, y, M, K, N, st);

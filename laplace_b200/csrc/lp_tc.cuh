@@ -41,16 +41,6 @@ __device__ __forceinline__ void ld32(uint32_t taddr, float (&v)[32]) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
-// 32 lanes x 16 consecutive columns
-__device__ __forceinline__ void ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr));
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
 // 16 lanes x 16 consecutive 32-bit columns in the 16x256b shape -> 8 registers per thread: register 4 g + 2 q + e of
 // lane l holds TMEM lane (base + 8 q + l / 4), column 8 g + 2 (l % 4) + e (the layout of an m16n8 accumulator
 // fragment, once per 8 columns).
@@ -157,10 +147,6 @@ __device__ __forceinline__ bool wait_pair(uint32_t bar, uint32_t parity, volatil
     *abort_flag = 1;
     report_status(err, code);
     return false;
-}
-__device__ __forceinline__ void st_global_v8(float* p, const float (&v)[8]) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 :: "l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
 }
 
 #endif  // __CUDACC__
