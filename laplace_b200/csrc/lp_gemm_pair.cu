@@ -9,12 +9,13 @@
 // cycles of the tensor core. Measured (us, calls with quantizer and all, one-CTA kernels -> here): Q4_K 4096 x 14336, 512 tokens 180 -> 108,
 // 2048 tokens 703 -> 364; 4096 x 4096, 512 tokens 59.8 -> 48.9; Q6_K 14336 x 4096, 512 tokens 316 -> 144, 2048 tokens 1199 -> 521. At 2048
 // tokens the card's power limit holds the clock at 1.3 to 1.5 GHz: Q4_K takes 5250 cycles per super-block and tile for the MMAs' 4480.
-// hi and lo meet in one accumulator. Sums in it are truncated, not rounded, at every MMA step, so it is drained after every two or four
-// stages (figures at UNIT), and what goes in is small:
+// hi and lo meet in one accumulator. Sums in it are truncated, not rounded, at every MMA step, so it is drained after every two stages
+// (figures at UNIT), and what goes in is small:
 //   Q4_K   weight operand sc * (nibble - 8), exact in fp16. What is then missing is a contraction over the super-block's eight blocks and
 //          goes through the same accumulator as three more steps in bf16: (8 sc_j - dmin / d * mn_j) and the sums 2^e d_x sum(q), three
-//          pieces each, the products p1 g1 + p2 g1 + p1 g2 + p2 g2 + p3 g1 + p1 g3 of them. (With plain nibbles the two parts, each several
-//          times the result, would leave 1.5e-6 of error for 6e-7.)
+//          pieces each, the products p1 g1 + p2 g1 + p1 g2 + p2 g2 + p3 g1 + p1 g3 of them. They come last, the smallest first: where a
+//          block is not centred at 8 they are several times the result, and every step after them is truncated against them (first: random
+//          blocks 9.7e-7, min / max packed ones 6.2e-7; last: 3.6 and 6.8e-7, before the accumulator was drained twice a super-block).
 //   Q6_K   sc * (q6 - 32) reaches 4096, one bit more than fp16 holds: the rounded value and the rest (-1, 0 or 1); the rest meets hi only
 //          (times lo it is below 2^-22 of the largest product).
 //
@@ -49,11 +50,13 @@ constexpr int SA_TILE = 128 * 32 * 2;        // 8 KB: 128 weight rows' min piece
 constexpr int SLOT = TOK * ROWS;             // floats of a partial tile: [token][weight row]
 
 // PITCH: bytes between the packed rows in shared memory. Q6_K rows are copied from the 16-byte boundary below.
-// UNIT: stages that an accumulator takes in. Relative error against 64 bits on 512 x 4096 x 14336 (Q4_K) and 512 x 14336 x 4096 (Q6_K),
-// the one-CTA kernels 7.2e-7 and 4.5e-7: four stages 6.1e-7 and 7.7e-7, two 3.5e-7 and 4.2e-7, one 2.5e-7 and 2.9e-7. Time at 2048 tokens,
-// Q4_K: four 364, two 381, one 438 us.
+// UNIT: stages that an accumulator takes in: as many as leave no more error than the one-CTA kernels do, for any weights. Relative error
+// against 64 bits, 256 x 4096 x 512, N(0, 1) activations, random blocks / min-max packed / absmax packed weights:
+//   Q4_K   one-CTA kernel 3.0 / 6.6 / 2.8e-7; four stages 3.6 / 6.8 / 3.6, two 2.1 / 3.8 / 2.1, one 1.5 / 2.4 / 1.5
+//   Q6_K   one-CTA kernel 2.0 / 4.4 / 3.2e-7; two stages 2.8 / 4.2 / 3.3
+// Time at 2048 tokens, Q4_K 4096 x 14336: four 356, two 367, one 420 us.
 template <uint32_t TYPE> struct Geo;
-template <> struct Geo<LAPLACE_TYPE_Q4_K> { static constexpr int SB = Q4_K_BYTES, PITCH = Q4_K_BYTES, STAGES = 3, PIECES = 1, UNIT = 4; static constexpr bool MINS = true; };
+template <> struct Geo<LAPLACE_TYPE_Q4_K> { static constexpr int SB = Q4_K_BYTES, PITCH = Q4_K_BYTES, STAGES = 3, PIECES = 1, UNIT = 2; static constexpr bool MINS = true; };
 template <> struct Geo<LAPLACE_TYPE_Q6_K> { static constexpr int SB = Q6_K_BYTES, PITCH = 240, STAGES = 2, PIECES = 2, UNIT = 2; static constexpr bool MINS = false; };
 
 template <uint32_t TYPE> struct Lay {
@@ -285,16 +288,16 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ 
             for (int i = 0; ok && segment(p, i, sg); ++i) {
                 const int bk = box_bucket(sg.nt), box = 16 << bk, row = sg.m0 + static_cast<int>(rank) * box;
                 for (int sb = sg.sb0; sb < sg.sb1 && ok; ++sb, ++sbc) {
-                    if (G::MINS && pc == 1) {
-                        if (!wait_or_abort<false>(sbase + L::EMPTY_S, (sbc & 1) ^ 1, abort_flag, p.err, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-                        if (rank == 0) mbar_expect_tx(sbase + L::FULL_S, 2 * box * 128);
-                        tma_load_2d_pair(sbase + L::SB, &maps.s[bk], sb * 64, row, leader(L::FULL_S));
-                    }
                     for (int c = 0; c < 4; ++c, ++it) {
                         const int s = it % STAGES;
                         if (!wait_or_abort<false>(sbase + L::EMPTY + 8 * s, ((it / STAGES) & 1) ^ 1, abort_flag, p.err, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
                         if (rank == 0) mbar_expect_tx(sbase + L::FULL + 8 * s, 2 * box * 128);
                         tma_load_2d_pair(sbase + L::A + (2 * s + pc) * TILE, &maps.a[bk], sb * 256 + c * BKC, pc * p.m_pad + row, leader(L::FULL + 8 * s));
+                        if (G::MINS && pc == 1 && c == 2) {
+                            if (!wait_or_abort<false>(sbase + L::EMPTY_S, (sbc & 1) ^ 1, abort_flag, p.err, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+                            if (rank == 0) mbar_expect_tx(sbase + L::FULL_S, 2 * box * 128);
+                            tma_load_2d_pair(sbase + L::SB, &maps.s[bk], sb * 64, row, leader(L::FULL_S));
+                        }
                     }
                 }
             }
@@ -320,20 +323,10 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ 
                     for (int c = 0; c < 4; ++c, ++it) {
                         const int s = it % STAGES;
                         const uint32_t acc = tmem_base + (u & 1) * TOK;
-                        uint32_t more = c % UNIT != 0;
+                        const uint32_t more = c % UNIT != 0;
                         if (!more) {
                             if (!wait_pair(sbase + L::TMEM_EMPTY + 8 * (u & 1), ((u >> 1) & 1) ^ 1, abort_flag, p.err, DEV_TIMEOUT_TMEM)) { ok = false; break; }
                             fence_after();
-                        }
-                        if (G::MINS && c == 0) {
-                            if (!wait_pair(sbase + L::FULL_S, sbc & 1, abort_flag, p.err, DEV_TIMEOUT_FULL)) { ok = false; break; }
-                            fence_after();
-                            const uint64_t a = smem_desc_sw64(sbase + L::SA), b = smem_desc_sw128(sbase + L::SB);
-                            mma_f16_pair(acc, a, b, idesc_bf16, 0);
-                            mma_f16_pair(acc, a, b + 2, idesc_bf16, 1);
-                            mma_f16_pair(acc, a + 2, b + 4, idesc_bf16, 1);
-                            commit_pair(sbase + L::EMPTY_S);
-                            more = 1;
                         }
                         if (!wait_pair(sbase + L::FULL + 8 * s, (it / STAGES) & 1, abort_flag, p.err, DEV_TIMEOUT_FULL)) { ok = false; break; }
                         fence_after();
@@ -345,6 +338,15 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ 
                             if (G::PIECES == 2) mma_f16_pair(acc, w + (TILE >> 4) + 2 * ks, x + 2 * ks, idesc, 1);
                         }
                         commit_pair(sbase + L::EMPTY + 8 * s);
+                        if (G::MINS && c == 3) {                                       // the smallest products first
+                            if (!wait_pair(sbase + L::FULL_S, sbc & 1, abort_flag, p.err, DEV_TIMEOUT_FULL)) { ok = false; break; }
+                            fence_after();
+                            const uint64_t a = smem_desc_sw64(sbase + L::SA), b = smem_desc_sw128(sbase + L::SB);
+                            mma_f16_pair(acc, a + 2, b + 4, idesc_bf16, 1);
+                            mma_f16_pair(acc, a, b + 2, idesc_bf16, 1);
+                            mma_f16_pair(acc, a, b, idesc_bf16, 1);
+                            commit_pair(sbase + L::EMPTY_S);
+                        }
                         if (c % UNIT == UNIT - 1) { commit_pair(sbase + L::TMEM_FULL + 8 * (u & 1)); ++u; }
                     }
                 }
@@ -435,28 +437,30 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ 
                         d = half_bits_to_float(hdr.x);
                     }
                     table(d);
-                    // what a block's sum is multiplied with: 8 sc_j (the nibbles' offset) - dmin / d * mn_j, as three bf16 pieces that add up
-                    // to it, in the order p1 p2 p3 p1
-                    const float cm = __fdiv_rn(-half_bits_to_float(hdr.x >> 16), d);
-                    uint32_t p1[4], p2[4], p3[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const uint32_t mn = j < 2 ? hdr.z & 0x3f3f3f3fu : ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u), sc = j < 2 ? sc_lo : sc_hi;
-                        const int at = 16 * (j & 1);
-                        split3(make_float2(fmaf(cm, static_cast<float>((mn >> at) & 0xffu), 8.0f * static_cast<float>((sc >> at) & 0xffu)),
-                                           fmaf(cm, static_cast<float>((mn >> (at + 8)) & 0xffu), 8.0f * static_cast<float>((sc >> (at + 8)) & 0xffu))), p1[j], p2[j], p3[j]);
-                    }
-                    if (!wait_or_abort<false>(sbase + L::EMPTY_S, (sbc & 1) ^ 1, abort_flag, p.err, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-                    const uint32_t srow = sbase + L::SA + r * 64;
-                    const int r3 = (r >> 1) & 3;
-                    sts128(srow + ((0 ^ r3) << 4), p1[0], p1[1], p1[2], p1[3]);
-                    sts128(srow + ((1 ^ r3) << 4), p2[0], p2[1], p2[2], p2[3]);
-                    sts128(srow + ((2 ^ r3) << 4), p3[0], p3[1], p3[2], p3[3]);
-                    sts128(srow + ((3 ^ r3) << 4), p1[0], p1[1], p1[2], p1[3]);
-                    publish(L::FULL_S);
 #pragma unroll 1
                     for (int c = 0; c < 4; ++c, ++it) {
                         const int s = it % STAGES;
+                        if (c == 3) {
+                            // what a block's sum is multiplied with: 8 sc_j (the nibbles' offset) - dmin / d * mn_j, as three bf16 pieces that add up
+                            // to it, in the order p1 p2 p3 p1
+                            const float cm = __fdiv_rn(-half_bits_to_float(hdr.x >> 16), d);
+                            uint32_t p1[4], p2[4], p3[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const uint32_t mn = j < 2 ? hdr.z & 0x3f3f3f3fu : ((hdr.w >> 4) & 0x0f0f0f0fu) | ((hdr.z >> 2) & 0x30303030u), sc = j < 2 ? sc_lo : sc_hi;
+                                const int at = 16 * (j & 1);
+                                split3(make_float2(fmaf(cm, static_cast<float>((mn >> at) & 0xffu), 8.0f * static_cast<float>((sc >> at) & 0xffu)),
+                                                   fmaf(cm, static_cast<float>((mn >> (at + 8)) & 0xffu), 8.0f * static_cast<float>((sc >> (at + 8)) & 0xffu))), p1[j], p2[j], p3[j]);
+                            }
+                            if (!wait_or_abort<false>(sbase + L::EMPTY_S, (sbc & 1) ^ 1, abort_flag, p.err, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
+                            const uint32_t srow = sbase + L::SA + r * 64;
+                            const int r3 = (r >> 1) & 3;
+                            sts128(srow + ((0 ^ r3) << 4), p1[0], p1[1], p1[2], p1[3]);
+                            sts128(srow + ((1 ^ r3) << 4), p2[0], p2[1], p2[2], p2[3]);
+                            sts128(srow + ((2 ^ r3) << 4), p3[0], p3[1], p3[2], p3[3]);
+                            sts128(srow + ((3 ^ r3) << 4), p1[0], p1[1], p1[2], p1[3]);
+                            publish(L::FULL_S);
+                        }
                         if (!begin(s)) { ok = false; break; }
                         convert_q4k(raw, c, sc_lo, sc_hi, sbase + L::W + s * TILE + r * 128, r7);
                         publish(L::FULL + 8 * s);

@@ -45,6 +45,27 @@ def test_matrices_of_one_call_have_the_bits_of_single_calls(oracle, t, M, K, Ns)
         assert np.array_equal(single, y)
 
 
+@pytest.mark.parametrize("t", [Q4_K])
+@pytest.mark.parametrize("pack", ["random", "affine", "ref"])
+@pytest.mark.parametrize("rows", ["normal", "outliers", "positive"])
+def test_pairs_are_no_further_from_64_bits_than_single_ctas(oracle, t, pack, rows):
+    """256 rows in one call, on pairs of SMs, against two calls of 128 rows, which run on the one-CTA kernels: other sums of the same
+    products, no larger error. 256 x 384 independent errors put 1 / sqrt(2 x 98304) = 0.23 % of spread on either norm; 2 % between the two
+    is six times that of their quotient."""
+    M, K, N = 256, 4096, 384
+    w = synth.random_blocks(t, K, N, seed=740) if pack == "random" else synth.weights(t, K, N, seed=740, how=pack)
+    x = synth.normal_f32(741, (M, K))
+    if rows == "outliers":
+        x[:, ::97] *= np.float32(50.0)
+    elif rows == "positive":
+        x = np.abs(x)
+    ref = oracle.gemm(x, w, t, M, K, N, mode=1, threads=THREADS).astype(np.float64)
+    (y,) = _run(t, x, [w], M, K, [N])
+    one = np.concatenate([_run(t, x[m:m + 128], [w], 128, K, [N])[0] for m in (0, 128)])
+    err, err_one = (np.linalg.norm(v - ref) for v in (y, one))
+    assert err <= 1.02 * err_one, f"{err / np.linalg.norm(ref):.3e} against {err_one / np.linalg.norm(ref):.3e}"
+
+
 @pytest.mark.parametrize("t", [Q4_K, Q6_K])
 def test_zero_super_blocks_and_rows(oracle, t):
     """A super-block with d = 0 (Q4_K: dmin stays) and activation rows of zeros, beside ordinary ones."""
