@@ -9,15 +9,15 @@
 // cycles of the tensor core. Measured (us, calls with quantizer and all, one-CTA kernels -> here): Q4_K 4096 x 14336, 512 tokens 180 -> 108,
 // 2048 tokens 703 -> 364; 4096 x 4096, 512 tokens 59.8 -> 48.9; Q6_K 14336 x 4096, 512 tokens 316 -> 144, 2048 tokens 1199 -> 521. At 2048
 // tokens the card's power limit holds the clock at 1.3 to 1.5 GHz: Q4_K takes 5250 cycles per super-block and tile for the MMAs' 4480.
-// hi and lo meet in one accumulator. Sums in it are truncated, not rounded, at every MMA step, so it is drained after every two stages
-// (figures at UNIT), and what goes in is small:
+// hi and lo meet in one accumulator. Sums in it are truncated, not rounded, at every MMA step, so it is drained after every stage or
+// two (figures at UNIT), lo goes in before hi, and what goes in is small:
 //   Q4_K   weight operand sc * (nibble - 8), exact in fp16. What is then missing is a contraction over the super-block's eight blocks and
 //          goes through the same accumulator as three more steps in bf16: (8 sc_j - dmin / d * mn_j) and the sums 2^e d_x sum(q), three
 //          pieces each, the products p1 g1 + p2 g1 + p1 g2 + p2 g2 + p3 g1 + p1 g3 of them. They come last, the smallest first: where a
 //          block is not centred at 8 they are several times the result, and every step after them is truncated against them (first: random
 //          blocks 9.7e-7, min / max packed ones 6.2e-7; last: 3.6 and 6.8e-7, before the accumulator was drained twice a super-block).
-//   Q6_K   sc * (q6 - 32) reaches 4096, one bit more than fp16 holds: the rounded value and the rest (-1, 0 or 1); the rest meets hi only
-//          (times lo it is below 2^-22 of the largest product).
+//   Q6_K   sc * (q6 - 32) reaches 4096, one bit more than fp16 holds: the rounded value and the rest (-1, 0 or 1). The rest meets hi only
+//          (times lo it is below 2^-22 of the largest product) and goes in first.
 //
 // One 512-thread CTA per SM, persistent; roles by warp:
 //   0, 2   copies: hi / lo piece of the activations (64 k x up to 128 tokens, 128-byte swizzle); warp 2 the sum pieces too
@@ -53,11 +53,11 @@ constexpr int SLOT = TOK * ROWS;             // floats of a partial tile: [token
 // UNIT: stages that an accumulator takes in: as many as leave no more error than the one-CTA kernels do, for any weights. Relative error
 // against 64 bits, 256 x 4096 x 512, N(0, 1) activations, random blocks / min-max packed / absmax packed weights:
 //   Q4_K   one-CTA kernel 3.0 / 6.6 / 2.8e-7; four stages 3.6 / 6.8 / 3.6, two 2.1 / 3.8 / 2.1, one 1.5 / 2.4 / 1.5
-//   Q6_K   one-CTA kernel 2.0 / 4.4 / 3.2e-7; two stages 2.8 / 4.2 / 3.3
-// Time at 2048 tokens, Q4_K 4096 x 14336: four 356, two 367, one 420 us.
+//   Q6_K   one-CTA kernel 2.0 / 4.4 / 3.2e-7; two stages 2.8 / 4.2 / 3.3, one 1.9 / 2.5 / 2.1, one with the rest first 1.7 / 2.0 / 1.8
+// Time at 2048 tokens: Q4_K 4096 x 14336 four 356, two 367, one 420 us; Q6_K 14336 x 4096 two 509, one 526 us.
 template <uint32_t TYPE> struct Geo;
 template <> struct Geo<LAPLACE_TYPE_Q4_K> { static constexpr int SB = Q4_K_BYTES, PITCH = Q4_K_BYTES, STAGES = 3, PIECES = 1, UNIT = 2; static constexpr bool MINS = true; };
-template <> struct Geo<LAPLACE_TYPE_Q6_K> { static constexpr int SB = Q6_K_BYTES, PITCH = 240, STAGES = 2, PIECES = 2, UNIT = 2; static constexpr bool MINS = false; };
+template <> struct Geo<LAPLACE_TYPE_Q6_K> { static constexpr int SB = Q6_K_BYTES, PITCH = 240, STAGES = 2, PIECES = 2, UNIT = 1; static constexpr bool MINS = false; };
 
 template <uint32_t TYPE> struct Lay {
     using G = Geo<TYPE>;
@@ -331,11 +331,15 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ 
                         if (!wait_pair(sbase + L::FULL + 8 * s, (it / STAGES) & 1, abort_flag, p.err, DEV_TIMEOUT_FULL)) { ok = false; break; }
                         fence_after();
                         const uint64_t w = smem_desc_sw128(sbase + L::W + s * G::PIECES * TILE), x = smem_desc_sw128(sbase + L::A + 2 * s * TILE);
+                        // 32 bytes >> 4 inside the swizzle row; the rest of Q6_K's weights, the smallest products, first
+                        if (G::PIECES == 2) {
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {                               // 32 bytes >> 4 inside the swizzle row
-                            mma_f16_pair_fill(acc, w + 2 * ks, x + 2 * ks, idesc, more | ks);
-                            mma_f16_pair_last(acc, w + 2 * ks, x + (TILE >> 4) + 2 * ks, idesc, 1);
-                            if (G::PIECES == 2) mma_f16_pair(acc, w + (TILE >> 4) + 2 * ks, x + 2 * ks, idesc, 1);
+                            for (int ks = 0; ks < 4; ++ks) mma_f16_pair(acc, w + (TILE >> 4) + 2 * ks, x + 2 * ks, idesc, more | ks);
+                        }
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks) {
+                            mma_f16_pair_fill(acc, w + 2 * ks, x + (TILE >> 4) + 2 * ks, idesc, (G::PIECES == 2) | more | ks);
+                            mma_f16_pair_last(acc, w + 2 * ks, x + 2 * ks, idesc, 1);
                         }
                         commit_pair(sbase + L::EMPTY + 8 * s);
                         if (G::MINS && c == 3) {                                       // the smallest products first

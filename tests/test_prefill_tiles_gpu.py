@@ -45,7 +45,7 @@ def test_matrices_of_one_call_have_the_bits_of_single_calls(oracle, t, M, K, Ns)
         assert np.array_equal(single, y)
 
 
-@pytest.mark.parametrize("t", [Q4_K])
+@pytest.mark.parametrize("t", [Q4_K, Q6_K])
 @pytest.mark.parametrize("pack", ["random", "affine", "ref"])
 @pytest.mark.parametrize("rows", ["normal", "outliers", "positive"])
 def test_pairs_are_no_further_from_64_bits_than_single_ctas(oracle, t, pack, rows):
