@@ -38,7 +38,8 @@ struct TileParams {
     int          N[MAX_MATS];
     // How a matrix's tiles (weight rows outside, tokens inside) are shared out, by its own size alone, so that it has the same bits alone and
     // beside others: the first `whole` are dealt round-robin from CTA `shift` on; of those behind, the super-blocks (`units` in tile order)
-    // go evenly to the `cut` CTAs from there on, partial results to slot 2c (continues a tile) or 2c + 1 (begins one) of the matrix's.
+    // go evenly to the `cut` CTAs from there on; the c-th CTA's piece of the t-th cut tile is the matrix's partial result c + t (from one
+    // piece to the next c or t grows, or both).
     int          whole[MAX_MATS], units[MAX_MATS], tiles[MAX_MATS], cut[MAX_MATS], shift[MAX_MATS], slot0[MAX_MATS];
 };
 struct Seg { int mat, m0, n0, nt, sb0, sb1, part; };      // nt: tokens
@@ -68,7 +69,7 @@ __device__ __forceinline__ bool segment(const TileParams& p, int i, Seg& s) {
             if (t <= last) {
                 s.sb0 = t == first ? u0 - first * nsb : 0;
                 s.sb1 = t == last ? u1 - last * nsb : nsb;
-                if (s.sb0 > 0 || s.sb1 < nsb) s.part = p.slot0[s.mat] + 2 * v + (s.sb0 == 0 ? 1 : 0);
+                if (s.sb0 > 0 || s.sb1 < nsb) s.part = p.slot0[s.mat] + v + t;
                 tile_at(p, whole + t, s);
                 return true;
             }
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(256) tile_fixup_kernel(const __grid_constant__
     if (ca == cb || n >= N) return;
     float4 a[2];
     for (int c = ca; c <= cb; ++c) {
-        const float* src = p.part + static_cast<size_t>(p.slot0[sg.mat] + 2 * c + (c == ca ? 1 : 0)) * (TT * TW) + r;      // ca's piece begins the tile
+        const float* src = p.part + static_cast<size_t>(p.slot0[sg.mat] + c + t) * (TT * TW) + r;
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const int tok = tok0 + 8 * j;
@@ -269,7 +270,7 @@ TilePlan plan_tiles(uint32_t type, int M, int K, const int* ns, int n_mats, bool
                 pl.whole[i] = tiles - rest;
                 pl.units[i] = units;
                 pl.cut[i] = used = cut;
-                slots += 2 * cut;
+                slots += cut + rest - 1;
                 pl.cut_tiles += rest;
             }
         }

@@ -86,8 +86,8 @@ struct PairParams {
     int          N[MAX_MATS];
     // How a matrix's tiles (weight rows outside, tokens inside) are shared out, by its own size alone, so that it has the same bits alone and
     // beside others. The first `whole` are dealt round-robin from pair `shift` on; those behind are cut: their super-blocks, `units` in tile
-    // order, go evenly to the `cut` pairs from there on (the c-th: [c * units / cut, (c + 1) * units / cut)), partial results to slot 2c
-    // (continues a tile) or 2c + 1 (begins one) of the matrix's.
+    // order, go evenly to the `cut` pairs from there on (the c-th: [c * units / cut, (c + 1) * units / cut)). The c-th pair's piece
+    // of the t-th cut tile is the matrix's partial result c + t: from one piece to the next c or t grows, or both.
     int          tiles[MAX_MATS], whole[MAX_MATS], units[MAX_MATS], cut[MAX_MATS], shift[MAX_MATS], slot0[MAX_MATS];
     float*       part;
 };
@@ -127,7 +127,7 @@ __device__ __forceinline__ bool segment(const PairParams& p, int i, Seg& s) {
             if (t <= last) {
                 s.sb0 = t == first ? u0 - first * nsb : 0;
                 s.sb1 = t == last ? u1 - last * nsb : nsb;
-                s.part = s.sb0 > 0 || s.sb1 < nsb ? p.slot0[s.mat] + 2 * vp + (s.sb0 == 0 ? 1 : 0) : -1;
+                s.part = s.sb0 > 0 || s.sb1 < nsb ? p.slot0[s.mat] + vp + t : -1;
                 tile_at(p, whole + t, s);
                 return true;
             }
@@ -723,8 +723,7 @@ __global__ void __launch_bounds__(256) pair_fixup_kernel(const __grid_constant__
     if (ca == cb || n >= N) return;
     float4 a[4];
     for (int c = ca; c <= cb; ++c) {
-        const int slot = p.slot0[sg.mat] + 2 * c + (c == ca ? 1 : 0);           // ca holds the tile's first unit: its piece begins the tile
-        const float* src = p.part + static_cast<size_t>(slot) * SLOT + col;
+        const float* src = p.part + static_cast<size_t>(p.slot0[sg.mat] + c + t) * SLOT + col;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int tok = tok0 + 4 * j;
@@ -785,7 +784,7 @@ PairPlan plan_pair(uint32_t type, int M, int K, const int* ns, int n_mats, int m
                 pl.units[i] = units;
                 pl.cut[i] = used = cut;
                 pl.cut_tiles += rest;
-                slots += 2 * cut;
+                slots += cut + rest - 1;
             }
         }
         const int need = tiles >= max_pairs ? max_pairs : used;

@@ -2,6 +2,8 @@
 (above 32 rows), at the edges of a tile of weight rows, of activation rows and of K, with rows that no tensor map can address, with
 super-blocks and activation rows of zeros, and where partial results have no room. Oracle and bar as in the other GPU tests."""
 import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -80,6 +82,33 @@ def test_zero_super_blocks_and_rows(oracle, t):
     (y,) = _run(t, x, [w], M, K, [N])
     check_close(y, oracle.gemm(x, w, t, M, K, N, mode=1, threads=THREADS), f"zero blocks {t.name}")
     assert not y[5].any()
+
+
+def test_scratch_of_a_call_with_several_matrices():
+    """q / k / v of 512 rows: the operand, and partial results of at most pairs + tiles - 1 pieces a matrix (and the eighth that scratch
+    grows by beyond what is asked for). In a process of its own, whose scratch is empty; a first small call loads the kernels."""
+    code = """
+import torch
+from laplace_b200 import device
+from laplace_b200.ggml import GGMLType
+K, Ns = 4096, [4096, 1024, 1024]
+ws = [torch.zeros(n * K // 256 * 144, dtype=torch.uint8, device="cuda") for n in Ns]
+x, ys = torch.ones(512, K, device="cuda"), None
+device.gemm(x[:130, :2048].contiguous(), ws[2], GGMLType.Q4_K, 130, 2048, 256)
+keep = [torch.empty(512, n, device="cuda") for n in Ns]
+del keep
+torch.cuda.synchronize()
+before = torch.cuda.mem_get_info()[0]
+device.gemm_multi(x, ws, GGMLType.Q4_K, 512, K, Ns)
+device.sync()
+print(before - torch.cuda.mem_get_info()[0], torch.cuda.get_device_properties(0).multi_processor_count // 2)
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr
+    grown, pairs = map(int, r.stdout.split())
+    operand = 512 * 4096 * 4.5 + 512 * 4
+    tiles = [2 * 16, 2 * 4, 2 * 4]
+    assert grown <= 9 / 8 * (operand + sum(pairs + t - 1 for t in tiles) * 256 * 256 * 4) + (4 << 20), f"{grown / 2 ** 20:.1f} MiB"
 
 
 @pytest.mark.parametrize("t,off", [(Q6_K, 2), (Q6_K, 8)])
