@@ -215,15 +215,21 @@ __global__ void __launch_bounds__(256) tile_fixup_kernel(const __grid_constant__
     asm volatile("griddepcontrol.wait;" ::: "memory");        // the pieces are there
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (ca == cb || n >= N) return;
+    // four pieces' loads in flight
     float4 a[2];
-    for (int c = ca; c <= cb; ++c) {
-        const float* src = p.part + static_cast<size_t>(p.slot0[sg.mat] + c + t) * (TT * TW) + r;
+    const float* src = p.part + static_cast<size_t>(p.slot0[sg.mat] + ca + t) * (TT * TW) + tok0 * TW + r;
+    for (int left = cb - ca + 1; left > 0; left -= 4, src += 4 * TT * TW) {
+        float4 v[4][2];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int tok = tok0 + 8 * j;
-            const float4 v = tok < sg.nt ? __ldg(reinterpret_cast<const float4*>(src + tok * TW)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            a[j] = c == ca ? v : make_float4(a[j].x + v.x, a[j].y + v.y, a[j].z + v.z, a[j].w + v.w);
-        }
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (q < left && tok0 + 8 * j < sg.nt) v[q][j] = __ldg(reinterpret_cast<const float4*>(src + q * TT * TW + 8 * j * TW));
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (q < left) a[j] = q == 0 && left == cb - ca + 1 ? v[q][j] : make_float4(a[j].x + v[q][j].x, a[j].y + v[q][j].y, a[j].z + v[q][j].z, a[j].w + v[q][j].w);
     }
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -246,7 +252,13 @@ __global__ void __launch_bounds__(256) tile_fixup_kernel(const __grid_constant__
 inline size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
 // How the tiles are shared out: as many rounds of whole tiles as every CTA gets, the rest cut evenly; a CTA takes no less than two
-// super-blocks of cut tiles.
+// super-blocks of cut tiles. Up to four super-blocks a CTA the pieces are as few as its work allows (Q8_0, 120 rows 1536 x 8960: 148 pieces of
+// three at most 26.1, 140 of three 21.7 us; 77 rows 14336 x 1024: 25.5 and 24.0; but Q6_K, 96 rows 4096 x 14336: 148 of thirteen at most 90.6,
+// 138 of thirteen 102). Tiles are cut if that gives each two CTAs or shortens the longest CTA's work by three super-blocks: pieces of many
+// tiles cost more than two are worth (512 rows 4096 x 4096 Q8_0, 128 tiles: cut 57.3, whole 54.9 us; 200 rows 2816 x 8448 44.2 and 40.8; 128
+// rows 4096 x 14336, a gain of three: 53.8 and 54.9). Where the last tokens' tiles are much smaller, whole tiles leave the CTAs unequal work,
+// and all are cut: a super-block costs some 62 + its tokens (Q8_0 4096 x 14336: 33 rows 31 us, 64 39, 96 45, 128 54), and the line lies at two
+// full super-blocks of difference (140 rows 4096 x 14336 twice: whole rounds 166, all cut 148 us).
 struct TilePlan {
     int tiles_m, ctas, cut_tiles, most_tokens, tiles[MAX_MATS], whole[MAX_MATS], units[MAX_MATS], cut[MAX_MATS], shift[MAX_MATS], slot0[MAX_MATS];
     size_t img, part;
@@ -257,16 +269,21 @@ TilePlan plan_tiles(uint32_t type, int M, int K, const int* ns, int n_mats, bool
     const int nsb = K / 256, sms = ctx().sm_count;
     pl.tiles_m = (M + TT - 1) / TT;
     pl.img = align256(static_cast<size_t>((M + 7) / 8) * nsb * gemm_i8_act_bytes(type));
+    const int full = 62 + TT, mean = pl.tiles_m == 1 ? full : ((pl.tiles_m - 1) * full + 62 + M - (pl.tiles_m - 1) * TT) / pl.tiles_m;       // work of a super-block
     int at = 0, slots = 0;
     for (int i = 0; i < n_mats; ++i) {
-        const int tiles = pl.tiles_m * ((ns[i] + TW - 1) / TW), rest = tiles % sms;
+        const int tiles = pl.tiles_m * ((ns[i] + TW - 1) / TW);
+        int rest = tiles % sms;
+        const bool uneven = rest && static_cast<long long>(tiles / sms) * nsb * (full - mean) >= 2 * full;
+        if (uneven && allow_cut) rest = tiles;
         int used = rest;
         pl.tiles[i] = pl.whole[i] = tiles;
         pl.shift[i] = at;
         pl.slot0[i] = slots;
         if (rest && allow_cut) {
-            const int units = rest * nsb, cut = units / 2 < sms ? units / 2 : sms;
-            if (cut > rest) {
+            const int units = rest * nsb, even = (units + sms - 1) / sms, longest = even > 2 ? even : 2;
+            const int cut = longest > 4 ? sms : (units + longest - 1) / longest;
+            if (uneven || cut >= 2 * rest || (cut > rest && nsb - longest >= 3)) {
                 pl.whole[i] = tiles - rest;
                 pl.units[i] = units;
                 pl.cut[i] = used = cut;
@@ -274,7 +291,7 @@ TilePlan plan_tiles(uint32_t type, int M, int K, const int* ns, int n_mats, bool
                 pl.cut_tiles += rest;
             }
         }
-        const int need = tiles >= sms ? sms : used;
+        const int need = pl.whole[i] >= sms ? sms : used;
         if (need > pl.ctas) pl.ctas = need;
         at = (at + used) % sms;
     }
