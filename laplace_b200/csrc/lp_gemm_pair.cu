@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(256) quantize_pair_kernel(const float* __restr
 
 // Adds up the pieces of every cut tile in k order. Block (t, j): tokens 16 j .. 16 j + 15 of cut tile t, four at a time; a thread has four rows.
 template <bool PEERS>
-__global__ void __launch_bounds__(256, 4) pair_fixup_kernel(const __grid_constant__ PairParams p, const PairPeers<PEERS> pe) {
+__global__ void __launch_bounds__(256) pair_fixup_kernel(const __grid_constant__ PairParams p, const PairPeers<PEERS> pe) {
     int t = blockIdx.x;
     const int nsb = p.K / 256;
     Seg sg;
@@ -721,7 +721,7 @@ __global__ void __launch_bounds__(256, 4) pair_fixup_kernel(const __grid_constan
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int tok0 = blockIdx.y * 16 + (threadIdx.x >> 6);
     if (ca == cb || n >= N) return;
-    // two pieces' loads in flight: a short wide matrix has a dozen and more a tile (144 rows, 14336 x 1024: 43.0 us one by one, 40.2 so)
+    // two pieces' loads in flight: a short wide matrix has a dozen and more a tile (144 rows, 14336 x 1024: 34.1 us one by one, 32.1 so)
     float4 a[4];
     const float* src = p.part + static_cast<size_t>(p.slot0[sg.mat] + ca + t) * SLOT + tok0 * ROWS + col;
     for (int left = cb - ca + 1; left > 0; left -= 2, src += 2 * SLOT) {
@@ -761,12 +761,13 @@ __global__ void __launch_bounds__(256, 4) pair_fixup_kernel(const __grid_constan
 
 inline size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 
-// How the tiles are shared out: as many rounds of whole tiles as every pair gets, the rest cut evenly, into as few pieces as the longest
-// pair's work allows. A pair takes three super-blocks of cut tiles or more, two of tiles that have eight at most if half of the pairs are
-// enough for that (2048 x 2048, 144 rows: three 23.7, two 18.9 us, the one-CTA kernel 21.7; with more of them the matrices of one call get
-// into each other's way, 2048 x 5632 + 5632, 190 rows: 42.7 -> 49.1 us). None are cut unless the longest pair's work shrinks by four
-// super-blocks (some 10 us: adding up the pieces is one more launch and 256 KB of partial results written and read for each; 4096 x 14336,
-// 256 rows: whole tiles 56.8, cut for a gain of three 63.3 us).
+// How the tiles are shared out: as many rounds of whole tiles as every pair gets, the rest cut evenly. A pair takes three super-blocks of
+// cut tiles or more, two of tiles that have eight at most if half of the pairs are enough for that (2048 x 2048, 144 rows: three 23.7, two
+// 18.9 us, the one-CTA kernel 21.7; with more of them the matrices of one call get into each other's way, 2048 x 5632 + 5632, 190 rows:
+// 42.7 -> 49.1 us); up to four a pair the pieces are as few as its work allows, beyond that there is one for every pair (320 rows 4096 x 14336,
+// nine at most: 68 pieces 91.4, 74 86.8 us). None are cut unless the longest pair's work shrinks by four super-blocks (some 10 us: adding up
+// the pieces is one more launch and 256 KB of partial results written and read for each; 4096 x 14336, 256 rows: whole tiles 56.8, cut for
+// a gain of three 63.3 us).
 struct PairPlan {
     int tiles_m, m_pad, pairs, cut_tiles, tiles[MAX_MATS], whole[MAX_MATS], units[MAX_MATS], cut[MAX_MATS], shift[MAX_MATS], slot0[MAX_MATS];
     size_t a, s, inv, part;
@@ -788,7 +789,7 @@ PairPlan plan_pair(uint32_t type, int M, int K, const int* ns, int n_mats, int m
         pl.slot0[i] = slots;
         if (allow_cut && rest) {
             const int units = rest * nsb, least = nsb <= 8 && units <= max_pairs ? 2 : 3, even = (units + max_pairs - 1) / max_pairs;
-            const int longest = even > least ? even : least, cut = (units + longest - 1) / longest;
+            const int longest = even > least ? even : least, cut = longest > 4 ? max_pairs : (units + longest - 1) / longest;
             if (cut > 1 && nsb - longest >= 4) {
                 pl.whole[i] = tiles - rest;
                 pl.units[i] = units;
