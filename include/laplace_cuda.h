@@ -362,6 +362,8 @@ int laplace_cuda_last_path(void);
 /* Which kernel the last matmul launched ran on: 1 = dp4a streaming, 2 = int8 MMA for a handful of rows and for experts
  * (mma.sync), 3 = int8 MMA tiles, 4 = tcgen05, 5 = tcgen05 with weights in two pieces, 6 = fp32 activations. For tests. */
 int laplace_cuda_last_kernel(void);
+/* How many CTAs worked on one tile of it together: 2 = a pair of SMs (tcgen05 cta_group::2), else 1. For tests. */
+int laplace_cuda_last_cta_group(void);
 /* Kernel launches issued by this library since the counter was last reset. */
 long long laplace_cuda_launch_count(int reset);
 

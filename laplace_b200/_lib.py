@@ -55,6 +55,7 @@ SYMBOLS = {
     "laplace_cuda_gguf_close": (None, [_vp]),
     "laplace_cuda_last_path": (_i, []),
     "laplace_cuda_last_kernel": (_i, []),
+    "laplace_cuda_last_cta_group": (_i, []),
     "laplace_cuda_launch_count": (C.c_longlong, [_i]),
 }
 

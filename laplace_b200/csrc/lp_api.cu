@@ -295,7 +295,8 @@ const char* laplace_cuda_last_error(void) { return g_err; }
 int laplace_cuda_sm_count(void) { return g_ctx.ready ? g_ctx.sm_count : 0; }
 
 int laplace_cuda_last_path(void) { return g_ctx.last_path; }
-int laplace_cuda_last_kernel(void) { return g_ctx.last_kernel; }
+int laplace_cuda_last_kernel(void) { return g_ctx.last_kernel & ~KERNEL_ON_PAIRS; }
+int laplace_cuda_last_cta_group(void) { return g_ctx.last_kernel & KERNEL_ON_PAIRS ? 2 : 1; }
 
 long long laplace_cuda_launch_count(int reset) {
     long long v = g_ctx.launches;

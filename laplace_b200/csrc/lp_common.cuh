@@ -51,7 +51,8 @@ struct Context {
     int          last_kernel = 0;      // KERNEL_*
     long long    launches = 0;
 };
-enum : int { KERNEL_DP4A = 1, KERNEL_INT8 = 2, KERNEL_INT8_TILES = 3, KERNEL_TCGEN05 = 4, KERNEL_TCGEN05_TWO_PIECE = 5, KERNEL_F32ACT = 6 };      // laplace_cuda_last_kernel
+enum : int { KERNEL_DP4A = 1, KERNEL_INT8 = 2, KERNEL_INT8_TILES = 3, KERNEL_TCGEN05 = 4, KERNEL_TCGEN05_TWO_PIECE = 5, KERNEL_F32ACT = 6,
+             KERNEL_ON_PAIRS = 8 };      // laplace_cuda_last_kernel; ON_PAIRS: added to it, laplace_cuda_last_cta_group
 Context& ctx();
 int  fail(int code, const char* fmt, ...);   // records the message, returns code
 int  cuda_check(cudaError_t e, const char* what);

@@ -905,7 +905,7 @@ int launch_gemm_pair(uint8_t* scratch, bool cut, const float* x, const float* no
     }
     if (rc) return rc;
     ctx().last_path = 2;
-    ctx().last_kernel = type == LAPLACE_TYPE_Q4_K ? KERNEL_TCGEN05 : KERNEL_TCGEN05_TWO_PIECE;
+    ctx().last_kernel = KERNEL_ON_PAIRS | (type == LAPLACE_TYPE_Q4_K ? KERNEL_TCGEN05 : KERNEL_TCGEN05_TWO_PIECE);
     return cuda_check(cudaGetLastError(), "gemm_pair launch");
 }
 

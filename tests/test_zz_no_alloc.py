@@ -53,7 +53,7 @@ def test_noalloc_matches_the_allocating_entry_point_twice(oracle):
 
 @pytest.mark.parametrize("t,M,K,N", [(GGMLType.Q4_K, 512, 4096, 1024),      # the K-split's partial sums do not fit the array: runs unsplit
                                      (GGMLType.Q6_K, 72, 2048, 200),        # the other type the prefill kernels take
-                                     (GGMLType.Q4_K, 500, 4096, 128)])      # scratch close to the array's size, K-split kept
+                                     (GGMLType.Q4_K, 500, 4096, 128)])      # the pair kernel's operand close to the array's size: whole tiles too
 def test_noalloc_other_plans_and_types(oracle, t, M, K, N):
     from laplace_b200 import device
     L = device.lib()
@@ -74,6 +74,31 @@ def test_noalloc_has_the_bits_of_the_allocating_entry_point(oracle, t, M, K, N):
     a, b = _call(device.lib(), t, x, w, M, K, N)
     assert np.array_equal(a, b)
     check_close(a, oracle.gemm(x, w, t, M, K, N, mode=1, threads=THREADS), f"noalloc {t.name} {M}x{K}x{N}")
+
+
+@pytest.mark.parametrize("t,M,K,N,ctas", [(GGMLType.Q4_K, 512, 4608, 300, 1),       # 4.5 bytes a value do not fit, the one-CTA kernel's 4.13 do
+                                          (GGMLType.Q6_K, 512, 4608, 300, 2)])      # 4 bytes a value: whole tiles on pairs
+def test_noalloc_close_to_its_limit(oracle, t, M, K, N, ctas):
+    from laplace_b200 import device
+    L = device.lib()
+    w, x = synth.random_blocks(t, K, N, seed=99), synth.normal_f32(100, (M, K))
+    a, b = _call(L, t, x, w, M, K, N)
+    assert L.laplace_cuda_last_cta_group() == ctas
+    check_close(a, b.astype(np.float64), "noalloc vs the allocating entry point")
+    check_close(a, oracle.gemm(x, w, t, M, K, N, mode=1, threads=THREADS), f"noalloc {t.name} {M}x{K}x{N}")
+
+
+@pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q6_K])
+def test_noalloc_keeps_cut_tiles_whose_pieces_fit(oracle, t):
+    """144 x 4096 x 256 on pairs: one tile of sixteen super-blocks in six pieces of 256 KB."""
+    from laplace_b200 import device
+    L = device.lib()
+    M, K, N = 144, 4096, 256
+    w, x = synth.random_blocks(t, K, N, seed=101), synth.normal_f32(102, (M, K))
+    L.laplace_cuda_launch_count(1)
+    a, b = _call(L, t, x, w, M, K, N)
+    assert L.laplace_cuda_last_cta_group() == 2 and L.laplace_cuda_launch_count(0) == 6          # quantizer, matmul, pieces; twice
+    assert np.array_equal(a, b)
 
 
 def test_noalloc_rejects_what_it_cannot_serve():
