@@ -16,8 +16,10 @@
 //          pieces each, the products p1 g1 + p2 g1 + p1 g2 + p2 g2 + p3 g1 + p1 g3 of them. They come last, the smallest first: where a
 //          block is not centred at 8 they are several times the result, and every step after them is truncated against them (first: random
 //          blocks 9.7e-7, min / max packed ones 6.2e-7; last: 3.6 and 6.8e-7, before the accumulator was drained twice a super-block).
-//   Q6_K   sc * (q6 - 32) reaches 4096, one bit more than fp16 holds: the rounded value and the rest (-1, 0 or 1). The rest meets hi only
-//          (times lo it is below 2^-22 of the largest product) and goes in first.
+//   Q6_K   sc * (q6 - 32) reaches 4096, one bit more than fp16 holds: the rounded value and the rest (-1, 0 or 1). Of a stage's products the
+//          smallest go in first: rest x hi (rest x lo is below 2^-22 of the largest and left out), value x lo, value x hi. What is
+//          drained after every stage makes long chains of additions in the drain's registers (224 of them at K = 14336, and more error than
+//          all else together), so after 28 super-blocks at most the sums are set aside in scratch memory, 128 KB a CTA.
 //
 // One 512-thread CTA per SM, persistent; roles by warp:
 //   0, 2   copies: hi / lo piece of the activations (64 k x up to 128 tokens, 128-byte swizzle); warp 2 the sum pieces too
@@ -53,11 +55,13 @@ constexpr int SLOT = TOK * ROWS;             // floats of a partial tile: [token
 // UNIT: stages that an accumulator takes in: as many as leave no more error than the one-CTA kernels do, for any weights. Relative error
 // against 64 bits, 256 x 4096 x 512, N(0, 1) activations, random blocks / min-max packed / absmax packed weights:
 //   Q4_K   one-CTA kernel 3.0 / 6.6 / 2.8e-7; four stages 3.6 / 6.8 / 3.6, two 2.1 / 3.8 / 2.1, one 1.5 / 2.4 / 1.5
-//   Q6_K   one-CTA kernel 2.0 / 4.4 / 3.2e-7; two stages 2.8 / 4.2 / 3.3, one 1.9 / 2.5 / 2.1, one with the rest first 1.7 / 2.0 / 1.8
+//   Q6_K   one-CTA kernel 2.0 / 4.4 / 3.2e-7; two stages 2.8 / 4.2 / 3.3, smallest products first 2.1 / 3.1 / 2.5, one stage so 1.2 / 1.4 / 1.3
 // Time at 2048 tokens: Q4_K 4096 x 14336 four 356, two 367, one 420 us; Q6_K 14336 x 4096 two 509, one 526 us.
+// CHAIN: most super-blocks after which the drain sets its sums aside. Q6_K, random blocks, one-CTA kernel / never / after 16 / 32: 2048 x 14336 x
+// 4096 2.25 / 2.8 / 1.67 / 2.07e-7 (16: 8 % of the time, 32: 2 %), K = 8192 in one sum 2.07 and 2.21e-7, so the line lies below that.
 template <uint32_t TYPE> struct Geo;
-template <> struct Geo<LAPLACE_TYPE_Q4_K> { static constexpr int SB = Q4_K_BYTES, PITCH = Q4_K_BYTES, STAGES = 3, PIECES = 1, UNIT = 2; static constexpr bool MINS = true; };
-template <> struct Geo<LAPLACE_TYPE_Q6_K> { static constexpr int SB = Q6_K_BYTES, PITCH = 240, STAGES = 2, PIECES = 2, UNIT = 1; static constexpr bool MINS = false; };
+template <> struct Geo<LAPLACE_TYPE_Q4_K> { static constexpr int SB = Q4_K_BYTES, PITCH = Q4_K_BYTES, STAGES = 3, PIECES = 1, UNIT = 2, CHAIN = 1 << 20; static constexpr bool MINS = true; };
+template <> struct Geo<LAPLACE_TYPE_Q6_K> { static constexpr int SB = Q6_K_BYTES, PITCH = 240, STAGES = 2, PIECES = 2, UNIT = 1, CHAIN = 28; static constexpr bool MINS = false; };
 
 template <uint32_t TYPE> struct Lay {
     using G = Geo<TYPE>;
@@ -90,6 +94,7 @@ struct PairParams {
     // of the t-th cut tile is the matrix's partial result c + t: from one piece to the next c or t grows, or both.
     int          tiles[MAX_MATS], whole[MAX_MATS], units[MAX_MATS], cut[MAX_MATS], shift[MAX_MATS], slot0[MAX_MATS];
     float*       part;
+    float*       aside;            // [CTA][TOK][128]: sums of K taken out of the drain's registers every CHAIN super-blocks
 };
 // Row-split over several GPUs: the result goes to row-major [M][ld] buffers of every GPU at column col0 + n instead of y[0].
 template <bool PEERS> struct PairPeers {};
@@ -331,15 +336,20 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ 
                         if (!wait_pair(sbase + L::FULL + 8 * s, (it / STAGES) & 1, abort_flag, p.err, DEV_TIMEOUT_FULL)) { ok = false; break; }
                         fence_after();
                         const uint64_t w = smem_desc_sw128(sbase + L::W + s * G::PIECES * TILE), x = smem_desc_sw128(sbase + L::A + 2 * s * TILE);
-                        // 32 bytes >> 4 inside the swizzle row; the rest of Q6_K's weights, the smallest products, first
-                        if (G::PIECES == 2) {
+                        // (32 bytes >> 4 inside the swizzle row)
+                        if constexpr (G::PIECES == 2) {                                // the smallest products first
 #pragma unroll
                             for (int ks = 0; ks < 4; ++ks) mma_f16_pair(acc, w + (TILE >> 4) + 2 * ks, x + 2 * ks, idesc, more | ks);
-                        }
 #pragma unroll
-                        for (int ks = 0; ks < 4; ++ks) {
-                            mma_f16_pair_fill(acc, w + 2 * ks, x + (TILE >> 4) + 2 * ks, idesc, (G::PIECES == 2) | more | ks);
-                            mma_f16_pair_last(acc, w + 2 * ks, x + 2 * ks, idesc, 1);
+                            for (int ks = 0; ks < 4; ++ks) mma_f16_pair(acc, w + 2 * ks, x + (TILE >> 4) + 2 * ks, idesc, 1);
+#pragma unroll
+                            for (int ks = 0; ks < 4; ++ks) mma_f16_pair(acc, w + 2 * ks, x + 2 * ks, idesc, 1);
+                        } else {
+#pragma unroll
+                            for (int ks = 0; ks < 4; ++ks) {
+                                mma_f16_pair_fill(acc, w + 2 * ks, x + (TILE >> 4) + 2 * ks, idesc, more | ks);
+                                mma_f16_pair_last(acc, w + 2 * ks, x + 2 * ks, idesc, 1);
+                            }
                         }
                         commit_pair(sbase + L::EMPTY + 8 * s);
                         if (G::MINS && c == 3) {                                       // the smallest products first
@@ -512,7 +522,32 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ 
             float2 y[64];
 #pragma unroll
             for (int c = 0; c < 64; ++c) y[c] = make_float2(0.f, 0.f);
-            for (int n = sg.sb1 - sg.sb0; n > 0 && ok; --n, ++sbc) {
+            // y of this thread's row set aside: kept here (first) or added to what is kept
+            float* aside = TYPE == LAPLACE_TYPE_Q6_K ? p.aside + (static_cast<size_t>(blockIdx.x) * TOK + half * 128) * 128 + wr : nullptr;
+            auto add_aside = [&](int h) {                            // sixteen tokens' sums, loads in flight together
+                float v[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) v[e] = aside[(16 * h + e) * 128];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) { y[8 * h + e].x += v[2 * e]; y[8 * h + e].y += v[2 * e + 1]; }
+            };
+            auto set_aside = [&](bool first) {
+#pragma unroll
+                for (int h = 0; h < 8; ++h) {
+                    if (16 * h >= live) break;
+                    if (!first) add_aside(h);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        aside[(16 * h + 2 * e) * 128] = y[8 * h + e].x;
+                        aside[(16 * h + 2 * e + 1) * 128] = y[8 * h + e].y;
+                        y[8 * h + e] = make_float2(0.f, 0.f);
+                    }
+                }
+            };
+            const int len = sg.sb1 - sg.sb0, chains = (len + G::CHAIN - 1) / G::CHAIN, step = (len + chains - 1) / chains;
+            int left = len - step;                                   // super-blocks to go when the sums are next set aside
+            for (int n = len; n > 0 && ok; --n, ++sbc) {
+                if (n == left) { set_aside(left == len - step); left -= step; }
                 const int slot = sbc % TABN;
                 if (!wait_or_abort<false>(sbase + L::TAB_FULL + 8 * slot, (sbc / TABN) & 1, abort_flag, p.err, DEV_TIMEOUT_FULL)) { ok = false; break; }
                 const float d = __uint_as_float(lds32(sbase + L::TAB + (slot * 128 + wr) * 4));
@@ -539,6 +574,11 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ 
                 }
             }
             if (!ok) break;
+            if (chains > 1) {
+#pragma unroll
+                for (int h = 0; h < 8; ++h)
+                    if (16 * h < live) add_aside(h);
+            }
             // for a fixed token the warp's 32 lanes write 32 consecutive floats
             const int n = sg.n0 + static_cast<int>(rank) * 128 + wr, N = p.N[sg.mat], tok0 = half * 128;
             float inv[4];                                            // of column 32 k + lane
@@ -770,8 +810,8 @@ inline size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 // a gain of three 63.3 us).
 struct PairPlan {
     int tiles_m, m_pad, pairs, cut_tiles, tiles[MAX_MATS], whole[MAX_MATS], units[MAX_MATS], cut[MAX_MATS], shift[MAX_MATS], slot0[MAX_MATS];
-    size_t a, s, inv, part;
-    size_t total() const { return a + s + inv + part; }
+    size_t a, s, inv, part, aside;
+    size_t total() const { return a + s + inv + part + aside; }
 };
 PairPlan plan_pair(uint32_t type, int M, int K, const int* ns, int n_mats, int max_pairs, bool allow_cut) {
     PairPlan pl{};
@@ -804,6 +844,7 @@ PairPlan plan_pair(uint32_t type, int M, int K, const int* ns, int n_mats, int m
     }
     if (n_mats > 1) pl.pairs = max_pairs;
     pl.part = static_cast<size_t>(slots) * SLOT * sizeof(float);
+    pl.aside = type == LAPLACE_TYPE_Q6_K && nsb > Geo<LAPLACE_TYPE_Q6_K>::CHAIN ? static_cast<size_t>(2 * pl.pairs) * TOK * 128 * sizeof(float) : 0;
     return pl;
 }
 
@@ -864,7 +905,8 @@ int launch_gemm_pair(uint8_t* scratch, bool cut, const float* x, const float* no
     p.inv_s = op.inv_s; p.err = ctx().d_err;
     p.M = M; p.K = K; p.m_pad = pl.m_pad; p.tiles_m = pl.tiles_m; p.n_mats = n_mats;
     p.rb = static_cast<int>(rb);
-    p.part = reinterpret_cast<float*>(scratch);
+    p.part = reinterpret_cast<float*>(scratch);             scratch += pl.part;
+    p.aside = reinterpret_cast<float*>(scratch);
     p.by_row = rb % 16 != 0;
     for (int i = 0; i < n_mats; ++i) {
         p.w[i] = ws[i]; p.y[i] = ys ? ys[i] : nullptr; p.N[i] = ns[i];

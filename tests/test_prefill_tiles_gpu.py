@@ -29,7 +29,7 @@ def _run(t, x, ws, M, K, Ns):
 
 
 @pytest.mark.parametrize("t,M,K,N", [(Q4_K, 129, 256, 1), (Q4_K, 256, 1024, 127), (Q4_K, 257, 512, 255), (Q4_K, 300, 2304, 257), (Q4_K, 144, 4096, 6000), (Q4_K, 513, 16640, 130),
-                                     (Q6_K, 129, 256, 129), (Q6_K, 256, 2048, 256), (Q6_K, 257, 768, 33), (Q6_K, 290, 4096, 4100), (Q6_K, 160, 14336, 300),
+                                     (Q6_K, 129, 256, 129), (Q6_K, 256, 2048, 256), (Q6_K, 257, 768, 33), (Q6_K, 290, 4096, 4100), (Q6_K, 160, 14336, 300), (Q6_K, 270, 16896, 100),
                                      (Q4_K, 144, 2048, 300), (Q4_K, 150, 14336, 260), (Q6_K, 300, 2048, 600),
                                      (Q8_0, 33, 256, 1), (Q8_0, 130, 1792, 9600), (Q8_0, 96, 2816, 129), (Q8_0, 97, 2816, 4000), (Q4_0, 129, 768, 127), (Q4_0, 64, 14336, 640), (Q4_K, 80, 1024, 700), (Q6_K, 112, 2048, 128)])
 def test_edges_of_tiles(oracle, t, M, K, N):
@@ -68,6 +68,20 @@ def test_pairs_are_no_further_from_64_bits_than_single_ctas(oracle, t, pack, row
     (y,) = _run(t, x, [w], M, K, [N])
     one = np.concatenate([_run(t, x[m:m + 128], [w], 128, K, [N])[0] for m in (0, 128)])
     err, err_one = (np.linalg.norm(v - ref) for v in (y, one))
+    assert err <= 1.02 * err_one, f"{err / np.linalg.norm(ref):.3e} against {err_one / np.linalg.norm(ref):.3e}"
+
+
+@pytest.mark.parametrize("t", [Q4_K, Q6_K])
+@pytest.mark.parametrize("K", [7168, 8192, 18432])
+def test_long_rows_on_pairs_are_no_further_from_64_bits(oracle, t, K):
+    """The same with whole tiles for every pair, so that a tile's K is summed by one CTA, at one go (7168) or, Q6_K, with sums set aside
+    once (8192) and twice (18432); 16 of the 130 rows, 16 x 18944 errors: 0.13 %."""
+    M, N = 130, 18944
+    w, x = synth.random_blocks(t, K, N, seed=750), synth.normal_f32(751, (M, K))
+    ref = oracle.gemm(x[:16], w, t, 16, K, N, mode=1, threads=THREADS).astype(np.float64)
+    (y,) = _run(t, x, [w], M, K, [N])
+    (one,) = _run(t, x[:128], [w], 128, K, [N])
+    err, err_one = (np.linalg.norm(v[:16] - ref) for v in (y, one))
     assert err <= 1.02 * err_one, f"{err / np.linalg.norm(ref):.3e} against {err_one / np.linalg.norm(ref):.3e}"
 
 

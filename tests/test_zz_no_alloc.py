@@ -77,7 +77,8 @@ def test_noalloc_has_the_bits_of_the_allocating_entry_point(oracle, t, M, K, N):
 
 
 @pytest.mark.parametrize("t,M,K,N,ctas", [(GGMLType.Q4_K, 512, 4608, 300, 1),       # 4.5 bytes a value do not fit, the one-CTA kernel's 4.13 do
-                                          (GGMLType.Q6_K, 512, 4608, 300, 2)])      # 4 bytes a value: whole tiles on pairs
+                                          (GGMLType.Q6_K, 512, 4608, 300, 2),       # 4 bytes a value: whole tiles on pairs
+                                          (GGMLType.Q6_K, 256, 9728, 600, 1)])      # but not what longer rows set aside
 def test_noalloc_close_to_its_limit(oracle, t, M, K, N, ctas):
     from laplace_b200 import device
     L = device.lib()
