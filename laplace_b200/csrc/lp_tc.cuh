@@ -97,6 +97,9 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
     return r;
 }
+// What such an arrival announces is read by the tensor cores alone, in the CTA that wrote it and after its fence.proxy.async, or is TMEM that
+// a fenced tcgen05.ld has read: no thread of the other CTA loads anything that a release at cluster scope would have to make visible to
+// it, as the sums in lp_gemm_i8.cu do (.release.cluster here: 19 % on the calls of the pair kernel, up to 55).
 __device__ __forceinline__ void arrive_cluster(uint32_t remote_bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" :: "r"(remote_bar) : "memory");
 }
@@ -135,11 +138,11 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr) {
     return static_cast<uint64_t>((addr >> 4) & 0x3fffu) | (static_cast<uint64_t>(1) << 16) | (static_cast<uint64_t>(512 >> 4) << 32) |
            (static_cast<uint64_t>(1) << 46) | (static_cast<uint64_t>(4) << 61);
 }
-// As wait_or_abort, for arrivals from the other CTA of the pair.
+// As wait_or_abort, for arrivals from the other CTA of the pair too (acquire at cluster scope, which costs nothing here).
 __device__ __forceinline__ bool wait_pair(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err, int code) {
     for (uint32_t it = 0; it < (1u << 24); ++it) {
         uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
         if (ok) return true;
         if (*abort_flag) return false;
