@@ -592,11 +592,12 @@ bool plan_dense(uint32_t type, int M, int K, long long rows, DensePlan& d) {
         d.smax = (nsb + c - 1) / c;
         d.kw = d.smax >= 8 ? 2 : 1;
         d.act = (static_cast<uint32_t>(d.nt * d.smax * g.act_bytes) + 127u) & ~127u;
-        // Two ring slots a warp; then partial results, a row group taking kw x 8 nt x 16 floats: two rounds of row groups, at least
-        // half a round and one place in every CTA; then more slots.
+        // Two ring slots a warp; then partial results, a row group taking kw x 8 nt x 16 floats from every CTA of the cluster: room for
+        // two rounds of row groups, at least for half a round and for two places in every CTA of four (with less room eight CTAs, whose
+        // activations take half of it, have more places than four would); then more slots.
         const long long slot = static_cast<long long>(CW) * 16 * g.pitch, group = d.kw * 8 * d.nt * 16 * 4, round = CW / d.kw * group;
         long long rest = static_cast<long long>(ctx().smem_optin) - OFF_ACT - d.act - 128 - 2 * slot;
-        const long long least = c == 1 ? 0 : (round / 2 > (MAX_MATS + 1) * group ? round / 2 : (MAX_MATS + 1) * group), most = c == 1 ? 0 : 2 * round > 32 * 1024 ? 2 * round : 32 * 1024;
+        const long long least = c == 1 ? 0 : (round / 2 > 9 * group ? round / 2 : 9 * group), most = c == 1 ? 0 : 2 * round > 32 * 1024 ? 2 * round : 32 * 1024;
         if (rest < least) continue;
         d.part_budget = static_cast<uint32_t>(rest < most ? rest : most) & ~127u;
         rest -= d.part_budget;

@@ -84,7 +84,7 @@ struct PairParams {
     const float* inv_s;            // [m_pad]: 2^-e of the row
     int*         err;
     int          M, K, m_pad, tiles_m, n_mats;
-    int          rb, by_row;       // bytes per weight row; 1: rows that a tensor map cannot address are copied one by one
+    int          rb, by_row;       // bytes per weight row; 1 (Q6_K): rows that a tensor map cannot address are copied one by one
     const uint8_t* w[MAX_MATS];
     float*       y[MAX_MATS];
     int          N[MAX_MATS];
@@ -142,11 +142,6 @@ __device__ __forceinline__ bool segment(const PairParams& p, int i, Seg& s) {
     return false;
 }
 
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-    return r;
-}
 __device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t*>(&v); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2*>(&v); }
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -380,7 +375,7 @@ gemm_pair_kernel(const __grid_constant__ PairMaps maps, const __grid_constant__ 
                     const int s = sbc % RAWN;
                     const uint32_t dst = sbase + L::RAW + s * 128 * G::PITCH, bar = sbase + L::RAW_FULL + 8 * s;
                     if (!wait_or_abort<false>(sbase + L::RAW_EMPTY + 8 * s, ((sbc / RAWN) & 1) ^ 1, abort_flag, p.err, DEV_TIMEOUT_EMPTY)) { ok = false; break; }
-                    if (!p.by_row) {
+                    if (TYPE == LAPLACE_TYPE_Q4_K || !p.by_row) {
                         if (lane == 0) {
                             mbar_expect_tx(bar, 128 * G::PITCH);
                             tma_load_2d(dst, &maps.w[sg.mat], ((sb * G::SB) & ~15) / 4, row, bar);

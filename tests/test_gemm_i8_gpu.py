@@ -39,8 +39,8 @@ def test_small_batches(oracle, t, M, K, N):
 
 @pytest.mark.parametrize("M", [8, 24])
 def test_more_rows_than_one_panel(oracle, M):
-    """A cluster's share of the rows goes through shared memory in several panels: about 2100 rows of 33 clusters' with room for 64
-    row groups (8 rows) or 32 (24 rows), the last panel ragged."""
+    """Far more row groups than a CTA has places for partial results: some 130 of a cluster's share, 33 a CTA, for eight places (8 rows) or
+    six (24 rows), the last group ragged."""
     t, K, N = GGMLType.Q4_K, 4096, 70001
     w = synth.weights(t, K, N, seed=610, how="affine")
     x = synth.normal_f32(611, (M, K))
@@ -62,9 +62,10 @@ def test_matrices_that_share_normalised_rows(oracle, t, M, K, Ns):
 
 
 @pytest.mark.parametrize("t,M,K", [(GGMLType.Q4_K, 16, 11008), (GGMLType.Q4_K, 24, 14336), (GGMLType.Q4_K, 8, 24832), (GGMLType.Q8_0, 24, 8192), (GGMLType.Q6_K, 32, 8192),
-                                   (GGMLType.Q4_0, 32, 11520)])
+                                   (GGMLType.Q4_0, 32, 11520), (GGMLType.Q8_0, 24, 16384)])
 def test_eight_matrices_where_partial_results_have_little_room(oracle, t, M, K):
-    """Room for eight row groups in clusters of four and of eight CTAs: panels end inside matrices and hold the ends of several."""
+    """Two places and one for partial results in every CTA of clusters of four and of eight (one: one of the two adding warps has nothing to
+    do; with one warp a row group and with two), the groups cut at the ends of several matrices."""
     Ns = (1500, 1, 700, 16, 5, 1290, 64, 800)
     ws = [synth.random_blocks(t, K, n, seed=650 + i) for i, n in enumerate(Ns)]
     x = synth.normal_f32(651, (M, K))
