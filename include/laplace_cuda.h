@@ -140,8 +140,9 @@ int laplace_cuda_moe_gemv_dev(const float* x, const uint8_t* w, uint32_t type,
  * every matrix streams past it: y_i[m*N_i + j] = dot(quantize(x_norm[m]), row j of matrix i). x_norm_out (optional)
  * receives the normalised rows [M][K]. 1..8 matrices. Device pointers. With M <= 8 (decode) everything is one launch;
  * with more rows (prefill; K a multiple of 256) one quantizer launch normalises and quantizes the rows once, and the
- * matrices then run as tensor-core GEMMs on that shared operand: all in one launch with up to 32 rows (weights as
- * for laplace_cuda_gemm_dev above), one by one with more. */
+ * matrices then run as tensor-core GEMMs on that shared operand, all in one launch (and one more that adds up partial
+ * results); one by one for Q4_K with 81 to 128 rows, Q6_K with 113 to 128, and where weights are not 16-byte aligned or
+ * rows are not a multiple of 16 bytes (Q6_K above 128 rows excepted). */
 typedef struct { const uint8_t* w; float* y; int N; } laplace_cuda_matrix;
 int laplace_cuda_gemm_multi_dev(const float* x, const float* norm_weight, float norm_eps, float* x_norm_out,
                                 const laplace_cuda_matrix* mats, int n_mats, uint32_t type, int M, int K, void* stream);

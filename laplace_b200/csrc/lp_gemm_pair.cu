@@ -7,8 +7,8 @@
 // outputs reads 12 KB of operands and takes in 13 KB, some 210 cycles of its bandwidth for 128 of the tensor core. Here a step of 128
 // rows x 256 tokens per CTA reads 12 KB (the weight operand once for both pieces: it stays in the collector) and takes in 14 KB for 256
 // cycles of the tensor core. Measured (us, calls with quantizer and all, one-CTA kernels -> here): Q4_K 4096 x 14336, 512 tokens 180 -> 108,
-// 2048 tokens 703 -> 364; 4096 x 4096, 512 tokens 59.8 -> 48.9; Q6_K 14336 x 4096, 512 tokens 316 -> 144, 2048 tokens 1199 -> 521. At 2048
-// tokens the card's power limit holds the clock at 1.3 to 1.5 GHz: Q4_K takes 5250 cycles per super-block and tile for the MMAs' 4480.
+// 1024 tokens 344 -> 194; 4096 x 4096, 512 tokens 59 -> 45; 2048 x 2048, 144 tokens 21.5 -> 18; Q6_K 14336 x 4096, 512 tokens 315 -> 144, 1024
+// tokens 601 -> 292. At 2048 tokens the card's power limit holds the clock at 1.3 to 1.5 GHz.
 // hi and lo meet in one accumulator. Sums in it are truncated, not rounded, at every MMA step, so it is drained after every stage or
 // two (figures at UNIT), lo goes in before hi, and what goes in is small:
 //   Q4_K   weight operand sc * (nibble - 8), exact in fp16. What is then missing is a contraction over the super-block's eight blocks and
@@ -56,9 +56,10 @@ constexpr int SLOT = TOK * ROWS;             // floats of a partial tile: [token
 // against 64 bits, 256 x 4096 x 512, N(0, 1) activations, random blocks / min-max packed / absmax packed weights:
 //   Q4_K   one-CTA kernel 3.0 / 6.6 / 2.8e-7; four stages 3.6 / 6.8 / 3.6, two 2.1 / 3.8 / 2.1, one 1.5 / 2.4 / 1.5
 //   Q6_K   one-CTA kernel 2.0 / 4.4 / 3.2e-7; two stages 2.8 / 4.2 / 3.3, smallest products first 2.1 / 3.1 / 2.5, one stage so 1.2 / 1.4 / 1.3
-// Time at 2048 tokens: Q4_K 4096 x 14336 four 356, two 367, one 420 us; Q6_K 14336 x 4096 two 509, one 526 us.
-// CHAIN: most super-blocks after which the drain sets its sums aside. Q6_K, random blocks, one-CTA kernel / never / after 16 / 32: 2048 x 14336 x
-// 4096 2.25 / 2.8 / 1.67 / 2.07e-7 (16: 8 % of the time, 32: 2 %), K = 8192 in one sum 2.07 and 2.21e-7, so the line lies below that.
+// Time at 2048 tokens: Q4_K 4096 x 14336 four 356, two 367, one 420 us; Q6_K 14336 x 4096 two 509, one 526 us (before sums were set aside).
+// CHAIN: most super-blocks after which the drain sets its sums aside. Q6_K, random blocks, one-CTA kernel / never (with lo and hi in turn) / after 16 / 32: 2048 x 14336 x
+// 4096 2.25 / 2.8 / 1.67 / 2.07e-7 (16: 8 % of the time, 32: 2 %); K = 8192 in one sum 2.12 and 2.21e-7, so the line lies below that: 28 gives
+// 1.99e-7 and, K = 28672, 1.94e-7 for 2.38.
 template <uint32_t TYPE> struct Geo;
 template <> struct Geo<LAPLACE_TYPE_Q4_K> { static constexpr int SB = Q4_K_BYTES, PITCH = Q4_K_BYTES, STAGES = 3, PIECES = 1, UNIT = 2, CHAIN = 1 << 20; static constexpr bool MINS = true; };
 template <> struct Geo<LAPLACE_TYPE_Q6_K> { static constexpr int SB = Q6_K_BYTES, PITCH = 240, STAGES = 2, PIECES = 2, UNIT = 1, CHAIN = 28; static constexpr bool MINS = false; };
@@ -800,7 +801,7 @@ inline size_t align256(size_t n) { return (n + 255) & ~size_t(255); }
 // cut tiles or more, two of tiles that have eight at most if half of the pairs are enough for that (2048 x 2048, 144 rows: three 23.7, two
 // 18.9 us, the one-CTA kernel 21.7; with more of them the matrices of one call get into each other's way, 2048 x 5632 + 5632, 190 rows:
 // 42.7 -> 49.1 us); up to four a pair the pieces are as few as its work allows, beyond that there is one for every pair (320 rows 4096 x 14336,
-// nine at most: 68 pieces 91.4, 74 86.8 us). None are cut unless the longest pair's work shrinks by four super-blocks (some 10 us: adding up
+// nine at most: 68 pieces 91.4, 74 90.6 us). None are cut unless the longest pair's work shrinks by four super-blocks (some 10 us: adding up
 // the pieces is one more launch and 256 KB of partial results written and read for each; 4096 x 14336, 256 rows: whole tiles 56.8, cut for
 // a gain of three 63.3 us).
 struct PairPlan {
