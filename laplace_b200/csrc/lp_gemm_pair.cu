@@ -57,9 +57,9 @@ constexpr int SLOT = TOK * ROWS;             // floats of a partial tile: [token
 //   Q4_K   one-CTA kernel 3.0 / 6.6 / 2.8e-7; four stages 3.6 / 6.8 / 3.6, two 2.1 / 3.8 / 2.1, one 1.5 / 2.4 / 1.5
 //   Q6_K   one-CTA kernel 2.0 / 4.4 / 3.2e-7; two stages 2.8 / 4.2 / 3.3, smallest products first 2.1 / 3.1 / 2.5, one stage so 1.2 / 1.4 / 1.3
 // Time at 2048 tokens: Q4_K 4096 x 14336 four 356, two 367, one 420 us; Q6_K 14336 x 4096 two 509, one 526 us (before sums were set aside).
-// CHAIN: most super-blocks after which the drain sets its sums aside. Q6_K, random blocks, one-CTA kernel / never (with lo and hi in turn) / after 16 / 32: 2048 x 14336 x
-// 4096 2.25 / 2.8 / 1.67 / 2.07e-7 (16: 8 % of the time, 32: 2 %); K = 8192 in one sum 2.12 and 2.21e-7, so the line lies below that: 28 gives
-// 1.99e-7 and, K = 28672, 1.94e-7 for 2.38.
+// CHAIN: most super-blocks after which the drain sets its sums aside. Q6_K, random blocks, error in 1e-7, one-CTA kernel / after 16 / 28 / 32:
+// 2048 x 14336 x 4096 2.25 / 1.67 / 1.99 / 2.07; K = 8192 in one sum is 2.21 where the one-CTA kernel has 2.12, so the line lies below that.
+// 14336 x 4096, 512 tokens: 28 144, 32 145 us.
 template <uint32_t TYPE> struct Geo;
 template <> struct Geo<LAPLACE_TYPE_Q4_K> { static constexpr int SB = Q4_K_BYTES, PITCH = Q4_K_BYTES, STAGES = 3, PIECES = 1, UNIT = 2, CHAIN = 1 << 20; static constexpr bool MINS = true; };
 template <> struct Geo<LAPLACE_TYPE_Q6_K> { static constexpr int SB = Q6_K_BYTES, PITCH = 240, STAGES = 2, PIECES = 2, UNIT = 1, CHAIN = 28; static constexpr bool MINS = false; };
